@@ -38,8 +38,16 @@ inline cudaError_t set_smem(K kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Room for the block's visit histogram after `smem` bytes, if it is wanted and
+// fits (else the kernel counts in global memory).
+inline size_t add_block_hist(TraceArgs& a, bool count, size_t smem) {
+  const size_t bytes = kHistBins * sizeof(uint32_t);
+  a.block_hist = count && a.depth_hist != nullptr && smem + bytes <= 227 * 1024;
+  return a.block_hist ? smem + bytes : smem;
+}
+
 template <int NM, int PROFILE, int KIND, bool COUNT, int FMT>
-inline cudaError_t launch_one(const SceneDev& sc, const TraceArgs& a, const LaunchCfg& cfg,
+inline cudaError_t launch_one(const SceneDev& sc, TraceArgs a, const LaunchCfg& cfg,
                               cudaStream_t s) {
   if (a.n == 0) return cudaSuccess;
   if (cfg.scheme == BVHGPU_PER_RAY) {
@@ -49,7 +57,8 @@ inline cudaError_t launch_one(const SceneDev& sc, const TraceArgs& a, const Laun
     constexpr bool kDist = KIND == BVHGPU_CLOSEST;
     const bool dist = kDist && cfg.save_distance;
     const bool local = cfg.stack_local && !dist && !COUNT && a.stack_cap <= kLocalStack;
-    const size_t smem = local ? 0 : (size_t)a.stack_cap * bs * 4 * (dist ? 2 : 1);
+    const size_t smem =
+        local ? 0 : add_block_hist(a, COUNT, (size_t)a.stack_cap * bs * 4 * (dist ? 2 : 1));
     auto k = dist ? trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, kDist>
              : local ? trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false, (COUNT ? 0 : kLocalStack)>
                      : trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false>;
@@ -91,7 +100,8 @@ inline cudaError_t launch_one(const SceneDev& sc, const TraceArgs& a, const Laun
   } else {
     if (FMT != kFmtFP32) return cudaErrorNotSupported;
     const int p = cfg.packet;
-    const size_t smem = stream_smem_bytes(p, a.stack_cap, COUNT, COUNT && a.step_stats);
+    const size_t smem = add_block_hist(
+        a, COUNT, stream_smem_bytes(p, a.stack_cap, COUNT, COUNT && a.step_stats));
     auto k = trace_stream_kernel<NM, PROFILE, KIND, COUNT>;
     cudaError_t e = set_smem(k, smem);
     if (e != cudaSuccess) return e;

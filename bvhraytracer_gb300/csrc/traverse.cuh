@@ -107,6 +107,9 @@ struct TraceArgs {
   // Step log of intersectWide's schedule (a node visit followed by a leaf
   // visit counts as one step) instead of intersectWideAlternative's.
   bool step_wide = false;
+  // With depth_hist: the block has kHistBins words of shared memory for its
+  // own histogram (see hist_flush).
+  bool block_hist = false;
 };
 
 BVHGPU_DEV uint64_t out_slot(const TraceArgs& a, uint64_t rid) {
@@ -796,18 +799,56 @@ BVHGPU_DEV bool leaf_step(const SceneDev& sc, uint32_t e, const Ray& r, float& t
 
 BVHGPU_DEV void record_error(int* status, int code) { atomicCAS(status, 0, code); }
 
+// Visit histograms of a counting launch: [0, 64) node visits per depth,
+// [64, 128) leaf visits per depth, [128, 145) visits of nodes with c children,
+// [145, 162) of leaves with c triangles.
+constexpr int kHistBins = 128 + 34;
+
 // Counting launches: one node visit (depth_count = depth | child count << 8,
 // as node_step returns it) into the per-depth histogram and childFullness
 // (compactNode.cpp:714-716), one leaf visit into the per-depth histogram and
-// primitiveFullness (compactNode.cpp:653-656).
-BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count) {
-  if (a.depth_hist) atomicAdd(a.depth_hist + min(depth_count & 0xFF, 63), 1ull);
-  if (a.fullness) atomicAdd(a.fullness + min(depth_count >> 8, 16), 1ull);
+// primitiveFullness (compactNode.cpp:653-656). hist: the block's own
+// histogram in shared memory, or null: straight to global memory.
+BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count, uint32_t* hist) {
+  const int depth = min(depth_count & 0xFF, 63), fill = 128 + min(depth_count >> 8, 16);
+  if (hist != nullptr) {
+    atomicAdd(hist + depth, 1u);
+    atomicAdd(hist + fill, 1u);
+    return;
+  }
+  if (a.depth_hist) atomicAdd(a.depth_hist + depth, 1ull);
+  if (a.fullness) atomicAdd(a.fullness + fill - 128, 1ull);
 }
-BVHGPU_DEV void count_leaf(const SceneDev& sc, const TraceArgs& a, uint32_t e) {
+BVHGPU_DEV void count_leaf(const SceneDev& sc, const TraceArgs& a, uint32_t e, uint32_t* hist) {
+  const int fill = 128 + 17 + (int)((e >> kLeafCountShift) & 15u) + 1;
+  if (hist != nullptr) {
+    atomicAdd(hist + 64 + min((int)sc.leaf_depth[e & kLeafIndexMask], 63), 1u);
+    atomicAdd(hist + fill, 1u);
+    return;
+  }
   if (a.depth_hist)
     atomicAdd(a.depth_hist + 64 + min((int)sc.leaf_depth[e & kLeafIndexMask], 63), 1ull);
-  if (a.fullness) atomicAdd(a.fullness + 17 + (int)((e >> kLeafCountShift) & 15u) + 1, 1ull);
+  if (a.fullness) atomicAdd(a.fullness + fill - 128, 1ull);
+}
+
+// The block's histogram: every visit of a launch adds to a few dozen bins, so
+// 64-bit atomics on global memory queue up behind one another in L2. A block
+// adds to its own copy in shared memory (32-bit: a block has at most 256 rays)
+// and to global memory once per bin at its end: 640 x 360 primary and shadow
+// rays on a 251k-triangle N16L16 tree 4.31 -> 0.36 ms, now bound by the
+// traversal itself. The persistent kernel, whose blocks take any number of
+// rays, keeps the 64-bit atomics on global memory.
+BVHGPU_DEV void hist_clear(uint32_t* hist) {
+  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0u;
+  __syncthreads();
+}
+BVHGPU_DEV void hist_flush(const TraceArgs& a, const uint32_t* hist) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
+    if (hist[i] == 0u) continue;
+    if (i < 128) atomicAdd(a.depth_hist + i, (unsigned long long)hist[i]);
+    else if (a.fullness) atomicAdd(a.fullness + i - 128, (unsigned long long)hist[i]);
+  }
 }
 
 // Rays are 32-byte records read with two 128-bit loads (16-byte aligned buffer).
@@ -858,29 +899,10 @@ BVHGPU_DEV void write_result(const SceneDev& sc, const TraceArgs& a, uint64_t ri
       make_float4(__int_as_float(h.prim), h.t, h.u, h.v);
 }
 
-// ---------------------------------------------------------------------------
-// Per-ray depth-first traversal: one thread per ray, the traversal stack in
-// shared memory (stack[slot][thread], conflict-free across a warp).
-// DIST: intersectSaveDistance (fastNodeManager.h:1232-1326) /
-// intersectImmediately(ray, useDistance = true) (compactNode.cpp:623-645):
-// every entry also carries its box's entry distance (in a second shared
-// array after the stack), the root enters with 0, and a pop whose distance
-// exceeds the current tMax is dropped before it is visited or counted.
-// LSTACK > 0: the stack is a per-thread array of LSTACK entries in local
-// memory (stride 1) instead of shared memory (the stack-placement knob of the
-// autotuner); the caller guarantees a_stack_cap <= LSTACK.
-template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST = false, int LSTACK = 0>
-__global__ void __launch_bounds__(128) trace_dfs_kernel(SceneDev sc, TraceArgs a) {
-  extern __shared__ uint32_t smem[];
-  uint32_t lstack[LSTACK > 0 ? LSTACK : 1];
-  const int stride = LSTACK > 0 ? 1 : (int)blockDim.x;
-  uint32_t* stack = LSTACK > 0 ? lstack : smem + threadIdx.x;
-  float* dstack = DIST ? reinterpret_cast<float*>(smem + (size_t)a.stack_cap * stride) + threadIdx.x
-                       : nullptr;
-  unsigned long long* hist = nullptr;
-  const uint64_t rid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (rid >= a.n) return;
-
+// One ray of the per-ray scheme, from its record to its result.
+template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST>
+BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t rid,
+                              uint32_t* stack, float* dstack, int stride, uint32_t* hist) {
   const bvhgpu_ray_t in = load_ray(a.rays, out_slot(a, rid));
   if (isnan(in.ox)) {
     Best none;
@@ -904,7 +926,7 @@ __global__ void __launch_bounds__(128) trace_dfs_kernel(SceneDev sc, TraceArgs a
     const uint32_t e = stack[sp * stride];
     if (DIST && dstack[sp * stride] > tmax) continue;
     if (e & kLeafBit) {
-      if (COUNT) count_leaf(sc, a, e);
+      if (COUNT) count_leaf(sc, a, e, hist);
       bool h = leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr);
       if (h) {
         hit = true;
@@ -919,13 +941,44 @@ __global__ void __launch_bounds__(128) trace_dfs_kernel(SceneDev sc, TraceArgs a
         best = Best();
         break;
       }
-      if (COUNT) count_node(a, depth);
+      if (COUNT) count_node(a, depth, hist);
       if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
     }
   }
-  (void)hist;
   write_result<KIND>(sc, a, rid, hit, tmax, best);
   flush_counters<COUNT>(a, rid, ctr);
+}
+
+// ---------------------------------------------------------------------------
+// Per-ray depth-first traversal: one thread per ray, the traversal stack in
+// shared memory (stack[slot][thread], conflict-free across a warp).
+// DIST: intersectSaveDistance (fastNodeManager.h:1232-1326) /
+// intersectImmediately(ray, useDistance = true) (compactNode.cpp:623-645):
+// every entry also carries its box's entry distance (in a second shared
+// array after the stack), the root enters with 0, and a pop whose distance
+// exceeds the current tMax is dropped before it is visited or counted.
+// LSTACK > 0: the stack is a per-thread array of LSTACK entries in local
+// memory (stride 1) instead of shared memory (the stack-placement knob of the
+// autotuner); the caller guarantees a_stack_cap <= LSTACK.
+template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST = false, int LSTACK = 0>
+__global__ void __launch_bounds__(128) trace_dfs_kernel(SceneDev sc, TraceArgs a) {
+  extern __shared__ uint32_t smem[];
+  uint32_t lstack[LSTACK > 0 ? LSTACK : 1];
+  const int stride = LSTACK > 0 ? 1 : (int)blockDim.x;
+  uint32_t* stack = LSTACK > 0 ? lstack : smem + threadIdx.x;
+  float* dstack = DIST ? reinterpret_cast<float*>(smem + (size_t)a.stack_cap * stride) + threadIdx.x
+                       : nullptr;
+  const uint64_t rid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (COUNT) {
+    // After the stacks, where it fits (TraceArgs::block_hist).
+    uint32_t* hist = a.block_hist ? smem + (size_t)a.stack_cap * stride * (DIST ? 2 : 1) : nullptr;
+    if (hist != nullptr) hist_clear(hist);
+    if (rid < a.n)
+      trace_dfs_ray<N, PROFILE, KIND, COUNT, FMT, DIST>(sc, a, rid, stack, dstack, stride, hist);
+    if (hist != nullptr) hist_flush(a, hist);
+  } else if (rid < a.n) {
+    trace_dfs_ray<N, PROFILE, KIND, COUNT, FMT, DIST>(sc, a, rid, stack, dstack, stride, nullptr);
+  }
 }
 
 
@@ -1041,6 +1094,8 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
   uint16_t* work0 = reinterpret_cast<uint16_t*>(base);  // list c at work0 + c * P
   base += (size_t)P * 4;
   uint32_t* ctrs = reinterpret_cast<uint32_t*>(base);  // [8][P]
+  uint32_t* hist = COUNT && a.block_hist ? ctrs + 8 * P : nullptr;
+  if (COUNT && hist != nullptr) hist_clear(hist);
 
   const uint64_t first = (uint64_t)blockIdx.x * P;
   const uint64_t rid = first + tid;
@@ -1134,7 +1189,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
       if (log && set_insert(set, 2 * P, e))
         atomicAdd(is_node ? &ctl->unique_nodes : &ctl->unique_leaves, 1);
       auto leaf_visit = [&](uint32_t le) {
-        if (COUNT) count_leaf(sc, a, le);
+        if (COUNT) count_leaf(sc, a, le, hist);
         Best best;
         best.leaf = best_leaf[ray];
         best.lane = (int)(int8_t)(misc & 0xFF);
@@ -1163,7 +1218,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
           done = true;
           sp = 0;
         }
-        if (COUNT) count_node(a, depth);
+        if (COUNT) count_node(a, depth, hist);
         // intersectWide's schedule (compactNode.cpp:118-356, step log only):
         // a ray whose next entry is a leaf visits it in the same step.
         if (log && a.step_wide && !done && sp > 0 && (stacks[(sp - 1) * P + ray] & kLeafBit)) {
@@ -1243,6 +1298,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
     __syncthreads();
   }
   if (log && tid == 0) a.step_count[blockIdx.x] = (uint32_t)step;
+  if (COUNT && hist != nullptr) hist_flush(a, hist);
 
   // Results of this thread's own ray slot.
   if (rid < a.n) {
@@ -1610,14 +1666,14 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
             best = Best();
             sp = 0;
           }
-          if (COUNT) count_node(a, depth);
+          if (COUNT) count_node(a, depth, nullptr);
           if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
         }
       }
       if (active && sp > 0) {
         --sp;
         const uint32_t e = stack[sp * stride];
-        if (COUNT) count_leaf(sc, a, e);
+        if (COUNT) count_leaf(sc, a, e, nullptr);
         if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
           hit = true;
           if (KIND == BVHGPU_ANY) sp = 0;
@@ -1628,7 +1684,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
         --sp;
         const uint32_t e = stack[sp * stride];
         if (e & kLeafBit) {
-          if (COUNT) count_leaf(sc, a, e);
+          if (COUNT) count_leaf(sc, a, e, nullptr);
           if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
             hit = true;
             if (KIND == BVHGPU_ANY) sp = 0;
@@ -1642,7 +1698,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
             best = Best();
             sp = 0;
           }
-          if (COUNT) count_node(a, depth);
+          if (COUNT) count_node(a, depth, nullptr);
           if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
         }
       }
