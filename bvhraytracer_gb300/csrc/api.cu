@@ -17,6 +17,7 @@
 #include "bvhgpu.h"
 #include "bvhgpu_status.hpp"
 #include "launch.cuh"
+#include "pack.cuh"
 #include "reorder.cuh"
 #include "raygen.cuh"
 #include "q8_encode.cuh"
@@ -67,6 +68,10 @@ struct bvhgpu_scene {
   uint32_t* d_leaf_prim = nullptr;
   uint8_t* d_leaf_depth = nullptr;
   uint32_t* d_child_entry = nullptr;
+  // Packed scene of the ray-pool kernel (pack.cuh).
+  uint8_t* d_pack_nodes = nullptr;
+  float4* d_pack_blocks = nullptr;
+  uint32_t pack_root = 0;  // stack entry of the root in the packed scene
   float* d_leaf_bounds = nullptr;
   int* d_status = nullptr;
   uint32_t* d_prim_slot = nullptr;  // uploaded on first FP64 check
@@ -75,6 +80,7 @@ struct bvhgpu_scene {
   static constexpr int kQueueSlots = 64;
   unsigned long long* d_queue = nullptr;
   std::atomic<unsigned> queue_next{0};
+  unsigned long long* next_queue() { return d_queue + queue_next.fetch_add(1) % kQueueSlots; }
   int sm_count = 0;
   // Staging for bvhgpu_trace_host (grown on demand): one region per
   // pipeline stream, and the streams / events that order them.
@@ -109,6 +115,8 @@ struct bvhgpu_scene {
     cudaFree(d_leaf_prim);
     cudaFree(d_leaf_depth);
     cudaFree(d_child_entry);
+    cudaFree(d_pack_nodes);
+    cudaFree(d_pack_blocks);
     cudaFree(d_leaf_bounds);
     cudaFree(d_status);
     cudaFree(d_queue);
@@ -124,6 +132,8 @@ struct bvhgpu_scene {
     d_leaf_prim = nullptr;
     d_leaf_depth = nullptr;
     d_child_entry = nullptr;
+    d_pack_nodes = nullptr;
+    d_pack_blocks = nullptr;
     d_leaf_bounds = nullptr;
     d_status = nullptr;
     d_queue = nullptr;
@@ -203,37 +213,63 @@ static int check_smem_fit(const dev::LaunchCfg& cfg, int cap) {
 // Shared memory per block for the persistent kernel's copy of the top levels;
 // small enough to keep six blocks per SM next to the traversal stacks.
 constexpr uint32_t kTopStageBytes = 8192;
+// Deepest trees of the ray-pool kernel: their stacks leave two blocks per SM.
+constexpr int kPoolMaxLevels = 48;
 
-static int launch(bvhgpu_scene_t s, const dev::TraceArgs& a, dev::LaunchCfg cfg,
-                  cudaStream_t st) {
-  dev::SceneDev sc = s->dev_view();
-  sc.any_index_order = cfg.any_order ? 1 : 0;
-  cfg.sm_count = s->sm_count;
-  cfg.queue = s->d_queue + (s->queue_next.fetch_add(1) % bvhgpu_scene::kQueueSlots);
-  cfg.fmt = s->layout.node_format;
-  if (cfg.scheme == BVHGPU_PERSISTENT) {
-    // Stage the top levels (up to kTopStageBytes) in shared memory.
-    const uint32_t fit = kTopStageBytes / (uint32_t)s->layout.record_bytes;
-    cfg.top_nodes = std::min(s->layout.top_nodes, fit);
-    cfg.stall_bytes = s->stall_bytes;
-  }
-  if (cfg.scheme == BVHGPU_STREAM && cfg.fmt != BVHGPU_NODES_FP32)
-    return set_error(BVHGPU_ERR_UNSUPPORTED, "the stream scheme traverses FP32 nodes only");
-  cudaError_t e;
-  switch (s->layout.node_stride) {
-    case 4: e = dev::launch_trace_n4(sc, a, cfg, st); break;
-    case 8: e = dev::launch_trace_n8(sc, a, cfg, st); break;
-    case 12: e = dev::launch_trace_n12(sc, a, cfg, st); break;
-    case 16: e = dev::launch_trace_n16(sc, a, cfg, st); break;
-    default: return set_error(BVHGPU_ERR_UNSUPPORTED, "node width");
-  }
-  if (e != cudaSuccess) return cuda_error(e, "trace launch");
-  return BVHGPU_OK;
+// The packed scene, made on the device. The caller's streams may not be
+// ordered after the default stream, so this waits for it.
+static cudaError_t pack_scene(bvhgpu_scene* s) {
+  const DeviceLayout& L = s->layout;
+  const size_t node = dev::pack_node_bytes(L.node_stride, L.node_format);
+  const size_t blocks = L.leaf_block[L.n_leaves];
+  uint32_t* d_block = nullptr;
+  uint8_t* d_count = nullptr;
+  cudaError_t e = cudaMalloc((void**)&s->d_pack_nodes, std::max<size_t>(L.n_inner * node, 16));
+  if (e == cudaSuccess)
+    e = cudaMalloc((void**)&s->d_pack_blocks, blocks * dev::kBlockWords * sizeof(float4));
+  if (e == cudaSuccess)
+    e = cudaMalloc((void**)&s->d_leaf_bounds, (size_t)L.n_leaves * sizeof(float) *
+                                                  dev::leaf_bounds_floats(L.leaf_memory));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&d_block, L.leaf_block.size() * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&d_count, L.leaf_count.size());
+  if (e == cudaSuccess)
+    e = cudaMemcpy(d_block, L.leaf_block.data(), L.leaf_block.size() * sizeof(uint32_t),
+                   cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(d_count, L.leaf_count.data(), L.leaf_count.size(), cudaMemcpyHostToDevice);
+  const dev::SceneDev sc = s->dev_view();
+  if (e == cudaSuccess)
+    e = dev::pack_nodes(sc, L.node_stride, L.node_format, L.n_inner, d_block, s->d_pack_nodes,
+                        nullptr);
+  if (e == cudaSuccess)
+    e = dev::pack_leaves(sc, L.n_leaves, d_block, d_count, s->d_pack_blocks, s->d_leaf_bounds,
+                         nullptr);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+  cudaFree(d_block);
+  cudaFree(d_count);
+  // A root that is a leaf is leaf 0, whose first block is block 0.
+  s->pack_root = L.root_entry;
+  return e;
 }
 
-static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+// Whether a launch runs on the ray-pool kernel, which traces without counters
+// every ray kind, profile and scheme (results do not depend on the scheme).
+// The kernels of the schemes themselves run what it does not: counters and
+// step logs, save-distance closest hits, a capped traversal stack (their
+// stacks hold one entry per pushed child, which is what the cap counts), the
+// staging wait of the failure-detection tests, node records whose boxes are
+// not ordered (imported trees), trees too deep or large for its stack words,
+// and more than 2^32 - 1 rays.
+static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
+  const DeviceLayout& L = s->layout;
+  return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) &&
+         stack_cap(s) >= s->max_stack && s->stall_bytes == 0 && a.n <= 0xFFFFFFFFull &&
+         (L.node_format != BVHGPU_NODES_FP32 || L.boxes_ordered) &&
+         L.n_inner < dev::pool_max_inner(L.node_stride) && L.inner_levels <= kPoolMaxLevels &&
+         L.leaf_block[L.n_leaves] <= dev::kMaxBlocks;
+}
 
-// Stream-ordered scratch for the reorder passes comes from a memory pool of
+// Stream-ordered scratch (reorder passes, queues) comes from a memory pool of
 // the library's own (one per device, created on first use) that keeps freed
 // memory instead of returning it at every synchronisation, so repeated
 // traces reuse it; the process's default pool is left as the caller set it.
@@ -264,9 +300,87 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
   return e == cudaSuccess ? BVHGPU_OK : set_error(BVHGPU_ERR_OOM, "scratch allocation failed");
 }
 
-// Scratch bytes of a reordered launch of n rays into k x k cells per face.
+// A trace on the packed scene. A large batch needs two words of device memory
+// of its own while it runs: the caller's (c.pool_queue) or stream-ordered
+// scratch. A stream that is being captured gets none (an allocation would put
+// memory nodes into the caller's graph), nor does a full device: then every
+// ray has its own thread.
+static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
+                               cudaStream_t st) {
+  dev::PoolArgs p;
+  p.nodes = s->d_pack_nodes;
+  p.blocks = s->d_pack_blocks;
+  p.root_entry = s->pack_root;
+  p.gang = s->layout.gang;
+  p.levels = std::max(1, s->layout.inner_levels);
+  p.rays = a.rays;
+  p.n = (uint32_t)a.n;
+  p.hits = a.hits;
+  p.occluded = a.occluded;
+  p.out_index = a.out_index;
+  p.queue = c.pool_queue;
+  void* scratch = nullptr;
+  if (!p.queue && dev::pool_wants_queue(a.n)) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone &&
+        scratch_alloc(s->device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
+      p.queue = static_cast<unsigned long long*>(scratch);
+    else
+      cudaGetLastError();
+  }
+  cudaError_t e;
+  switch (s->layout.node_stride) {
+    case 4: e = dev::launch_pool_n4(p, c, st); break;
+    case 8: e = dev::launch_pool_n8(p, c, st); break;
+    case 12: e = dev::launch_pool_n12(p, c, st); break;
+    default: e = dev::launch_pool_n16(p, c, st); break;
+  }
+  if (scratch) {
+    const cudaError_t f = cudaFreeAsync(scratch, st);
+    if (e == cudaSuccess) e = f;
+  }
+  return e;
+}
+
+static int launch(bvhgpu_scene_t s, const dev::TraceArgs& a, dev::LaunchCfg cfg,
+                  cudaStream_t st) {
+  dev::SceneDev sc = s->dev_view();
+  sc.any_index_order = cfg.any_order ? 1 : 0;
+  cfg.sm_count = s->sm_count;
+  cfg.queue = s->next_queue();
+  cfg.fmt = s->layout.node_format;
+  if (cfg.scheme == BVHGPU_PERSISTENT) {
+    // Stage the top levels (up to kTopStageBytes) in shared memory.
+    const uint32_t fit = kTopStageBytes / (uint32_t)s->layout.record_bytes;
+    cfg.top_nodes = std::min(s->layout.top_nodes, fit);
+    cfg.stall_bytes = s->stall_bytes;
+  }
+  if (cfg.scheme == BVHGPU_STREAM && cfg.fmt != BVHGPU_NODES_FP32)
+    return set_error(BVHGPU_ERR_UNSUPPORTED, "the stream scheme traverses FP32 nodes only");
+  cudaError_t e;
+  if (uses_pool(s, a, cfg)) {
+    e = launch_pool(s, a, cfg, st);
+    return e == cudaSuccess ? BVHGPU_OK : cuda_error(e, "trace launch");
+  }
+  switch (s->layout.node_stride) {
+    case 4: e = dev::launch_trace_n4(sc, a, cfg, st); break;
+    case 8: e = dev::launch_trace_n8(sc, a, cfg, st); break;
+    case 12: e = dev::launch_trace_n12(sc, a, cfg, st); break;
+    case 16: e = dev::launch_trace_n16(sc, a, cfg, st); break;
+    default: return set_error(BVHGPU_ERR_UNSUPPORTED, "node width");
+  }
+  if (e != cudaSuccess) return cuda_error(e, "trace launch");
+  return BVHGPU_OK;
+}
+
+static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+// Scratch bytes of a reordered launch of n rays into k x k cells per face; the
+// launch's pool queue is at their end.
+constexpr size_t kPoolQueueBytes = 256;
 static size_t reorder_bytes(uint64_t n, int k) {
-  return align256(n * 4) + dev::reorder_scratch_bytes(n, k);
+  return align256(n * 4) + align256(dev::reorder_scratch_bytes(n, k)) + kPoolQueueBytes;
 }
 
 // launch() after grouping the rays by direction when cfg.reorder > 0: a
@@ -274,7 +388,7 @@ static size_t reorder_bytes(uint64_t n, int k) {
 // rays in that order and write every result to its input slot. The scratch
 // (about 6 bytes per ray, reorder_bytes) is the caller's `scratch` or is
 // allocated and freed on the stream.
-static int launch_reordered(bvhgpu_scene_t s, dev::TraceArgs a, const dev::LaunchCfg& cfg,
+static int launch_reordered(bvhgpu_scene_t s, dev::TraceArgs a, dev::LaunchCfg cfg,
                             cudaStream_t st, void* scratch = nullptr) {
   if (cfg.reorder <= 0 || a.n < 2) return launch(s, a, cfg, st);
   if (a.n > 0xFFFFFFFFull)
@@ -294,6 +408,8 @@ static int launch_reordered(bvhgpu_scene_t s, dev::TraceArgs a, const dev::Launc
     rc = cuda_error(e, "reorder");
   } else {
     a.out_index = perm;
+    cfg.pool_queue = reinterpret_cast<unsigned long long*>(
+        static_cast<uint8_t*>(p) + reorder_bytes(a.n, cfg.reorder) - kPoolQueueBytes);
     rc = launch(s, a, cfg, st);
   }
   if (!scratch) {
@@ -504,8 +620,7 @@ int bvhgpu_scene_create(bvhgpu_bvh_t h, const bvhgpu_scene_params_t* params, bvh
   if ((rc = upload(&s->d_nodes, s->layout.nodes)) || (rc = upload(&s->d_leaves, s->layout.leaves)) ||
       (rc = upload(&s->d_leaf_prim, s->layout.leaf_prim)) ||
       (rc = upload(&s->d_leaf_depth, s->layout.leaf_depth)) ||
-      (rc = upload(&s->d_child_entry, s->layout.child_entry)) ||
-      (rc = upload(&s->d_leaf_bounds, s->layout.leaf_bounds))) {
+      (rc = upload(&s->d_child_entry, s->layout.child_entry))) {
     s->release();
     delete s;
     return rc;
@@ -532,6 +647,7 @@ int bvhgpu_scene_create(bvhgpu_bvh_t h, const bvhgpu_scene_params_t* params, bvh
       return set_error(BVHGPU_ERR_UNSUPPORTED, "Q8 encoding: a box could not be enclosed");
     }
   }
+  if (e == cudaSuccess) e = pack_scene(s);
   if (e == cudaSuccess)
     e = cudaMalloc((void**)&s->d_queue, sizeof(unsigned long long) * bvhgpu_scene::kQueueSlots);
   if (e == cudaSuccess)
@@ -799,7 +915,7 @@ static int trace_host_pipeline(bvhgpu_scene_t s, const HostBatch* b, int nb, cud
       sort_bytes = std::max(sort_bytes, reorder_bytes(c.n, b[c.batch].cfg.reorder));
   const size_t ray_bytes = align256(max_chunk * sizeof(bvhgpu_ray_t));
   const size_t out_bytes = align256(max_chunk * sizeof(bvhgpu_hit_t));
-  const size_t per_stream = ray_bytes + out_bytes + sort_bytes;
+  const size_t per_stream = ray_bytes + out_bytes + sort_bytes + kPoolQueueBytes;
   const size_t need = per_stream * NS;
   if (need > s->stage_bytes) {
     cudaStreamSynchronize(st);
@@ -842,7 +958,9 @@ static int trace_host_pipeline(bvhgpu_scene_t s, const HostBatch* b, int nb, cud
     a.counters = nullptr;
     a.depth_hist = nullptr;
     a.stack_cap = stack_cap(s);
-    rc = launch_reordered(s, a, B.cfg, cs, sort_bytes ? base + ray_bytes + out_bytes : nullptr);
+    dev::LaunchCfg cfg = B.cfg;
+    cfg.pool_queue = reinterpret_cast<unsigned long long*>(base + per_stream - kPoolQueueBytes);
+    rc = launch_reordered(s, a, cfg, cs, sort_bytes ? base + ray_bytes + out_bytes : nullptr);
     if (rc) break;
     void* dst = closest ? (void*)(B.hits + first) : (void*)(B.occluded + first);
     e = cudaMemcpyAsync(dst, d_out, m * out_rec, cudaMemcpyDeviceToHost, cs);
@@ -1048,7 +1166,7 @@ int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_tra
     return set_error(BVHGPU_ERR_UNSUPPORTED, "stack does not fit shared memory for these trees");
   t->n_jobs = nj;
   t->total = total;
-  t->head = first->d_queue + (first->queue_next.fetch_add(1) % bvhgpu_scene::kQueueSlots);
+  t->head = first->next_queue();
   t->refill_min = cfg.refill_min;
   t->stack_cap = stack;
   t->policy = cfg.policy;
@@ -1109,7 +1227,7 @@ int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_tra
       one->split = 0;
       for (int i = 0; i < nj; ++i)
         if (t->jobs[i].kind != BVHGPU_ANY) one->split += t->jobs[i].n;
-      one->head_any = first->d_queue + (first->queue_next.fetch_add(1) % bvhgpu_scene::kQueueSlots);
+      one->head_any = first->next_queue();
       e = dev::launch_batched(*one, cfg.profile, 3, sms, st);
     }
   } else if (!BVHGPU_JOBS_SPLIT) {
@@ -1135,7 +1253,7 @@ int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_tra
       }
       part->n_jobs = m;
       part->total = begin;
-      part->head = first->d_queue + (first->queue_next.fetch_add(1) % bvhgpu_scene::kQueueSlots);
+      part->head = first->next_queue();
       e = dev::launch_batched(*part, cfg.profile, kind == BVHGPU_ANY ? 2 : 1, sms, st);
     }
   }
@@ -1465,11 +1583,11 @@ int bvhgpu_scene_status(bvhgpu_scene_t s, void* stream) {
 // after start-up, or a frame loop that cannot afford the device-wide
 // synchronisation an allocation may cause. bvhgpu_trace_batches_noalloc
 // serves them: it runs the persistent traversal kernel with its only scratch
-// (one ray-queue head per batch) in the fixed array below, so the call itself
+// (a ray-queue head and the batch's kernel per batch) in the fixed array below, so the call itself
 // allocates nothing; the caller passes the rays and the result buffers.
 //
 // The array is a file-scope device variable: every GPU that loads the library
-// holds its kNoAllocQueueSlots * 8 bytes until the process exits. Host code
+// holds its kNoAllocQueueSlots * 16 bytes until the process exits. Host code
 // may not use the symbol as an address, so the device address is looked up
 // with cudaGetSymbolAddress (with that device current) on the first call for
 // that device, and again on the first call after the device's context was
@@ -1484,8 +1602,8 @@ int bvhgpu_scene_status(bvhgpu_scene_t s, void* stream) {
 // (different streams of one device) race on the heads, so serialise them.
 namespace {
 
-constexpr int kNoAllocQueueSlots = 64;  // at most 64 batches per call (512 bytes)
-static __device__ __align__(256) unsigned long long g_noalloc_queue[kNoAllocQueueSlots];
+constexpr int kNoAllocQueueSlots = 64;  // at most 64 batches per call (1 KB)
+static __device__ __align__(256) unsigned long long g_noalloc_queue[2 * kNoAllocQueueSlots];
 
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
@@ -1577,7 +1695,7 @@ int bvhgpu_trace_batches_noalloc(bvhgpu_scene_t s, const bvhgpu_batch_t* batches
   unsigned long long* heads = nullptr;
   if ((rc = noalloc_scratch(s->device, &heads))) return rc;
   // The heads keep the previous call's values: clear the ones this call uses.
-  e = cudaMemsetAsync(heads, 0, sizeof(unsigned long long) * (size_t)n_batches, st);
+  e = cudaMemsetAsync(heads, 0, 2 * sizeof(unsigned long long) * (size_t)n_batches, st);
   if (e != cudaSuccess) return cuda_error(e, "no-alloc trace: clear queue heads");
   dev::SceneDev sc = s->dev_view();
   sc.any_index_order = cfg.any_order ? 1 : 0;
@@ -1596,12 +1714,18 @@ int bvhgpu_trace_batches_noalloc(bvhgpu_scene_t s, const bvhgpu_batch_t* batches
     c.kind = b.kind;
     c.count = false;
     c.sm_count = s->sm_count;
-    c.queue = heads + i;
+    c.queue = heads + 2 * i;
+    c.pool_queue = c.queue;
     c.queue_cleared = true;
     c.fmt = s->layout.node_format;
     // Top levels staged in shared memory, as the regular persistent launches do.
     c.top_nodes = std::min(s->layout.top_nodes, kTopStageBytes / (uint32_t)s->layout.record_bytes);
     c.stall_bytes = s->stall_bytes;
+    if (uses_pool(s, a, c)) {
+      e = launch_pool(s, a, c, st);
+      if (e != cudaSuccess) return cuda_error(e, "no-alloc trace launch");
+      continue;
+    }
     switch (s->layout.node_stride) {
       case 4: e = dev::launch_trace_n4(sc, a, c, st); break;
       case 8: e = dev::launch_trace_n8(sc, a, c, st); break;

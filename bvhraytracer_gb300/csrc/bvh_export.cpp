@@ -4,6 +4,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <algorithm>
 #include <limits>
 
 #include "bvhgpu_status.hpp"
@@ -310,7 +311,8 @@ int build_device_layout(const Bvh& bvh, int gang, int leaf_memory, int node_form
   out.leaves.assign((size_t)nl * 9 * leaf_memory, 0.0f);
   out.leaf_prim.assign((size_t)nl * leaf_memory, 0xFFFFFFFFu);
   out.leaf_depth.assign(nl, 0);
-  out.leaf_bounds.assign((size_t)nl * 6 * leaf_memory, 0.0f);
+  out.leaf_count.assign(nl, 0);
+  out.leaf_block.assign((size_t)nl + 1, 0);
   const float qnan = std::numeric_limits<float>::quiet_NaN();
   for (size_t id = 0; id < n; ++id) {
     const CompactNode& c = bvh.nodes[id];
@@ -324,17 +326,24 @@ int build_device_layout(const Bvh& bvh, int gang, int leaf_memory, int node_form
       for (int v = 0; v < 3; ++v)
         for (int a = 0; a < 3; ++a) blk[(v * 3 + a) * real + i] = t.p[v][a];
       out.leaf_prim[k * leaf_memory + i] = t.id;
-      float* bnd = &out.leaf_bounds[k * 6 * leaf_memory];
-      for (int a = 0; a < 3; ++a) {
-        bnd[a * leaf_memory + i] = std::fmin(std::fmin(t.p[0][a], t.p[1][a]), t.p[2][a]);
-        bnd[(3 + a) * leaf_memory + i] = std::fmax(std::fmax(t.p[0][a], t.p[1][a]), t.p[2][a]);
-      }
     }
     if (real != leaf_memory) {
       blk[leaf_memory * 9 - 2] = (float)real;
       blk[leaf_memory * 9 - 1] = qnan;
     }
     out.leaf_depth[k] = c.depth;
+    out.leaf_count[k] = (uint8_t)c.prim_count;
+    out.leaf_block[k + 1] = (c.prim_count + 3) / 4;
+  }
+  for (uint32_t k = 0; k < nl; ++k) out.leaf_block[k + 1] += out.leaf_block[k];
+  // Children come after their parent in the node order.
+  std::vector<int> level(n, 0);
+  out.inner_levels = 0;
+  for (size_t id = 0; id < n; ++id) {
+    const CompactNode& c = bvh.nodes[id];
+    if (c.child_count == 0) continue;
+    out.inner_levels = std::max(out.inner_levels, level[id] + 1);
+    for (uint32_t j = 0; j < c.child_count; ++j) level[c.child_begin + j] = level[id] + 1;
   }
   return BVHGPU_OK;
 }

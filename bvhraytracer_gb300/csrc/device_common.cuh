@@ -375,6 +375,11 @@ BVHGPU_DEV uint64_t f2mul(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+BVHGPU_DEV uint64_t f2add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 // a + b rounded up / down per half (the pairs of __fadd_ru / __fadd_rd).
 BVHGPU_DEV uint64_t f2add_ru(uint64_t a, uint64_t b) {
   uint64_t d;

@@ -1,0 +1,692 @@
+// Traces without counters, on the packed scene (pack.cuh): two kernels with the
+// same node and leaf visits.
+//
+// trace_solo_kernel: one thread per ray. trace_pool_kernel: each warp owns a
+// pool of kPoolRays rays in shared memory and three lists of them: rays whose
+// next entry is an inner node, rays whose next entry is a leaf, and free
+// slots. A step takes up to 32 rays of one list, so all lanes of the warp
+// visit nodes, or all visit leaves, or all set up new rays from the launch's
+// queue; the lists are kept by ballots, and no step needs a block barrier. A
+// ray's own visits stay in depth-first order, so results are those of the
+// scheme kernels in traverse.cuh (any-hit rays: occlusion does not depend on
+// the order of their visits, tMax is fixed).
+//
+// A ray's stack holds one word per level instead of one entry per pushed
+// child: the inner node and the set of its hit children still to visit (as
+// positions in the ray's push sequence). Its depth is bounded by the tree's
+// levels.
+//
+// What bounds them. Pool, ambient-occlusion rays in direction order (3.7M rays,
+// 251k triangles, N8L8): the L1 data pipe is busy 82 % of the time (a node
+// visit gathers 192 bytes of boxes), 21 lanes per instruction, issue 66 %;
+// 0.81 ms, against 1.18 ms of the persistent kernel (17.4 lanes, and 16 of 100
+// L1 cycles lost to bank conflicts of the leaf bounds' 192-byte stride).
+// 8.3M such rays of the 1M-triangle frame: 3.13 -> 2.04 ms; unordered, from
+// the per-ray kernel (6.7 lanes): 4.5M rays, N4L8, 2.97 -> 1.33 ms. Solo, 2.1M
+// primary rays of that frame 0.62 -> 0.51 ms, shadow rays 0.41 -> 0.31 ms
+// (latency: 20 % of the warps resident at the end of a launch).
+#pragma once
+#include "pack.cuh"
+#include "traverse.cuh"
+
+namespace bvhgpu {
+namespace dev {
+
+// Rays per pool. More rays fill the steps better and take L1 from the node
+// records (frame of the 1M-triangle scene / 4.5M unordered N4 rays: 48 rays
+// 4.94 / 1.47 ms, 56 4.69 / 1.48, 64 4.74 / 1.58, 96 5.5 / 1.77).
+#ifndef BVHGPU_POOL_RAYS
+#define BVHGPU_POOL_RAYS 56
+#endif
+constexpr int kPoolRays = BVHGPU_POOL_RAYS;
+constexpr int kPoolWarps = 4;  // per block
+// Resident blocks per SM (64 registers per thread): same frame with 64 rays
+// per pool, 8 blocks 4.80 ms, 7 4.95, 6 5.15, 5 5.4.
+#ifndef BVHGPU_POOL_MIN_BLOCKS
+#define BVHGPU_POOL_MIN_BLOCKS 8
+#endif
+// Free slots at which a warp takes new rays: a full step of them (same frame:
+// 32 4.80 ms, 24 5.0, 16 5.15, 8 5.4).
+#ifndef BVHGPU_POOL_REFILL
+#define BVHGPU_POOL_REFILL 32
+#endif
+
+#ifndef BVHGPU_SOLO_MIN_BLOCKS
+#define BVHGPU_SOLO_MIN_BLOCKS 4
+#endif
+
+struct PoolArgs {
+  const uint8_t* nodes;   // packed node records (PackFmt)
+  const float4* blocks;   // leaf blocks
+  uint32_t root_entry;    // stack entries of the packed records
+  int gang;
+  int levels;             // inner levels of the tree: words of a ray's stack
+  const bvhgpu_ray_t* rays;
+  uint32_t n;
+  bvhgpu_hit_t* hits;
+  uint8_t* occluded;
+  const uint32_t* out_index;  // as TraceArgs
+  // Two words of this launch's own: [0] next unclaimed ray of the pool kernel,
+  // [1] the kernel chosen by plan_kernel. Null: one thread per ray.
+  unsigned long long* queue;
+  int planned;                // 1: a kernel other than the chosen one returns at once
+  int slots;                  // rays a warp takes at once (32 or kPoolRays)
+};
+
+// Which of the two kernels traces a batch.
+constexpr unsigned long long kPlanSolo = 1, kPlanPool = 2;
+
+// A level of a ray's stack: the node and the set of its children left, in one
+// word for up to 8 children and 2^24 inner nodes.
+template <int NM>
+struct PoolWord {
+  using T = uint32_t;
+  static BVHGPU_DEV uint32_t make(uint32_t node, uint32_t left) { return node | (left << 24); }
+  static BVHGPU_DEV uint32_t node(uint32_t w) { return w & 0xFFFFFFu; }
+  static BVHGPU_DEV uint32_t left(uint32_t w) { return w >> 24; }
+};
+struct PoolWordWide {
+  using T = uint2;
+  static BVHGPU_DEV uint2 make(uint32_t node, uint32_t left) { return make_uint2(node, left); }
+  static BVHGPU_DEV uint32_t node(const uint2& w) { return w.x; }
+  static BVHGPU_DEV uint32_t left(const uint2& w) { return w.y; }
+};
+template <> struct PoolWord<12> : PoolWordWide {};
+template <> struct PoolWord<16> : PoolWordWide {};
+constexpr uint32_t pool_max_inner(int nm) { return nm <= 8 ? 1u << 24 : kLeafBit; }
+
+// Shared memory of one warp: three float4 and a word pair per ray, the stacks
+// and the lists.
+template <int NM>
+__host__ __device__ inline size_t pool_warp_bytes(int levels) {
+  return (size_t)kPoolRays * (3 * 16 + 8 + sizeof(typename PoolWord<NM>::T) * (size_t)levels) +
+         (3 * kPoolRays + 15) / 16 * 16;
+}
+
+// max / min of three.
+BVHGPU_DEV float max3f(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+BVHGPU_DEV float min3f(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+struct PoolRay {
+  float o[3], inv[3], tmax;
+  uint32_t bits;  // code | reverse << 2 | exact << 3
+};
+
+// The traversal's view of a ray record; c: its leaf constants and result slot.
+template <int PROFILE>
+BVHGPU_DEV PoolRay pool_ray(const bvhgpu_ray_t& in, uint32_t slot, float4& c) {
+  const Ray q = make_ray<PROFILE>(in);
+  PoolRay r;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) { r.o[a] = q.o[a]; r.inv[a] = q.inv[a]; }
+  r.tmax = q.tmax;
+  // 1 / direction = 0 (an infinite direction) takes the exact form too: it
+  // would make NaNs of the empty slots' rows.
+  const bool exact = q.exact || q.inv[0] == 0.0f || q.inv[1] == 0.0f || q.inv[2] == 0.0f;
+  r.bits = (uint32_t)q.code | ((q.reverse ? 1u : 0u) << 2) | ((exact ? 1u : 0u) << 3);
+  c = PROFILE == BVHGPU_PROFILE_INSTRUMENTED
+          ? make_float4(q.sx, q.sy, q.sz, __uint_as_float(slot))
+          : make_float4(q.d[0], q.d[1], q.d[2], __uint_as_float(slot));
+  return r;
+}
+
+// Slab test of four boxes given as rows (near and far plane of each axis,
+// four floats each): bit k of the result is set where box k is missed. The
+// booleans are slab_mm's for NaN-free rays and ordered boxes (see visit_node),
+// t0 <= t1 taken from the sign of t1 - t0 (t1 is at most tMax, which is finite,
+// and t0 at least 0, so the difference is no NaN; the +inf / -inf rows of empty
+// slots give a miss).
+BVHGPU_DEV uint32_t miss4(const float4& nx, const float4& ny, const float4& nz, const float4& fx,
+                          const float4& fy, const float4& fz, const PoolRay& r, uint32_t miss) {
+  const uint64_t ox = f2splat(r.o[0]), oy = f2splat(r.o[1]), oz = f2splat(r.o[2]);
+  const uint64_t ix = f2splat(r.inv[0]), iy = f2splat(r.inv[1]), iz = f2splat(r.inv[2]);
+#pragma unroll
+  for (int p = 1; p >= 0; --p) {
+    const int k = 2 * p;
+    const float2 a = f2plane(f4get(nx, k), f4get(nx, k + 1), ox, ix);
+    const float2 b = f2plane(f4get(ny, k), f4get(ny, k + 1), oy, iy);
+    const float2 c = f2plane(f4get(nz, k), f4get(nz, k + 1), oz, iz);
+    const float2 d = f2plane(f4get(fx, k), f4get(fx, k + 1), ox, ix);
+    const float2 e = f2plane(f4get(fy, k), f4get(fy, k + 1), oy, iy);
+    const float2 f = f2plane(f4get(fz, k), f4get(fz, k + 1), oz, iz);
+    const float t0x = fmaxf(max3f(a.x, b.x, c.x), 0.0f), t0y = fmaxf(max3f(a.y, b.y, c.y), 0.0f);
+    const float t1x = fminf(min3f(d.x, e.x, f.x), r.tmax), t1y = fminf(min3f(d.y, e.y, f.y), r.tmax);
+    // + 0 turns the -0 of t1 = -0, t0 = 0 (a hit) into +0.
+    const float2 s = f2unpack(f2add(f2sub(f2pack(t1x, t1y), f2pack(t0x, t0y)), 0ull));
+    miss = __funnelshift_l(__float_as_uint(s.y), miss, 1);
+    miss = __funnelshift_l(__float_as_uint(s.x), miss, 1);
+  }
+  return miss;
+}
+
+// The reference's comparison form for rays that can produce a NaN: same
+// boolean as slab(), one child at a time.
+BVHGPU_DEV bool slab_exact(float lx, float ly, float lz, float hx, float hy, float hz,
+                           const PoolRay& r) {
+  Ray q;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) { q.o[a] = r.o[a]; q.inv[a] = r.inv[a]; }
+  return slab(lx, ly, lz, hx, hy, hz, q, r.tmax);
+}
+
+// Children of node e that the ray hits, bit c for child c.
+template <int NM, int FMT>
+BVHGPU_DEV uint32_t pool_node_hits(const uint8_t* rec, const PoolRay& r) {
+  using F = PackFmt<NM, FMT>;
+  const int nx = r.inv[0] >= 0.0f ? 0 : 3, ny = r.inv[1] >= 0.0f ? 1 : 4;
+  const int nz = r.inv[2] >= 0.0f ? 2 : 5;
+  const int fx = 3 - nx, fy = 5 - ny, fz = 7 - nz;
+  uint32_t miss = 0;
+  if (FMT == kFmtFP32) {
+    if ((r.bits >> 3) & 1u) {
+      const float* b = reinterpret_cast<const float*>(rec);
+      const int count = (int)ldgu(rec + F::COUNT);
+      uint32_t hit = 0;
+      for (int c = 0; c < count; ++c)
+        if (slab_exact(__ldg(b + c), __ldg(b + NM + c), __ldg(b + 2 * NM + c),
+                       __ldg(b + 3 * NM + c), __ldg(b + 4 * NM + c), __ldg(b + 5 * NM + c), r))
+          hit |= 1u << c;
+      return hit;
+    }
+#pragma unroll
+    for (int q = NM / 4 - 1; q >= 0; --q)
+      miss = miss4(ldg4(rec + (nx * NM + 4 * q) * 4), ldg4(rec + (ny * NM + 4 * q) * 4),
+                   ldg4(rec + (nz * NM + 4 * q) * 4), ldg4(rec + (fx * NM + 4 * q) * 4),
+                   ldg4(rec + (fy * NM + 4 * q) * 4), ldg4(rec + (fz * NM + 4 * q) * 4), r, miss);
+    return ~miss & ((1u << NM) - 1u);
+  } else {
+    const uint4 h = ldgu4(rec);
+    const float org[3] = {__uint_as_float(h.x), __uint_as_float(h.y), __uint_as_float(h.z)};
+    const float st[3] = {exp2i((int)(int8_t)(h.w & 0xFFu)), exp2i((int)(int8_t)((h.w >> 8) & 0xFFu)),
+                         exp2i((int)(int8_t)((h.w >> 16) & 0xFFu))};
+    const int count = (int)(h.w >> 24);
+    if ((r.bits >> 3) & 1u) {
+      uint32_t hit = 0;
+      for (int c = 0; c < count; ++c) {
+        float v[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) {
+          const float q = (float)__ldg(rec + F::BOX + a * NM + c) * st[a % 3];
+          v[a] = a < 3 ? __fadd_rd(org[a], q) : __fadd_ru(org[a % 3], q);
+        }
+        if (slab_exact(v[0], v[1], v[2], v[3], v[4], v[5], r)) hit |= 1u << c;
+      }
+      return hit;
+    }
+    const uint8_t* qb = rec + F::BOX;
+#pragma unroll
+    for (int q = NM / 4 - 1; q >= 0; --q) {
+      float4 near[3], far[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const bool up = (a == 0 ? nx : (a == 1 ? ny : nz)) >= 3;
+        const float4 lo = q8_row(ldgu(qb + a * NM + 4 * q), org[a], st[a], false);
+        const float4 hi = q8_row(ldgu(qb + (3 + a) * NM + 4 * q), org[a], st[a], true);
+        near[a] = up ? hi : lo;
+        far[a] = up ? lo : hi;
+      }
+      miss = miss4(near[0], near[1], near[2], far[0], far[1], far[2], r, miss);
+    }
+    return ~miss & ((1u << count) - 1u);
+  }
+}
+
+// Hit children as positions in the push sequence of the ray's major axis.
+template <int NM, int FMT>
+BVHGPU_DEV uint32_t pool_positions(const uint8_t* rec, uint32_t code, uint32_t hit) {
+  using F = PackFmt<NM, FMT>;
+  if (NM <= 8) {
+    // Each hit bit spread to a byte, the bytes permuted by the sequence (its
+    // nibbles are the selectors of the byte permute), and gathered again.
+    const uint32_t seq = ldgu(rec + F::SEQ + 4 * code);
+    const uint32_t lo = ((hit & 15u) * 0x00204081u) & 0x01010101u;
+    const uint32_t hi = NM > 4 ? ((hit >> 4) * 0x00204081u) & 0x01010101u : 0u;
+    const uint32_t p0 = __byte_perm(lo, hi, seq & 0xFFFFu);
+    uint32_t pm = (p0 * 0x01020408u) >> 24;
+    if (NM > 4) {
+      const uint32_t p1 = __byte_perm(lo, hi, seq >> 16);
+      pm |= ((p1 * 0x01020408u) >> 24) << 4;
+    }
+    return pm;
+  }
+  const uint64_t inv = (uint64_t)ldgu(rec + F::SEQ + 8 * code) |
+                       ((uint64_t)ldgu(rec + F::SEQ + 8 * code + 4) << 32);
+  uint32_t pm = 0;
+  while (hit) {
+    const int c = __ffs(hit) - 1;
+    hit &= hit - 1u;
+    pm |= 1u << (uint32_t)((inv >> (4 * c)) & 15u);
+  }
+  return pm;
+}
+
+// One lane's view of its warp's pool.
+template <int NM>
+struct Pool {
+  float4 *a, *b, *c;  // origin, tMax | 1 / direction, bits | leaf constants, result slot
+  uint2* state;       // next entry, stack words in use
+  typename PoolWord<NM>::T* stack;  // [level][ray]
+  uint8_t* list;      // node rays, leaf rays, free slots: kPoolRays each
+  BVHGPU_DEV PoolRay ray(int j) const {
+    const float4 x = a[j], y = b[j];
+    PoolRay r;
+    r.o[0] = x.x; r.o[1] = x.y; r.o[2] = x.z; r.tmax = x.w;
+    r.inv[0] = y.x; r.inv[1] = y.y; r.inv[2] = y.z;
+    r.bits = __float_as_uint(y.w);
+    return r;
+  }
+};
+
+// A ray's next entry: the first of `left` (children of `node` still to visit,
+// non-empty), the others back on the ray's stack (level l at stack[l *
+// stride]). fresh: node is not on the stack yet.
+template <int NM, int FMT, bool ORDERED>
+BVHGPU_DEV uint32_t pool_take(const PoolArgs& p, typename PoolWord<NM>::T* stack, int stride,
+                              uint32_t bits, uint32_t node, uint32_t left, bool fresh,
+                              uint32_t& sp) {
+  using F = PackFmt<NM, FMT>;
+  int k;
+  if (ORDERED && ((bits >> 2) & 1u)) k = 31 - __clz(left);
+  else k = __ffs(left) - 1;
+  left &= ~(1u << k);
+  if (fresh) {
+    if (left) stack[sp++ * stride] = PoolWord<NM>::make(node, left);
+  } else if (left) {
+    stack[(sp - 1) * stride] = PoolWord<NM>::make(node, left);
+  } else {
+    --sp;
+  }
+  const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+  return ldgu(rec + (ORDERED ? F::SORTED + (bits & 3u) * (4 * NM) : F::ENTRY) + 4 * k);
+}
+
+template <bool MM>
+BVHGPU_DEV bool pool_watertight(const float4& t0, const float4& t1, const float4& t2, const Ray& r,
+                                float tmax, float& t, float& b1, float& b2) {
+  // Vertices in the ray's permuted axes (kx, ky, code).
+  float p[3][3];
+  const float v[9] = {t0.x, t0.y, t0.z, t0.w, t1.x, t1.y, t1.z, t1.w, t2.x};
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const float x = v[3 * q], y = v[3 * q + 1], z = v[3 * q + 2];
+    p[q][0] = r.code == 0 ? y : (r.code == 1 ? z : x);
+    p[q][1] = r.code == 0 ? z : (r.code == 1 ? x : y);
+    p[q][2] = r.code == 0 ? x : (r.code == 1 ? y : z);
+  }
+  return watertight<MM, !MM>(p, r, tmax, t, b1, b2);
+}
+
+// Whether Moller-Trumbore certainly rejects a triangle by its first
+// barycentric b1 = n1 * (1 / div): of the other sign than it may have and far
+// from underflow, or well above 1 (comparisons with a NaN are false, so it is
+// left to the full test).
+BVHGPU_DEV bool mt_rejects(float n1, float div) {
+  const float an = fabsf(n1), ad = fabsf(div);
+  const bool neg = (int)(__float_as_uint(n1) ^ __float_as_uint(div)) < 0;
+  return an > ad * (neg ? 1e-30f : 1.0001f);
+}
+
+// One leaf visit: returns whether any triangle was hit. Closest-hit rays
+// lower tmax and write their hit record. First a cheap test of every triangle
+// of the leaf, four at a time (the stored bounds, or the first barycentric
+// without its division), then the full test of the few that pass, so that a
+// warp runs as many full tests as one of its rays needs at most.
+template <int PROFILE, int KIND>
+BVHGPU_DEV bool pool_leaf(const PoolArgs& p, uint32_t e, const PoolRay pr, const float4 c,
+                          float& tmax) {
+  const int cnt = (int)((e >> kLeafCountShift) & 15u) + 1;
+  const float4* blk = p.blocks + (size_t)(e & kLeafIndexMask) * kBlockWords;
+  const uint32_t slot = __float_as_uint(c.w);
+  Ray r;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) { r.o[a] = pr.o[a]; r.inv[a] = pr.inv[a]; }
+  r.code = (int)(pr.bits & 3u);
+  r.kx = r.code == 2 ? 0 : r.code + 1;
+  r.ky = r.code == 0 ? 2 : r.code - 1;
+  bool any = false;
+  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+    r.sx = c.x; r.sy = c.y; r.sz = c.z;
+    const bool exact = (pr.bits >> 3) & 1u;
+    uint32_t pass = (1u << cnt) - 1u;
+    if (!exact) {
+      const int nx = pr.inv[0] >= 0.0f ? 0 : 3, ny = pr.inv[1] >= 0.0f ? 1 : 4;
+      const int nz = pr.inv[2] >= 0.0f ? 2 : 5;
+      const int fx = 3 - nx, fy = 5 - ny, fz = 7 - nz;
+      uint32_t miss = 0;
+      for (int g = (cnt - 1) >> 2; g >= 0; --g) {
+        const float4* b = blk + g * kBlockWords;
+        miss = miss4(__ldg(b + nx), __ldg(b + ny), __ldg(b + nz), __ldg(b + fx), __ldg(b + fy),
+                     __ldg(b + fz), pr, miss);
+      }
+      pass &= ~miss;
+    }
+    while (pass) {
+      const int i = __ffs(pass) - 1;
+      pass &= pass - 1u;
+      const float4* b = blk + (i >> 2) * kBlockWords;
+      if (KIND == BVHGPU_CLOSEST && !exact && tmax != pr.tmax) {
+        // tMax fell in this leaf: the pre-test's tMax condition again.
+        const float* bf = reinterpret_cast<const float*>(b) + (i & 3);
+        float m[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float lo = (__ldg(bf + 4 * a) - r.o[a]) * r.inv[a];
+          const float hi = (__ldg(bf + 4 * (3 + a)) - r.o[a]) * r.inv[a];
+          m[a] = fminf(lo, hi);
+        }
+        if (tmax < fmaxf(fmaxf(m[0], m[1]), m[2])) continue;
+      }
+      const float4* tri = b + kBlockTris + 3 * (i & 3);
+      const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
+      float t, b1, b2;
+      const bool h = exact ? pool_watertight<false>(t0, t1, t2, r, tmax, t, b1, b2)
+                           : pool_watertight<true>(t0, t1, t2, r, tmax, t, b1, b2);
+      if (!h) continue;
+      any = true;
+      if (KIND == BVHGPU_ANY) break;
+      // Each accepted triangle overwrites the hit (triangle.cpp:243).
+      tmax = t;
+      reinterpret_cast<float4*>(p.hits)[slot] = make_float4(t2.y, t, b1, b2);
+    }
+    return any;
+  }
+  // Fast profile: Moller-Trumbore on every triangle; the tie rule of
+  // triIntersect{L} as in visit_leaf_points.
+  r.d[0] = c.x; r.d[1] = c.y; r.d[2] = c.z;
+  uint32_t miss = 0;
+  for (int g = (cnt - 1) >> 2; g >= 0; --g) {
+    const float4* tri = blk + g * kBlockWords + kBlockTris;
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+      const float4 t0 = __ldg(tri + 3 * i), t1 = __ldg(tri + 3 * i + 1), t2 = __ldg(tri + 3 * i + 2);
+      // moller_trumbore()'s divisor and numerator of b1.
+      const float e1x = t0.w - t0.x, e1y = t1.x - t0.y, e1z = t1.y - t0.z;
+      const float e2x = t1.z - t0.x, e2y = t1.w - t0.y, e2z = t2.x - t0.z;
+      const float s1x = r.d[1] * e2z - r.d[2] * e2y;
+      const float s1y = r.d[2] * e2x - r.d[0] * e2z;
+      const float s1z = r.d[0] * e2y - r.d[1] * e2x;
+      const float div = s1x * e1x + s1y * e1y + s1z * e1z;
+      const float n1 = (r.o[0] - t0.x) * s1x + (r.o[1] - t0.y) * s1y + (r.o[2] - t0.z) * s1z;
+      miss = (miss << 1) | (mt_rejects(n1, div) ? 1u : 0u);
+    }
+  }
+  uint32_t pass = ~miss & ((1u << cnt) - 1u);
+  float leaf_best = 1000000.0f, wu = 0.f, wv = 0.f, wprim = 0.f;
+  int winner = -1;
+  uint32_t lanes_at_best = 0;
+  while (pass) {
+    const int i = __ffs(pass) - 1;
+    pass &= pass - 1u;
+    const float4* tri = blk + (i >> 2) * kBlockWords + kBlockTris + 3 * (i & 3);
+    const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
+    const float q[3][3] = {{t0.x, t0.y, t0.z}, {t0.w, t1.x, t1.y}, {t1.z, t1.w, t2.x}};
+    float t, b1, b2;
+    if (!moller_trumbore(q, r, tmax, t, b1, b2)) continue;
+    any = true;
+    if (KIND == BVHGPU_ANY) break;
+    const uint32_t lane_bit = 1u << (i % p.gang);
+    if (t < leaf_best || (winner >= 0 && t == leaf_best && !(lanes_at_best & lane_bit))) {
+      // (a tie keeps the first one's t: it may be a zero of the other sign)
+      lanes_at_best = t < leaf_best ? lane_bit : lanes_at_best | lane_bit;
+      leaf_best = t < leaf_best ? t : leaf_best;
+      winner = i;
+      wu = b1;
+      wv = b2;
+      wprim = t2.y;
+    }
+  }
+  if (KIND == BVHGPU_CLOSEST && winner >= 0) {
+    tmax = leaf_best;
+    reinterpret_cast<float4*>(p.hits)[slot] = make_float4(wprim, leaf_best, wu, wv);
+  }
+  return any;
+}
+
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
+__global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
+    trace_pool_kernel(const __grid_constant__ PoolArgs p) {
+  using F = PackFmt<NM, FMT>;
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  constexpr int K = kPoolRays;
+  extern __shared__ __align__(16) uint8_t pool_smem[];
+  if (p.planned && p.queue[1] != kPlanPool) return;
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned below = (1u << lane) - 1u;
+  using W = PoolWord<NM>;
+  Pool<NM> P;
+  {
+    uint8_t* w = pool_smem + pool_warp_bytes<NM>(p.levels) * (threadIdx.x >> 5);
+    P.a = reinterpret_cast<float4*>(w);
+    P.b = P.a + K;
+    P.c = P.b + K;
+    P.state = reinterpret_cast<uint2*>(P.c + K);
+    P.stack = reinterpret_cast<typename W::T*>(P.state + K);
+    P.list = reinterpret_cast<uint8_t*>(P.stack + (size_t)p.levels * K);
+  }
+  // Lists 0 node rays, 1 leaf rays, 2 free slots; each grows and shrinks at
+  // its end, so rays that went together last stay together.
+  for (int i = (int)lane; i < K; i += 32) P.list[2 * K + i] = (uint8_t)i;
+  int n_node = 0, n_leaf = 0, n_free = p.slots;
+  bool drained = false;
+  __syncwarp();
+
+  while (true) {
+    // The step's rays: one per lane below m. next: the list this lane's ray
+    // goes to (-1: no ray).
+    int next = -1, j = 0, m = 0;
+    if (!drained && n_free >= BVHGPU_POOL_REFILL &&
+        (n_free >= 32 || (n_node < 32 && n_leaf < 32))) {
+      // New rays into free slots.
+      const int want = min(32, n_free);
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(p.queue, (unsigned long long)want);
+      base = __shfl_sync(FULL, base, 0);
+      m = base >= p.n ? 0 : (int)min((unsigned long long)want, p.n - base);
+      drained = base + want >= p.n;
+      n_free -= m;
+      if ((int)lane < m) {
+        j = P.list[2 * K + n_free + lane];
+        const uint32_t i = (uint32_t)base + lane;
+        const uint32_t slot = p.out_index ? __ldg(p.out_index + i) : i;
+        const bvhgpu_ray_t in = load_ray(p.rays, slot);
+        next = 2;
+        if (KIND == BVHGPU_CLOSEST)
+          reinterpret_cast<float4*>(p.hits)[slot] =
+              make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
+        if (!isnan(in.ox)) {
+          float4 c;
+          const PoolRay r = pool_ray<PROFILE>(in, slot, c);
+          P.a[j] = make_float4(r.o[0], r.o[1], r.o[2], r.tmax);
+          P.b[j] = make_float4(r.inv[0], r.inv[1], r.inv[2], __uint_as_float(r.bits));
+          P.c[j] = c;
+          P.state[j] = make_uint2(p.root_entry, 0u);
+          next = (p.root_entry & kLeafBit) ? 1 : 0;
+        } else if (KIND == BVHGPU_ANY) {
+          p.occluded[slot] = 0;
+        }
+      }
+    } else if (n_node >= 32 || (n_node > 0 && n_node >= n_leaf)) {
+      m = min(32, n_node);
+      n_node -= m;
+      if ((int)lane < m) {
+        j = P.list[n_node + (int)lane];
+        const PoolRay r = P.ray(j);
+        const uint2 st = P.state[j];
+        uint32_t node = st.x, sp = st.y;
+        const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+        uint32_t left = pool_node_hits<NM, FMT>(rec, r);
+        const bool fresh = left != 0;
+        if (fresh) {
+          if (ORDERED) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        } else if (sp > 0) {
+          const typename W::T g = P.stack[(sp - 1) * K + j];
+          node = W::node(g);
+          left = W::left(g);
+        }
+        next = 2;
+        if (left) {
+          const uint32_t e = pool_take<NM, FMT, ORDERED>(p, P.stack + j, K, r.bits, node, left,
+                                                         fresh, sp);
+          P.state[j] = make_uint2(e, sp);
+          next = (int)(e >> 31);
+        } else if (KIND == BVHGPU_ANY) {
+          p.occluded[__float_as_uint(P.c[j].w)] = 0;
+        }
+      }
+    } else if (n_leaf > 0) {
+      m = min(32, n_leaf);
+      n_leaf -= m;
+      if ((int)lane < m) {
+        j = P.list[K + n_leaf + (int)lane];
+        const PoolRay r = P.ray(j);
+        const float4 c = P.c[j];
+        const uint2 st = P.state[j];
+        uint32_t sp = st.y;
+        float tmax = r.tmax;
+        const bool hit = pool_leaf<PROFILE, KIND>(p, st.x, r, c, tmax);
+        next = 2;
+        if (KIND == BVHGPU_ANY && hit) {
+          p.occluded[__float_as_uint(c.w)] = 1;
+        } else if (sp > 0) {
+          const typename W::T g = P.stack[(sp - 1) * K + j];
+          const uint32_t e = pool_take<NM, FMT, ORDERED>(p, P.stack + j, K, r.bits, W::node(g),
+                                                         W::left(g), false, sp);
+          P.state[j] = make_uint2(e, sp);
+          if (KIND == BVHGPU_CLOSEST && hit) P.a[j].w = tmax;
+          next = (int)(e >> 31);
+        } else if (KIND == BVHGPU_ANY) {
+          p.occluded[__float_as_uint(c.w)] = 0;
+        }
+      }
+    } else if (drained) {
+      break;
+    }
+    // The step's rays onto their next lists.
+    const unsigned mn = __ballot_sync(FULL, next == 0), ml = __ballot_sync(FULL, next == 1);
+    const unsigned mf = (m == 32 ? FULL : (1u << m) - 1u) & ~(mn | ml);
+    const unsigned mine = next == 0 ? mn : (next == 1 ? ml : mf);
+    const int at = next == 0 ? n_node : (next == 1 ? K + n_leaf : 2 * K + n_free);
+    if (next >= 0) P.list[at + __popc(mine & below)] = (uint8_t)j;
+    n_node += __popc(mn);
+    n_leaf += __popc(ml);
+    n_free += __popc(mf);
+    __syncwarp();
+  }
+}
+
+// Chooses the kernel of a batch by its rays: 64 groups of 32 consecutive rays,
+// spread over the batch, each lane compared with the group's first active ray.
+// Rays that run alike (primary rays of a tile, shadow rays of neighbouring
+// hits) start close to it and point the same way; then one thread per ray
+// keeps most of a warp busy without the pool's lists. Also clears the pool's
+// queue head.
+constexpr int kPlanWarps = 8, kPlanGroups = 8;  // groups per warp
+static __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const bvhgpu_ray_t* rays, uint32_t n,
+                                                               unsigned long long* queue) {
+  __shared__ int votes[2];  // lanes that agree with their group's first ray, active lanes
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  if (threadIdx.x < 2) votes[threadIdx.x] = 0;
+  __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  constexpr uint32_t kGroups = kPlanWarps * kPlanGroups;
+  int agree = 0, active = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kPlanGroups; ++k) {
+    const uint64_t first = (uint64_t)n * (warp * kPlanGroups + k) / kGroups / 32u * 32u;
+    const uint64_t i = first + lane < n ? first + lane : n - 1u;
+    const bvhgpu_ray_t q = load_ray(rays, i);
+    const unsigned live = __ballot_sync(FULL, !isnan(q.ox));
+    if (live == 0) continue;
+    const int lead = __ffs(live) - 1;
+    const float ox = q.ox - __shfl_sync(FULL, q.ox, lead), oy = q.oy - __shfl_sync(FULL, q.oy, lead);
+    const float oz = q.oz - __shfl_sync(FULL, q.oz, lead);
+    const float dx = __shfl_sync(FULL, q.dx, lead), dy = __shfl_sync(FULL, q.dy, lead);
+    const float dz = __shfl_sync(FULL, q.dz, lead), tmax = __shfl_sync(FULL, q.tmax, lead);
+    const float dd = dx * dx + dy * dy + dz * dz;
+    const float qq = q.dx * q.dx + q.dy * q.dy + q.dz * q.dz;
+    const float dot = q.dx * dx + q.dy * dy + q.dz * dz;
+    // Within a twentieth of the ray's length and 18 degrees.
+    const bool same = ox * ox + oy * oy + oz * oz <= 0.0025f * tmax * tmax * dd && dot > 0.0f &&
+                      dot * dot >= 0.9f * dd * qq;
+    agree += __popc(__ballot_sync(FULL, same) & live);
+    active += __popc(live);
+  }
+  if (lane == 0) {
+    atomicAdd(&votes[0], agree);
+    atomicAdd(&votes[1], active);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    queue[0] = 0ull;
+    queue[1] = 4 * votes[0] >= 3 * votes[1] ? kPlanSolo : kPlanPool;
+  }
+}
+
+// One thread per ray on the packed scene, its stack in shared memory
+// ([level][thread]).
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
+__global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
+    trace_solo_kernel(const __grid_constant__ PoolArgs p) {
+  using F = PackFmt<NM, FMT>;
+  using W = PoolWord<NM>;
+  extern __shared__ __align__(16) uint8_t pool_smem[];
+  if (p.planned && p.queue[1] != kPlanSolo) return;
+  typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
+  const int stride = (int)blockDim.x;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= p.n) return;
+  const uint32_t slot = p.out_index ? __ldg(p.out_index + i) : i;
+  const bvhgpu_ray_t in = load_ray(p.rays, slot);
+  if (KIND == BVHGPU_CLOSEST)
+    reinterpret_cast<float4*>(p.hits)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
+  bool hit = false;
+  if (!isnan(in.ox)) {
+    float4 c;
+    PoolRay r = pool_ray<PROFILE>(in, slot, c);
+    uint32_t e = p.root_entry, sp = 0;
+    while (true) {
+      uint32_t node = 0, left = 0;
+      bool fresh = false;
+      bool end = false;
+      while (!(e & kLeafBit)) {
+        node = e;
+        const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+        left = pool_node_hits<NM, FMT>(rec, r);
+        fresh = left != 0;
+        if (fresh) {
+          if (ORDERED) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        } else if (sp > 0) {
+          const typename W::T g = stack[(sp - 1) * stride];
+          node = W::node(g);
+          left = W::left(g);
+        } else {
+          end = true;
+          break;
+        }
+        e = pool_take<NM, FMT, ORDERED>(p, stack, stride, r.bits, node, left, fresh, sp);
+      }
+      if (end) break;
+      float tmax = r.tmax;
+      if (pool_leaf<PROFILE, KIND>(p, e, r, c, tmax)) {
+        hit = true;
+        if (KIND == BVHGPU_ANY) break;
+        r.tmax = tmax;
+      }
+      if (sp == 0) break;
+      const typename W::T g = stack[(sp - 1) * stride];
+      e = pool_take<NM, FMT, ORDERED>(p, stack, stride, r.bits, W::node(g), W::left(g), false, sp);
+    }
+  }
+  if (KIND == BVHGPU_ANY) p.occluded[slot] = hit ? 1 : 0;
+}
+
+}  // namespace dev
+}  // namespace bvhgpu

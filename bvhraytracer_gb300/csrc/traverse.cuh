@@ -41,8 +41,9 @@ struct SceneDev {
   // NodeFmt<N>::NM stack entries per inner node, one per child slot (null:
   // computed from the record).
   const uint32_t* child_entry = nullptr;
-  // 6 * leaf_memory floats per leaf: each triangle slot's vertex minima
-  // (rows 0-2) and maxima (rows 3-5) per axis (read when BVHGPU_LEAF_BOUNDS).
+  // Packed leaf records (pack.cuh), 6 * leaf_memory + 4 floats per leaf: each
+  // triangle slot's vertex minima (rows 0-2) and maxima (rows 3-5) per axis
+  // (read when BVHGPU_LEAF_BOUNDS).
   const float* leaf_bounds = nullptr;
 };
 
@@ -629,7 +630,7 @@ BVHGPU_DEV bool visit_leaf_bounds(const SceneDev& sc, uint32_t e, const Ray& r, 
   bool any = false;
   const int ax0 = r.kx, ax1 = r.ky, ax2 = r.code;
   const int lm = sc.leaf_memory;
-  const float* bnd = sc.leaf_bounds + (size_t)leaf * 6 * lm;
+  const float* bnd = sc.leaf_bounds + (size_t)leaf * (6 * lm + 4);
   if ((BVHGPU_LEAF_COMPACT >= 1 && KIND == BVHGPU_ANY) || BVHGPU_LEAF_COMPACT >= 2) {
     // Every pre-test of the leaf first, with the tMax the ray enters the
     // leaf with: a mask of the triangles that pass, then the full tests of

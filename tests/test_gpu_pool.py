@@ -1,0 +1,120 @@
+"""The ray-pool kernel and the choice between it and one thread per ray:
+results equal, bit for bit, to the counting kernels' (which are checked
+against the oracle elsewhere) at the sizes where the choice changes, for every
+node width and format, both profiles and ray kinds, and for rays that take the
+exact forms."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import bvhraytracer_gb300 as pkg  # noqa: E402
+from bvhraytracer_gb300 import scenes as S  # noqa: E402
+from tests import _scenes as TS  # noqa: E402
+from tests.test_gpu_histograms import _chain  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+LINE = 1 << 18  # more rays than this may run on the pool kernel
+
+
+def _rays(tris, n, seed, extreme=False):
+    """Incoherent rays between points of the scene's box; every fourth short,
+    some inactive."""
+    rng = np.random.default_rng(seed)
+    p = tris.reshape(-1, 3)
+    lo, hi = p.min(0), p.max(0)
+    r = np.zeros((n, 8), np.float32)
+    r[:, 0:3] = rng.uniform(lo, hi, (n, 3))
+    r[:, 4:7] = rng.normal(size=(n, 3))
+    r[:, 3] = np.where(np.arange(n) % 4 == 0, 0.05 * np.linalg.norm(hi - lo), 1e4)
+    r[rng.integers(0, n, 50), 0] = np.nan
+    if extreme:
+        vals = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1e-40, 3e38, 1e-20], np.float32)
+        at = rng.integers(0, n, 4000)
+        r[at, rng.integers(3, 7, 4000)] = vals[rng.integers(0, 8, 4000)]
+    return torch.from_numpy(r).cuda()
+
+
+def _same(scene, rays, **kw):
+    for kind in ("closest", "any"):
+        key = "hits" if kind == "closest" else "occluded"
+        for profile in ("instrumented", "fast"):
+            want = scene.trace(rays, kind=kind, profile=profile, counters=True)[key]
+            for order in ({}, {"any_order": True}) if kind == "any" else ({},):
+                got = scene.trace(rays, kind=kind, profile=profile, **kw, **order)[key]
+                a, b = got.view(torch.uint8), want.view(torch.uint8)
+                if kind == "closest":  # a NaN of a degenerate ray matches any NaN
+                    a = torch.where(torch.isnan(got[:, 1:]), 0.0, got[:, 1:]).view(torch.int32)
+                    b = torch.where(torch.isnan(want[:, 1:]), 0.0, want[:, 1:]).view(torch.int32)
+                    assert torch.equal(got.view(torch.int32)[:, 0], want.view(torch.int32)[:, 0])
+                assert torch.equal(a, b), (kind, profile, kw, order)
+    scene.status()
+
+
+@pytest.mark.parametrize("n,l,fmt", [(2, 1, "fp32"), (4, 4, "fp32"), (5, 7, "q8"), (8, 8, "fp32"),
+                                     (8, 4, "q8"), (9, 13, "fp32"), (12, 16, "q8"),
+                                     (16, 16, "fp32"), (16, 5, "q8")])
+def test_pool_equals_counting_kernel(n, l, fmt):
+    tris = S.clutter(30, 2)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    rays = _rays(tris, LINE + 1, n * 16 + l, extreme=True)
+    _same(scene, rays)               # the rays' own choice: the pool
+    _same(scene, rays, reorder=3)    # direction order: the pool
+    _same(scene, rays[:LINE])        # one thread per ray
+
+
+@pytest.mark.parametrize("n", [LINE + 1, LINE + 31, 1000003])
+def test_rays_that_stay_together(n):
+    tris = S.clutter(30, 2)
+    scene = pkg.Scene(pkg.Bvh(tris, 8, 8))
+    cam, target, _ = S.clutter_viewpoints(30, 2)
+    rays = pkg.camera_rays(cam, target, 1024, 1024)[:n].contiguous()
+    _same(scene, rays)
+    _same(scene, rays, scheme="persistent", policy=4, refill=3)
+
+
+def test_root_leaf_deep_tree_and_inactive_batch():
+    one = np.array([[0, 0, 0, 1, 0, 0, 0, 1, 0]], np.float32)
+    _same(pkg.Scene(pkg.Bvh(one, 8, 8)), _rays(np.array([[-1, -1, -1, 1, 1, 1, 0, 0, 0]]), LINE + 5, 1))
+    deep = pkg.Scene(_chain(2, 60, 2))  # more levels than the pool's stacks
+    _same(deep, _rays(np.array([[0, 0, 0, 1, 1, 1, 0, 0, 0]]), LINE + 5, 2))
+    tris = S.clutter(30, 2)
+    rays = _rays(tris, LINE + 64, 3)
+    rays[:, 0] = float("nan")
+    _same(pkg.Scene(pkg.Bvh(tris, 4, 4)), rays)
+
+
+def test_unordered_boxes_take_the_general_kernels():
+    tris, bvh, _ = TS.bvh("clutter120", 8, 4)
+    arrays = bvh.export_compact()
+    arrays["lo3"] = arrays["lo3"].copy()
+    leaf = np.flatnonzero(arrays["child_count"] == 0)[:5]
+    arrays["lo3"][leaf, 0] = np.inf
+    scene = pkg.Scene(pkg.Bvh.from_compact(arrays, 8, 4))
+    _same(scene, _rays(tris, LINE + 1, 4))
+
+
+def test_captured_and_concurrent_traces():
+    tris = S.clutter(60, 2)
+    scene = pkg.Scene(pkg.Bvh(tris, 8, 8))
+    rays = _rays(tris, LINE + 1000, 5)
+    want = scene.trace(rays, kind="any", counters=True)["occluded"]
+    out = torch.full_like(want, 7)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        scene.trace(rays, kind="any", out=out)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    # more launches in flight than any ring of slots could hold
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    outs = []
+    for k in range(160):
+        with torch.cuda.stream(streams[k % 4]):
+            outs.append(scene.trace(rays, kind="any")["occluded"])
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs)
+    scene.status()
