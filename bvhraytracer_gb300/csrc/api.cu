@@ -18,6 +18,7 @@
 #include "bvhgpu_status.hpp"
 #include "launch.cuh"
 #include "pack.cuh"
+#include "pool_launch.cuh"
 #include "reorder.cuh"
 #include "raygen.cuh"
 #include "q8_encode.cuh"
@@ -260,13 +261,16 @@ static cudaError_t pack_scene(bvhgpu_scene* s) {
 // staging wait of the failure-detection tests, node records whose boxes are
 // not ordered (imported trees), trees too deep or large for its stack words,
 // and more than 2^32 - 1 rays.
-static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
+static bool scene_uses_pool(const bvhgpu_scene* s) {
   const DeviceLayout& L = s->layout;
-  return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) &&
-         stack_cap(s) >= s->max_stack && s->stall_bytes == 0 && a.n <= 0xFFFFFFFFull &&
+  return stack_cap(s) >= s->max_stack && s->stall_bytes == 0 &&
          (L.node_format != BVHGPU_NODES_FP32 || L.boxes_ordered) &&
          L.n_inner < dev::pool_max_inner(L.node_stride) && L.inner_levels <= kPoolMaxLevels &&
          L.leaf_block[L.n_leaves] <= dev::kMaxBlocks;
+}
+static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
+  return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&
+         scene_uses_pool(s);
 }
 
 // Stream-ordered scratch (reorder passes, queues) comes from a memory pool of
@@ -300,47 +304,54 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
   return e == cudaSuccess ? BVHGPU_OK : set_error(BVHGPU_ERR_OOM, "scratch allocation failed");
 }
 
-// A trace on the packed scene. A large batch needs two words of device memory
-// of its own while it runs: the caller's (c.pool_queue) or stream-ordered
-// scratch. A stream that is being captured gets none (an allocation would put
-// memory nodes into the caller's graph), nor does a full device: then every
-// ray has its own thread.
-static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
-                               cudaStream_t st) {
-  dev::PoolArgs p;
-  p.nodes = s->d_pack_nodes;
-  p.blocks = s->d_pack_blocks;
-  p.root_entry = s->pack_root;
-  p.gang = s->layout.gang;
-  p.levels = std::max(1, s->layout.inner_levels);
-  p.rays = a.rays;
-  p.n = (uint32_t)a.n;
-  p.hits = a.hits;
-  p.occluded = a.occluded;
-  p.out_index = a.out_index;
-  p.queue = c.pool_queue;
+// Two words of device memory for a large launch on the packed scene: the
+// caller's or stream-ordered scratch, freed behind the launch. A stream that is
+// being captured gets none (an allocation would put memory nodes into the
+// caller's graph), nor does a full device: then every ray has its own thread.
+struct PoolQueue {
+  unsigned long long* words = nullptr;
   void* scratch = nullptr;
-  if (!p.queue && dev::pool_wants_queue(a.n)) {
+  PoolQueue(int device, uint64_t n, unsigned long long* given, cudaStream_t st) : words(given) {
+    if (given || !dev::pool_wants_queue(n)) return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
     if (cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone &&
-        scratch_alloc(s->device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
-      p.queue = static_cast<unsigned long long*>(scratch);
+        scratch_alloc(device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
+      words = static_cast<unsigned long long*>(scratch);
     else
       cudaGetLastError();
   }
+  cudaError_t free(cudaStream_t st) {
+    return scratch ? cudaFreeAsync(scratch, st) : cudaSuccess;
+  }
+};
+
+static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
+  return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root, s->layout.gang};
+}
+
+// A trace on the packed scene.
+static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
+                               cudaStream_t st) {
+  PoolQueue queue(s->device, a.n, c.pool_queue, st);
+  dev::OneScene p{};
+  p.n = a.n;
+  p.levels = std::max(1, s->layout.inner_levels);
+  p.queue = queue.words;
+  p.scene = pack_view(s, c.kind == BVHGPU_ANY ? (void*)a.occluded : (void*)a.hits);
+  p.rays = a.rays;
+  p.out_index = a.out_index;
+  const dev::PackedCfg cfg{s->layout.node_stride, s->layout.node_format, c.kind, c.profile,
+                           c.any_order, a.out_index != nullptr, s->sm_count};
   cudaError_t e;
-  switch (s->layout.node_stride) {
-    case 4: e = dev::launch_pool_n4(p, c, st); break;
-    case 8: e = dev::launch_pool_n8(p, c, st); break;
-    case 12: e = dev::launch_pool_n12(p, c, st); break;
-    default: e = dev::launch_pool_n16(p, c, st); break;
+  switch (cfg.nm) {
+    case 4: e = dev::launch_one_scene<4>(p, cfg, st); break;
+    case 8: e = dev::launch_one_scene<8>(p, cfg, st); break;
+    case 12: e = dev::launch_one_scene<12>(p, cfg, st); break;
+    default: e = dev::launch_one_scene<16>(p, cfg, st); break;
   }
-  if (scratch) {
-    const cudaError_t f = cudaFreeAsync(scratch, st);
-    if (e == cudaSuccess) e = f;
-  }
-  return e;
+  const cudaError_t f = queue.free(st);
+  return e == cudaSuccess ? f : e;
 }
 
 static int launch(bvhgpu_scene_t s, const dev::TraceArgs& a, dev::LaunchCfg cfg,
@@ -1088,6 +1099,64 @@ extern "C" {
 #define BVHGPU_JOBS_SPLIT 2
 #endif
 
+}  // extern "C"
+
+// The jobs on their packed scenes, in groups of one node width and format, ray
+// kind, push order and ray order: a launch's kernel is compiled for what its
+// jobs have in common. t: the job table (jobs with rays, in order; perm set).
+static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, const dev::JobTable& t,
+                                      int profile, int device, int sms, cudaStream_t st) {
+  static_assert(dev::kPoolMaxJobs == dev::kMaxJobs, "job limit");
+  std::unique_ptr<dev::ManyScenes> p(new (std::nothrow) dev::ManyScenes());
+  if (!p) return cudaErrorMemoryAllocation;
+  std::vector<dev::PackedCfg> cfg;
+  std::vector<int> group;  // of each job of the table
+  for (int i = 0, k = 0; i < n_jobs; ++i) {
+    if (jobs[i].n == 0) continue;
+    const dev::JobDev& d = t.jobs[k++];
+    const dev::PackedCfg c{d.nm, d.fmt, d.kind, profile, d.kind == BVHGPU_ANY && d.any_index_order,
+                           d.perm != nullptr, sms};
+    size_t g = 0;
+    while (g < cfg.size() && !(cfg[g].nm == c.nm && cfg[g].fmt == c.fmt && cfg[g].kind == c.kind &&
+                               cfg[g].any_order == c.any_order &&
+                               cfg[g].direction_order == c.direction_order))
+      ++g;
+    if (g == cfg.size()) cfg.push_back(c);
+    group.push_back((int)g);
+  }
+  for (size_t g = 0; g < cfg.size(); ++g) {
+    p->n = 0;
+    p->n_jobs = 0;
+    p->levels = 1;
+    for (int i = 0, k = 0; i < n_jobs; ++i) {
+      if (jobs[i].n == 0) continue;
+      const dev::JobDev& d = t.jobs[k];
+      if (group[k++] != (int)g) continue;
+      dev::PoolJob& j = p->jobs[p->n_jobs++];
+      j.scene = pack_view(jobs[i].scene, d.out);
+      j.rays = d.rays;
+      j.out_index = d.perm;
+      j.begin = p->n;
+      p->n += d.n;
+      p->levels = std::max(p->levels, jobs[i].scene->layout.inner_levels);
+    }
+    PoolQueue queue(device, p->n, nullptr, st);
+    p->queue = queue.words;
+    cudaError_t e;
+    switch (cfg[g].nm) {
+      case 4: e = dev::launch_many_scenes<4>(*p, cfg[g], st); break;
+      case 8: e = dev::launch_many_scenes<8>(*p, cfg[g], st); break;
+      case 12: e = dev::launch_many_scenes<12>(*p, cfg[g], st); break;
+      default: e = dev::launch_many_scenes<16>(*p, cfg[g], st); break;
+    }
+    const cudaError_t f = queue.free(st);
+    if (e != cudaSuccess || f != cudaSuccess) return e != cudaSuccess ? e : f;
+  }
+  return cudaSuccess;
+}
+
+extern "C" {
+
 int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_trace_opts_t* opts,
                       void* stream) {
   if (n_jobs < 0 || n_jobs > dev::kMaxJobs)
@@ -1192,6 +1261,17 @@ int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_tra
       cudaFreeAsync(scratch, st);
       return cuda_error(e, "job reorder");
     }
+  }
+  bool packed = true;
+  for (int i = 0; i < n_jobs; ++i)
+    if (jobs[i].n != 0 && !scene_uses_pool(jobs[i].scene)) packed = false;
+  if (packed) {
+    e = launch_packed_jobs(jobs, n_jobs, *t, cfg.profile, device, sms, st);
+    if (scratch) {
+      cudaError_t f = cudaFreeAsync(scratch, st);
+      if (e == cudaSuccess) e = f;
+    }
+    return e == cudaSuccess ? BVHGPU_OK : cuda_error(e, "batched launch");
   }
   // Jobs run in groups of one ray kind (BVHGPU_JOBS_SPLIT 1), or of one ray
   // kind and node width and format (2), one persistent launch per group on

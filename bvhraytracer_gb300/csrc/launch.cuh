@@ -2,7 +2,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "pool.cuh"
 #include "traverse.cuh"
 
 namespace bvhgpu {
@@ -22,7 +21,7 @@ struct LaunchCfg {
   unsigned long long* queue = nullptr;  // persistent scheme: queue head
   bool queue_cleared = false;  // true: the caller zeroed the head already
   // Packed scene: two words of device memory for this launch alone (null: it
-  // may take them from the stream, see launch_pool).
+  // may take them from the stream, see PoolQueue in api.cu).
   unsigned long long* pool_queue = nullptr;
   int sm_count = 152;
   int fmt = BVHGPU_NODES_FP32;  // node record format of the scene
@@ -139,85 +138,6 @@ inline cudaError_t launch_for_width(const SceneDev& sc, const TraceArgs& a, cons
   return cudaErrorInvalidValue;
 }
 
-// Shared memory of an SM that the pools may take; the rest of its 256 KB is
-// L1, which the node records need.
-#ifndef BVHGPU_POOL_SMEM
-#define BVHGPU_POOL_SMEM (196 * 1024)
-#endif
-// Rays per resident warp from which a warp takes kPoolRays rays at once.
-#ifndef BVHGPU_POOL_FULL
-#define BVHGPU_POOL_FULL 48
-#endif
-// Batches of more rays may run on the pool kernel. Solo / pool, us: unordered
-// ambient-occlusion rays (N8L8, 251k triangles) 131k rays 110 / 115, 262k
-// 172 / 146, 1M 558 / 365, 4.2M 1953 / 1134; primary rays, which stay
-// together, 262k 124 / 148, 1M 253 / 290. The lines cross at about 200k rays
-// for rays that part and nowhere for rays that do not.
-#ifndef BVHGPU_POOL_MIN_RAYS
-#define BVHGPU_POOL_MIN_RAYS (1u << 18)
-#endif
-inline bool pool_wants_queue(uint64_t n) { return n > BVHGPU_POOL_MIN_RAYS; }
-constexpr int kSoloBlock = 64;
-
-template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
-inline cudaError_t launch_packed(PoolArgs& p, const LaunchCfg& cfg, cudaStream_t s) {
-  cudaError_t e;
-  const bool large = pool_wants_queue(p.n) && p.queue != nullptr;
-  // Rays in direction order are for the pool; otherwise the rays themselves
-  // decide.
-  const bool pool = large && p.out_index != nullptr;
-  p.planned = large && !pool;
-  if (p.planned) {
-    plan_kernel<<<1, kPlanWarps * 32, 0, s>>>(p.rays, p.n, p.queue);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  if (!pool) {
-    auto k = trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED>;
-    const size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * kSoloBlock;
-    const uint64_t grid = ((uint64_t)p.n + kSoloBlock - 1) / kSoloBlock;
-    k<<<(unsigned)grid, kSoloBlock, smem, s>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess || !large) return e;
-  }
-  auto k = trace_pool_kernel<NM, PROFILE, KIND, FMT, ORDERED>;
-  const size_t smem = kPoolWarps * pool_warp_bytes<NM>(p.levels);
-  if ((e = set_smem(k, smem)) != cudaSuccess) return e;
-  // Resident warps; blocks past them would find the queue empty.
-  const size_t fit = BVHGPU_POOL_SMEM / smem;
-  const uint64_t per_sm = fit < 1 ? 1 : fit > BVHGPU_POOL_MIN_BLOCKS ? BVHGPU_POOL_MIN_BLOCKS : fit;
-  const uint64_t warps = (uint64_t)cfg.sm_count * per_sm * kPoolWarps;
-  p.slots = p.n >= warps * BVHGPU_POOL_FULL ? kPoolRays : 32;
-  const uint64_t need = ((uint64_t)p.n + kPoolWarps * 32 - 1) / (kPoolWarps * 32);
-  const uint64_t grid = need < warps / kPoolWarps ? need : warps / kPoolWarps;
-  if (!p.planned) {
-    e = cudaMemsetAsync(p.queue, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-  }
-  k<<<(unsigned)grid, kPoolWarps * 32, smem, s>>>(p);
-  return cudaGetLastError();
-}
-
-template <int NM, int FMT>
-inline cudaError_t launch_pool_fmt(PoolArgs& p, const LaunchCfg& c, cudaStream_t s) {
-  constexpr int F = BVHGPU_PROFILE_FAST, I = BVHGPU_PROFILE_INSTRUMENTED;
-  if (c.kind == BVHGPU_CLOSEST)
-    return c.profile == F ? launch_packed<NM, F, BVHGPU_CLOSEST, FMT, true>(p, c, s)
-                          : launch_packed<NM, I, BVHGPU_CLOSEST, FMT, true>(p, c, s);
-  if (c.profile == F) return launch_packed<NM, F, BVHGPU_ANY, FMT, false>(p, c, s);
-  return c.any_order ? launch_packed<NM, I, BVHGPU_ANY, FMT, false>(p, c, s)
-                     : launch_packed<NM, I, BVHGPU_ANY, FMT, true>(p, c, s);
-}
-
-template <int NM>
-inline cudaError_t launch_pool_for_width(PoolArgs p, const LaunchCfg& c, cudaStream_t s) {
-  if (p.n == 0) return cudaSuccess;
-  return c.fmt == kFmtQ8 ? launch_pool_fmt<NM, kFmtQ8>(p, c, s)
-                         : launch_pool_fmt<NM, kFmtFP32>(p, c, s);
-}
-
-cudaError_t launch_pool_n4(const PoolArgs&, const LaunchCfg&, cudaStream_t);
-cudaError_t launch_pool_n8(const PoolArgs&, const LaunchCfg&, cudaStream_t);
-cudaError_t launch_pool_n12(const PoolArgs&, const LaunchCfg&, cudaStream_t);
-cudaError_t launch_pool_n16(const PoolArgs&, const LaunchCfg&, cudaStream_t);
 cudaError_t launch_trace_n4(const SceneDev&, const TraceArgs&, const LaunchCfg&, cudaStream_t);
 cudaError_t launch_trace_n8(const SceneDev&, const TraceArgs&, const LaunchCfg&, cudaStream_t);
 cudaError_t launch_trace_n12(const SceneDev&, const TraceArgs&, const LaunchCfg&, cudaStream_t);

@@ -55,22 +55,66 @@ constexpr int kPoolWarps = 4;  // per block
 #define BVHGPU_SOLO_MIN_BLOCKS 4
 #endif
 
-struct PoolArgs {
-  const uint8_t* nodes;   // packed node records (PackFmt)
-  const float4* blocks;   // leaf blocks
-  uint32_t root_entry;    // stack entries of the packed records
+// What a ray's visits need of its scene, and where its result goes.
+struct PackView {
+  const uint8_t* nodes;  // packed node records (PackFmt)
+  const float4* blocks;  // leaf blocks
+  void* out;             // hits or occlusion bytes
+  uint32_t root;         // stack entry of the root
   int gang;
-  int levels;             // inner levels of the tree: words of a ray's stack
-  const bvhgpu_ray_t* rays;
-  uint32_t n;
-  bvhgpu_hit_t* hits;
-  uint8_t* occluded;
-  const uint32_t* out_index;  // as TraceArgs
+};
+
+// Common arguments of a launch.
+struct PoolArgs {
+  uint64_t n;   // rays
+  int levels;   // inner levels of the deepest tree: words of a ray's stack
   // Two words of this launch's own: [0] next unclaimed ray of the pool kernel,
   // [1] the kernel chosen by plan_kernel. Null: one thread per ray.
   unsigned long long* queue;
-  int planned;                // 1: a kernel other than the chosen one returns at once
-  int slots;                  // rays a warp takes at once (32 or kPoolRays)
+  int planned;  // 1: a kernel other than the chosen one returns at once
+  int slots;    // rays a warp takes at once (32 or kPoolRays)
+};
+
+// A batch of rays of one scene.
+struct OneScene : PoolArgs {
+  PackView scene;
+  const bvhgpu_ray_t* rays;
+  const uint32_t* out_index;  // as TraceArgs
+  BVHGPU_DEV const PackView& view(uint32_t) const { return scene; }
+  // The i-th ray of the launch, its result slot and its job.
+  BVHGPU_DEV bvhgpu_ray_t ray(uint64_t i, uint32_t& slot, uint32_t& job) const {
+    job = 0;
+    slot = out_index ? __ldg(out_index + i) : (uint32_t)i;
+    return load_ray(rays, slot);
+  }
+};
+
+// Batches of several scenes, one after the other.
+constexpr int kPoolMaxJobs = 192;
+struct PoolJob {
+  PackView scene;
+  const bvhgpu_ray_t* rays;
+  const uint32_t* out_index;
+  uint64_t begin;  // the job's first ray in the launch
+};
+struct ManyScenes : PoolArgs {
+  int n_jobs;
+  PoolJob jobs[kPoolMaxJobs];
+  BVHGPU_DEV const PackView& view(uint32_t job) const { return jobs[job].scene; }
+  BVHGPU_DEV bvhgpu_ray_t ray(uint64_t i, uint32_t& slot, uint32_t& job) const {
+    // The last job that begins at or before ray i.
+    int lo = 0, hi = n_jobs - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (jobs[mid].begin <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    job = (uint32_t)lo;
+    const PoolJob& J = jobs[lo];
+    slot = (uint32_t)(i - J.begin);
+    if (J.out_index) slot = __ldg(J.out_index + slot);
+    return load_ray(J.rays, slot);
+  }
 };
 
 // Which of the two kernels traces a batch.
@@ -117,7 +161,7 @@ BVHGPU_DEV float min3f(float a, float b, float c) {
 
 struct PoolRay {
   float o[3], inv[3], tmax;
-  uint32_t bits;  // code | reverse << 2 | exact << 3
+  uint32_t bits;  // code | reverse << 2 | exact << 3 | job << 4
 };
 
 // The traversal's view of a ray record; c: its leaf constants and result slot.
@@ -289,7 +333,7 @@ struct Pool {
 // non-empty), the others back on the ray's stack (level l at stack[l *
 // stride]). fresh: node is not on the stack yet.
 template <int NM, int FMT, bool ORDERED>
-BVHGPU_DEV uint32_t pool_take(const PoolArgs& p, typename PoolWord<NM>::T* stack, int stride,
+BVHGPU_DEV uint32_t pool_take(const PackView& v, typename PoolWord<NM>::T* stack, int stride,
                               uint32_t bits, uint32_t node, uint32_t left, bool fresh,
                               uint32_t& sp) {
   using F = PackFmt<NM, FMT>;
@@ -304,7 +348,7 @@ BVHGPU_DEV uint32_t pool_take(const PoolArgs& p, typename PoolWord<NM>::T* stack
   } else {
     --sp;
   }
-  const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+  const uint8_t* rec = v.nodes + (size_t)node * F::REC;
   return ldgu(rec + (ORDERED ? F::SORTED + (bits & 3u) * (4 * NM) : F::ENTRY) + 4 * k);
 }
 
@@ -340,10 +384,10 @@ BVHGPU_DEV bool mt_rejects(float n1, float div) {
 // without its division), then the full test of the few that pass, so that a
 // warp runs as many full tests as one of its rays needs at most.
 template <int PROFILE, int KIND>
-BVHGPU_DEV bool pool_leaf(const PoolArgs& p, uint32_t e, const PoolRay pr, const float4 c,
+BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const float4 c,
                           float& tmax) {
   const int cnt = (int)((e >> kLeafCountShift) & 15u) + 1;
-  const float4* blk = p.blocks + (size_t)(e & kLeafIndexMask) * kBlockWords;
+  const float4* blk = v.blocks + (size_t)(e & kLeafIndexMask) * kBlockWords;
   const uint32_t slot = __float_as_uint(c.w);
   Ray r;
 #pragma unroll
@@ -394,7 +438,7 @@ BVHGPU_DEV bool pool_leaf(const PoolArgs& p, uint32_t e, const PoolRay pr, const
       if (KIND == BVHGPU_ANY) break;
       // Each accepted triangle overwrites the hit (triangle.cpp:243).
       tmax = t;
-      reinterpret_cast<float4*>(p.hits)[slot] = make_float4(t2.y, t, b1, b2);
+      static_cast<float4*>(v.out)[slot] = make_float4(t2.y, t, b1, b2);
     }
     return any;
   }
@@ -432,7 +476,7 @@ BVHGPU_DEV bool pool_leaf(const PoolArgs& p, uint32_t e, const PoolRay pr, const
     if (!moller_trumbore(q, r, tmax, t, b1, b2)) continue;
     any = true;
     if (KIND == BVHGPU_ANY) break;
-    const uint32_t lane_bit = 1u << (i % p.gang);
+    const uint32_t lane_bit = 1u << (i % v.gang);
     if (t < leaf_best || (winner >= 0 && t == leaf_best && !(lanes_at_best & lane_bit))) {
       // (a tie keeps the first one's t: it may be a zero of the other sign)
       lanes_at_best = t < leaf_best ? lane_bit : lanes_at_best | lane_bit;
@@ -445,14 +489,14 @@ BVHGPU_DEV bool pool_leaf(const PoolArgs& p, uint32_t e, const PoolRay pr, const
   }
   if (KIND == BVHGPU_CLOSEST && winner >= 0) {
     tmax = leaf_best;
-    reinterpret_cast<float4*>(p.hits)[slot] = make_float4(wprim, leaf_best, wu, wv);
+    static_cast<float4*>(v.out)[slot] = make_float4(wprim, leaf_best, wu, wv);
   }
   return any;
 }
 
-template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
 __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
-    trace_pool_kernel(const __grid_constant__ PoolArgs p) {
+    trace_pool_kernel(const __grid_constant__ SRC p) {
   using F = PackFmt<NM, FMT>;
   constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int K = kPoolRays;
@@ -494,23 +538,23 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
       n_free -= m;
       if ((int)lane < m) {
         j = P.list[2 * K + n_free + lane];
-        const uint32_t i = (uint32_t)base + lane;
-        const uint32_t slot = p.out_index ? __ldg(p.out_index + i) : i;
-        const bvhgpu_ray_t in = load_ray(p.rays, slot);
+        uint32_t slot, job;
+        const bvhgpu_ray_t in = p.ray(base + lane, slot, job);
+        const PackView& v = p.view(job);
         next = 2;
         if (KIND == BVHGPU_CLOSEST)
-          reinterpret_cast<float4*>(p.hits)[slot] =
-              make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
+          static_cast<float4*>(v.out)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
         if (!isnan(in.ox)) {
           float4 c;
-          const PoolRay r = pool_ray<PROFILE>(in, slot, c);
+          PoolRay r = pool_ray<PROFILE>(in, slot, c);
+          r.bits |= job << 4;
           P.a[j] = make_float4(r.o[0], r.o[1], r.o[2], r.tmax);
           P.b[j] = make_float4(r.inv[0], r.inv[1], r.inv[2], __uint_as_float(r.bits));
           P.c[j] = c;
-          P.state[j] = make_uint2(p.root_entry, 0u);
-          next = (p.root_entry & kLeafBit) ? 1 : 0;
+          P.state[j] = make_uint2(v.root, 0u);
+          next = (v.root & kLeafBit) ? 1 : 0;
         } else if (KIND == BVHGPU_ANY) {
-          p.occluded[slot] = 0;
+          static_cast<uint8_t*>(v.out)[slot] = 0;
         }
       }
     } else if (n_node >= 32 || (n_node > 0 && n_node >= n_leaf)) {
@@ -519,9 +563,10 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
       if ((int)lane < m) {
         j = P.list[n_node + (int)lane];
         const PoolRay r = P.ray(j);
+        const PackView& v = p.view(r.bits >> 4);
         const uint2 st = P.state[j];
         uint32_t node = st.x, sp = st.y;
-        const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+        const uint8_t* rec = v.nodes + (size_t)node * F::REC;
         uint32_t left = pool_node_hits<NM, FMT>(rec, r);
         const bool fresh = left != 0;
         if (fresh) {
@@ -533,12 +578,12 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
         }
         next = 2;
         if (left) {
-          const uint32_t e = pool_take<NM, FMT, ORDERED>(p, P.stack + j, K, r.bits, node, left,
+          const uint32_t e = pool_take<NM, FMT, ORDERED>(v, P.stack + j, K, r.bits, node, left,
                                                          fresh, sp);
           P.state[j] = make_uint2(e, sp);
           next = (int)(e >> 31);
         } else if (KIND == BVHGPU_ANY) {
-          p.occluded[__float_as_uint(P.c[j].w)] = 0;
+          static_cast<uint8_t*>(v.out)[__float_as_uint(P.c[j].w)] = 0;
         }
       }
     } else if (n_leaf > 0) {
@@ -547,23 +592,24 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
       if ((int)lane < m) {
         j = P.list[K + n_leaf + (int)lane];
         const PoolRay r = P.ray(j);
+        const PackView& v = p.view(r.bits >> 4);
         const float4 c = P.c[j];
         const uint2 st = P.state[j];
         uint32_t sp = st.y;
         float tmax = r.tmax;
-        const bool hit = pool_leaf<PROFILE, KIND>(p, st.x, r, c, tmax);
+        const bool hit = pool_leaf<PROFILE, KIND>(v, st.x, r, c, tmax);
         next = 2;
         if (KIND == BVHGPU_ANY && hit) {
-          p.occluded[__float_as_uint(c.w)] = 1;
+          static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 1;
         } else if (sp > 0) {
           const typename W::T g = P.stack[(sp - 1) * K + j];
-          const uint32_t e = pool_take<NM, FMT, ORDERED>(p, P.stack + j, K, r.bits, W::node(g),
+          const uint32_t e = pool_take<NM, FMT, ORDERED>(v, P.stack + j, K, r.bits, W::node(g),
                                                          W::left(g), false, sp);
           P.state[j] = make_uint2(e, sp);
           if (KIND == BVHGPU_CLOSEST && hit) P.a[j].w = tmax;
           next = (int)(e >> 31);
         } else if (KIND == BVHGPU_ANY) {
-          p.occluded[__float_as_uint(c.w)] = 0;
+          static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 0;
         }
       }
     } else if (drained) {
@@ -583,14 +629,14 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
 }
 
 // Chooses the kernel of a batch by its rays: 64 groups of 32 consecutive rays,
-// spread over the batch, each lane compared with the group's first active ray.
+// spread over the launch, each lane compared with the group's first active ray.
 // Rays that run alike (primary rays of a tile, shadow rays of neighbouring
 // hits) start close to it and point the same way; then one thread per ray
 // keeps most of a warp busy without the pool's lists. Also clears the pool's
 // queue head.
 constexpr int kPlanWarps = 8, kPlanGroups = 8;  // groups per warp
-static __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const bvhgpu_ray_t* rays, uint32_t n,
-                                                               unsigned long long* queue) {
+template <typename SRC>
+__global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_constant__ SRC p) {
   __shared__ int votes[2];  // lanes that agree with their group's first ray, active lanes
   constexpr unsigned FULL = 0xFFFFFFFFu;
   if (threadIdx.x < 2) votes[threadIdx.x] = 0;
@@ -600,9 +646,10 @@ static __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const bvhg
   int agree = 0, active = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kPlanGroups; ++k) {
-    const uint64_t first = (uint64_t)n * (warp * kPlanGroups + k) / kGroups / 32u * 32u;
-    const uint64_t i = first + lane < n ? first + lane : n - 1u;
-    const bvhgpu_ray_t q = load_ray(rays, i);
+    const uint64_t first = p.n / kGroups * (warp * kPlanGroups + k);
+    const uint64_t i = first + lane < p.n ? first + lane : p.n - 1u;
+    uint32_t slot, job;
+    const bvhgpu_ray_t q = p.ray(i, slot, job);
     const unsigned live = __ballot_sync(FULL, !isnan(q.ox));
     if (live == 0) continue;
     const int lead = __ffs(live) - 1;
@@ -625,40 +672,41 @@ static __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const bvhg
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    queue[0] = 0ull;
-    queue[1] = 4 * votes[0] >= 3 * votes[1] ? kPlanSolo : kPlanPool;
+    p.queue[0] = 0ull;
+    p.queue[1] = 4 * votes[0] >= 3 * votes[1] ? kPlanSolo : kPlanPool;
   }
 }
 
 // One thread per ray on the packed scene, its stack in shared memory
 // ([level][thread]).
-template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
 __global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
-    trace_solo_kernel(const __grid_constant__ PoolArgs p) {
+    trace_solo_kernel(const __grid_constant__ SRC p) {
   using F = PackFmt<NM, FMT>;
   using W = PoolWord<NM>;
   extern __shared__ __align__(16) uint8_t pool_smem[];
   if (p.planned && p.queue[1] != kPlanSolo) return;
   typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
   const int stride = (int)blockDim.x;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.n) return;
-  const uint32_t slot = p.out_index ? __ldg(p.out_index + i) : i;
-  const bvhgpu_ray_t in = load_ray(p.rays, slot);
+  uint32_t slot, job;
+  const bvhgpu_ray_t in = p.ray(i, slot, job);
+  const PackView v = p.view(job);
   if (KIND == BVHGPU_CLOSEST)
-    reinterpret_cast<float4*>(p.hits)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
+    static_cast<float4*>(v.out)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
   bool hit = false;
   if (!isnan(in.ox)) {
     float4 c;
     PoolRay r = pool_ray<PROFILE>(in, slot, c);
-    uint32_t e = p.root_entry, sp = 0;
+    uint32_t e = v.root, sp = 0;
     while (true) {
       uint32_t node = 0, left = 0;
       bool fresh = false;
       bool end = false;
       while (!(e & kLeafBit)) {
         node = e;
-        const uint8_t* rec = p.nodes + (size_t)node * F::REC;
+        const uint8_t* rec = v.nodes + (size_t)node * F::REC;
         left = pool_node_hits<NM, FMT>(rec, r);
         fresh = left != 0;
         if (fresh) {
@@ -671,21 +719,21 @@ __global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
           end = true;
           break;
         }
-        e = pool_take<NM, FMT, ORDERED>(p, stack, stride, r.bits, node, left, fresh, sp);
+        e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, node, left, fresh, sp);
       }
       if (end) break;
       float tmax = r.tmax;
-      if (pool_leaf<PROFILE, KIND>(p, e, r, c, tmax)) {
+      if (pool_leaf<PROFILE, KIND>(v, e, r, c, tmax)) {
         hit = true;
         if (KIND == BVHGPU_ANY) break;
         r.tmax = tmax;
       }
       if (sp == 0) break;
       const typename W::T g = stack[(sp - 1) * stride];
-      e = pool_take<NM, FMT, ORDERED>(p, stack, stride, r.bits, W::node(g), W::left(g), false, sp);
+      e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, W::node(g), W::left(g), false, sp);
     }
   }
-  if (KIND == BVHGPU_ANY) p.occluded[slot] = hit ? 1 : 0;
+  if (KIND == BVHGPU_ANY) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
 }
 
 }  // namespace dev

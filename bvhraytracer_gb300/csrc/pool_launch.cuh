@@ -1,0 +1,108 @@
+// Host-side launch of the kernels on the packed scene (pool.cuh).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "pool.cuh"
+
+namespace bvhgpu {
+namespace dev {
+
+// What a launch's rays have in common.
+struct PackedCfg {
+  int nm, fmt;  // node width and format
+  int kind, profile;
+  bool any_order;        // any-hit rays push in child-index order
+  bool direction_order;  // the rays are sorted by direction
+  int sm_count;
+};
+
+// Width NM of one scene or many (pool_n*.cu, pool_jobs_n*.cu).
+template <int NM> cudaError_t launch_one_scene(OneScene& p, const PackedCfg& c, cudaStream_t s);
+template <int NM> cudaError_t launch_many_scenes(ManyScenes& p, const PackedCfg& c, cudaStream_t s);
+
+// Shared memory of an SM that the pools may take; the rest of its 256 KB is
+// L1, which the node records need.
+#ifndef BVHGPU_POOL_SMEM
+#define BVHGPU_POOL_SMEM (196 * 1024)
+#endif
+// Rays per resident warp from which a warp takes kPoolRays rays at once.
+#ifndef BVHGPU_POOL_FULL
+#define BVHGPU_POOL_FULL 48
+#endif
+// Batches of more rays may run on the pool kernel. Solo / pool, us: unordered
+// ambient-occlusion rays (N8L8, 251k triangles) 131k rays 110 / 115, 262k
+// 172 / 146, 1M 558 / 365, 4.2M 1953 / 1134; primary rays, which stay
+// together, 262k 124 / 148, 1M 253 / 290. The lines cross at about 200k rays
+// for rays that part and nowhere for rays that do not.
+#ifndef BVHGPU_POOL_MIN_RAYS
+#define BVHGPU_POOL_MIN_RAYS (1u << 18)
+#endif
+inline bool pool_wants_queue(uint64_t n) { return n > BVHGPU_POOL_MIN_RAYS; }
+constexpr int kSoloBlock = 64;
+
+// The traces of one launch: one thread per ray, pools, or both with the rays'
+// own choice between them. ordered: the rays are in direction order.
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
+inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cudaStream_t s) {
+  cudaError_t e;
+  const bool large = pool_wants_queue(p.n) && p.queue != nullptr;
+  // Rays in direction order are for the pool; otherwise the rays themselves
+  // decide.
+  const bool pool = large && direction_order;
+  p.planned = large && !pool;
+  if (p.planned) {
+    plan_kernel<SRC><<<1, kPlanWarps * 32, 0, s>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (!pool) {
+    auto k = trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
+    const size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * kSoloBlock;
+    const uint64_t grid = (p.n + kSoloBlock - 1) / kSoloBlock;
+    k<<<(unsigned)grid, kSoloBlock, smem, s>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess || !large) return e;
+  }
+  auto k = trace_pool_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
+  const size_t smem = kPoolWarps * pool_warp_bytes<NM>(p.levels);
+  if (smem > 48 * 1024 &&
+      (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+          cudaSuccess)
+    return e;
+  // Resident warps; blocks past them would find the queue empty.
+  const size_t fit = BVHGPU_POOL_SMEM / smem;
+  const uint64_t per_sm = fit < 1 ? 1 : fit > BVHGPU_POOL_MIN_BLOCKS ? BVHGPU_POOL_MIN_BLOCKS : fit;
+  const uint64_t warps = (uint64_t)sm_count * per_sm * kPoolWarps;
+  p.slots = p.n >= warps * BVHGPU_POOL_FULL ? kPoolRays : 32;
+  const uint64_t need = (p.n + kPoolWarps * 32 - 1) / (kPoolWarps * 32);
+  const uint64_t grid = need < warps / kPoolWarps ? need : warps / kPoolWarps;
+  if (!p.planned) {
+    e = cudaMemsetAsync(p.queue, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+  }
+  k<<<(unsigned)grid, kPoolWarps * 32, smem, s>>>(p);
+  return cudaGetLastError();
+}
+
+template <int NM, int FMT, typename SRC>
+inline cudaError_t launch_packed_fmt(SRC& p, const PackedCfg& c, cudaStream_t s) {
+  constexpr int F = BVHGPU_PROFILE_FAST, I = BVHGPU_PROFILE_INSTRUMENTED;
+  constexpr int C = BVHGPU_CLOSEST, A = BVHGPU_ANY;
+  const bool d = c.direction_order;
+  const int sms = c.sm_count;
+  if (c.kind == C)
+    return c.profile == F ? launch_packed<NM, F, C, FMT, true>(p, d, sms, s)
+                          : launch_packed<NM, I, C, FMT, true>(p, d, sms, s);
+  // Any-hit rays of the fast profile push in child-index order always.
+  if (c.profile == F) return launch_packed<NM, F, A, FMT, false>(p, d, sms, s);
+  return c.any_order ? launch_packed<NM, I, A, FMT, false>(p, d, sms, s)
+                     : launch_packed<NM, I, A, FMT, true>(p, d, sms, s);
+}
+
+template <int NM, typename SRC>
+inline cudaError_t launch_packed_width(SRC& p, const PackedCfg& c, cudaStream_t s) {
+  if (p.n == 0) return cudaSuccess;
+  return c.fmt == kFmtQ8 ? launch_packed_fmt<NM, kFmtQ8>(p, c, s)
+                         : launch_packed_fmt<NM, kFmtFP32>(p, c, s);
+}
+
+}  // namespace dev
+}  // namespace bvhgpu

@@ -1,0 +1,10 @@
+// Kernels on the packed scene for node records with 12 child slots: one scene.
+#include "pool_launch.cuh"
+
+namespace bvhgpu {
+namespace dev {
+template <> cudaError_t launch_one_scene<12>(OneScene& p, const PackedCfg& c, cudaStream_t s) {
+  return launch_packed_width<12>(p, c, s);
+}
+}  // namespace dev
+}  // namespace bvhgpu

@@ -7,8 +7,5 @@ cudaError_t launch_trace_n12(const SceneDev& sc, const TraceArgs& a, const Launc
                               cudaStream_t s) {
   return launch_for_width<12>(sc, a, cfg, s);
 }
-cudaError_t launch_pool_n12(const PoolArgs& p, const LaunchCfg& c, cudaStream_t s) {
-  return launch_pool_for_width<12>(p, c, s);
-}
 }  // namespace dev
 }  // namespace bvhgpu

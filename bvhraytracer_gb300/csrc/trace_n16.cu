@@ -7,8 +7,5 @@ cudaError_t launch_trace_n16(const SceneDev& sc, const TraceArgs& a, const Launc
                               cudaStream_t s) {
   return launch_for_width<16>(sc, a, cfg, s);
 }
-cudaError_t launch_pool_n16(const PoolArgs& p, const LaunchCfg& c, cudaStream_t s) {
-  return launch_pool_for_width<16>(p, c, s);
-}
 }  // namespace dev
 }  // namespace bvhgpu

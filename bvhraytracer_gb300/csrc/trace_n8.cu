@@ -7,8 +7,5 @@ cudaError_t launch_trace_n8(const SceneDev& sc, const TraceArgs& a, const Launch
                               cudaStream_t s) {
   return launch_for_width<8>(sc, a, cfg, s);
 }
-cudaError_t launch_pool_n8(const PoolArgs& p, const LaunchCfg& c, cudaStream_t s) {
-  return launch_pool_for_width<8>(p, c, s);
-}
 }  // namespace dev
 }  // namespace bvhgpu

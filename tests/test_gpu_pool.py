@@ -118,3 +118,31 @@ def test_captured_and_concurrent_traces():
     torch.cuda.synchronize()
     assert all(torch.equal(o, want) for o in outs)
     scene.status()
+
+
+@pytest.mark.parametrize("profile", ["instrumented", "fast"])
+@pytest.mark.parametrize("reorder,any_order", [(0, False), (4, True), (4, False)])
+@pytest.mark.parametrize("each", [3, 40001, 140001])
+def test_many_scenes_on_the_packed_kernels(profile, reorder, any_order, each):
+    """Jobs of scenes of several widths and formats, small and large in all."""
+    jobs, want = [], []
+    for i, (n, l, fmt) in enumerate([(8, 8, "fp32"), (8, 4, "fp32"), (4, 4, "q8"), (16, 3, "fp32"),
+                                     (12, 9, "q8"), (8, 8, "fp32")]):
+        tris = S.clutter(10 + 7 * i, i)
+        scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+        rays = _rays(tris, each + i, i, extreme=each > 3)
+        for kind in ("closest", "any"):
+            ref = scene.trace(rays, kind=kind, profile=profile, counters=True)
+            ref = ref["hits" if kind == "closest" else "occluded"]
+            want.append(ref)
+            jobs.append((scene, rays, kind, torch.zeros_like(ref), reorder, any_order))
+    pkg.trace_jobs(jobs, profile=profile)
+    torch.cuda.synchronize()
+    for (scene, rays, kind, got, _, _), ref in zip(jobs, want):
+        if kind == "closest":
+            same = (got == ref) | (torch.isnan(got) & torch.isnan(ref))
+            assert torch.equal(got.view(torch.int32)[:, 0], ref.view(torch.int32)[:, 0])
+            assert bool(same[:, 1:].all())
+        else:
+            assert torch.equal(got, ref)
+        scene.status()
