@@ -1,6 +1,7 @@
-// Traces without counters, on the packed scene (pack.cuh): two kernels with the
-// same node and leaf visits.
+// Traces without counters, on the packed scene (pack.cuh): three kernels with
+// the same node and leaf visits.
 //
+// trace_team_kernel: several lanes per ray, for small batches.
 // trace_solo_kernel: one thread per ray. trace_pool_kernel: each warp owns a
 // pool of kPoolRays rays in shared memory and three lists of them: rays whose
 // next entry is an inner node, rays whose next entry is a leaf, and free
@@ -734,6 +735,204 @@ __global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
     }
   }
   if (KIND == BVHGPU_ANY) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
+}
+
+// A team of lanes per ray, one child or triangle per lane, for batches too
+// small to fill the GPU with a ray per thread, whose time is the longest
+// ray's: a visit then costs one slab or triangle test instead of a loop over
+// them, and few rays share a warp's control flow. Every lane of a team keeps
+// the ray and its own copy of the stack.
+template <int NM> constexpr int kTeam = NM <= 4 ? 4 : (NM <= 8 ? 8 : 16);
+
+// Whether the ray hits child `c` of the node.
+template <int NM, int FMT>
+BVHGPU_DEV bool team_child_hit(const uint8_t* rec, const PoolRay& r, int c) {
+  using F = PackFmt<NM, FMT>;
+  if (c >= NM) return false;
+  const bool exact = (r.bits >> 3) & 1u;
+  float lo[3], hi[3];
+  if (FMT == kFmtFP32) {
+    const float* b = reinterpret_cast<const float*>(rec) + c;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = __ldg(b + a * NM);
+      hi[a] = __ldg(b + (3 + a) * NM);
+    }
+    if (exact && c >= (int)ldgu(rec + F::COUNT)) return false;
+  } else {
+    const uint4 h = ldgu4(rec);
+    if (c >= (int)(h.w >> 24)) return false;
+    const uint32_t org[3] = {h.x, h.y, h.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float o = __uint_as_float(org[a]), st = exp2i((int)(int8_t)(h.w >> (8 * a)));
+      lo[a] = __fadd_rd(o, (float)__ldg(rec + F::BOX + a * NM + c) * st);
+      hi[a] = __fadd_ru(o, (float)__ldg(rec + F::BOX + (3 + a) * NM + c) * st);
+    }
+  }
+  if (exact) return slab_exact(lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], r);
+  float n[3], f[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float x = (lo[a] - r.o[a]) * r.inv[a], y = (hi[a] - r.o[a]) * r.inv[a];
+    n[a] = r.inv[a] >= 0.0f ? x : y;
+    f[a] = r.inv[a] >= 0.0f ? y : x;
+  }
+  return fmaxf(max3f(n[0], n[1], n[2]), 0.0f) <= fminf(min3f(f[0], f[1], f[2]), r.tmax);
+}
+
+// One leaf visit of a team, as pool_leaf. c: the lane in its team; mask: the
+// team's lanes; base: its first lane.
+template <int T, int PROFILE, int KIND>
+BVHGPU_DEV bool team_leaf(const PackView& v, uint32_t e, const PoolRay pr, const float4& k, int c,
+                          unsigned mask, int base, float& tmax) {
+  const int cnt = (int)((e >> kLeafCountShift) & 15u) + 1;
+  const uint32_t slot = __float_as_uint(k.w);
+  const bool exact = (pr.bits >> 3) & 1u;
+  Ray r;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) { r.o[a] = pr.o[a]; r.inv[a] = pr.inv[a]; }
+  r.code = (int)(pr.bits & 3u);
+  r.kx = r.code == 2 ? 0 : r.code + 1;
+  r.ky = r.code == 0 ? 2 : r.code - 1;
+  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+    r.sx = k.x; r.sy = k.y; r.sz = k.z;
+  } else {
+    r.d[0] = k.x; r.d[1] = k.y; r.d[2] = k.z;
+  }
+  bool any = false;
+  // Fast profile: the leaf's first minimum per gang lane (visit_leaf_points).
+  float best = 1000000.0f, wu = 0.f, wv = 0.f, wprim = 0.f;
+  int winner = -1;
+  uint32_t lanes_at_best = 0;
+  for (int g = 0; g < cnt; g += T) {
+    const int i = g + c;
+    const bool mine = i < cnt;
+    const float4* b = v.blocks + ((size_t)(e & kLeafIndexMask) + ((mine ? i : g) >> 2)) * kBlockWords;
+    const float4* tri = b + kBlockTris + 3 * (i & 3);
+    const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
+    float t = 0.f, b1 = 0.f, b2 = 0.f;
+    bool h = mine;
+    if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+      // The triangle's part in the leaf's pre-test (with the tMax the leaf was
+      // entered with), and its tMax condition, repeated below.
+      float tmin = 0.0f;
+      if (!exact) {
+        const float* bf = reinterpret_cast<const float*>(b) + (i & 3);
+        float n[3], f[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const float x = (__ldg(bf + 4 * a) - r.o[a]) * r.inv[a];
+          const float y = (__ldg(bf + 4 * (3 + a)) - r.o[a]) * r.inv[a];
+          n[a] = r.inv[a] >= 0.0f ? x : y;
+          f[a] = r.inv[a] >= 0.0f ? y : x;
+        }
+        tmin = max3f(n[0], n[1], n[2]);
+        h = h && fmaxf(tmin, 0.0f) <= fminf(min3f(f[0], f[1], f[2]), pr.tmax);
+      }
+      // The triangles one after the other, each with the tMax that the
+      // accepted ones before it left: the first hit is accepted, and those
+      // behind it are tested again if they passed, or all of them if its t is
+      // not below the old tMax (it may round up, or be no number).
+      bool todo = h;
+      while (true) {
+        h = todo && (exact || !(tmax < tmin)) &&
+            (exact ? pool_watertight<false>(t0, t1, t2, r, tmax, t, b1, b2)
+                   : pool_watertight<true>(t0, t1, t2, r, tmax, t, b1, b2));
+        const unsigned hits = __ballot_sync(mask, h) & mask;
+        if (hits == 0) break;
+        any = true;
+        if (KIND == BVHGPU_ANY) return true;
+        const int first = __ffs(hits) - 1;
+        const float ti = __shfl_sync(mask, t, first);
+        const bool fell = ti < tmax;
+        tmax = ti;
+        if (base + c == first) static_cast<float4*>(v.out)[slot] = make_float4(t2.y, t, b1, b2);
+        __syncwarp(mask);
+        todo = todo && base + c > first && (h || !fell);
+        if ((__ballot_sync(mask, todo) & mask) == 0) break;
+      }
+      continue;
+    }
+    const float q[3][3] = {{t0.x, t0.y, t0.z}, {t0.w, t1.x, t1.y}, {t1.z, t1.w, t2.x}};
+    h = h && moller_trumbore(q, r, tmax, t, b1, b2);
+    unsigned hits = __ballot_sync(mask, h) & mask;
+    any = any || hits != 0;
+    if (KIND == BVHGPU_ANY) {
+      if (any) return true;
+      continue;
+    }
+    while (hits) {
+      const int from = __ffs(hits) - 1;
+      hits &= hits - 1u;
+      const float ti = __shfl_sync(mask, t, from);
+      const int id = g + from - base;
+      const uint32_t lane_bit = 1u << (id % v.gang);
+      if (ti < best || (winner >= 0 && ti == best && !(lanes_at_best & lane_bit))) {
+        lanes_at_best = ti < best ? lane_bit : lanes_at_best | lane_bit;
+        best = ti < best ? ti : best;
+        winner = id;
+        wu = __shfl_sync(mask, b1, from);
+        wv = __shfl_sync(mask, b2, from);
+        wprim = __shfl_sync(mask, t2.y, from);
+      }
+    }
+  }
+  if (PROFILE == BVHGPU_PROFILE_FAST && KIND == BVHGPU_CLOSEST && winner >= 0) {
+    tmax = best;
+    if (c == 0) static_cast<float4*>(v.out)[slot] = make_float4(wprim, best, wu, wv);
+  }
+  return any;
+}
+
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
+__global__ void __launch_bounds__(128) trace_team_kernel(const __grid_constant__ SRC p) {
+  using F = PackFmt<NM, FMT>;
+  using W = PoolWord<NM>;
+  constexpr int T = kTeam<NM>;
+  extern __shared__ __align__(16) uint8_t pool_smem[];
+  typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
+  const int stride = (int)blockDim.x;
+  // p.slots teams of each warp have a ray.
+  const int lane = (int)(threadIdx.x & 31u), c = lane & (T - 1), base = lane & ~(T - 1);
+  const unsigned mask = ((1u << T) - 1u) << base;
+  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t i = warp * (uint32_t)p.slots + (uint32_t)(lane / T);
+  if (lane / T >= p.slots || i >= p.n) return;
+  uint32_t slot, job;
+  const bvhgpu_ray_t in = p.ray(i, slot, job);
+  const PackView v = p.view(job);
+  if (KIND == BVHGPU_CLOSEST && c == 0)
+    static_cast<float4*>(v.out)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
+  __syncwarp(mask);
+  bool hit = false;
+  if (!isnan(in.ox)) {
+    float4 k;
+    PoolRay r = pool_ray<PROFILE>(in, slot, k);
+    uint32_t e = v.root, sp = 0;
+    while (true) {
+      uint32_t node = e, left = 0;
+      bool fresh = false;
+      if (!(e & kLeafBit)) {
+        const uint8_t* rec = v.nodes + (size_t)node * F::REC;
+        const bool h = team_child_hit<NM, FMT>(rec, r, c);
+        left = (__ballot_sync(mask, h) & mask) >> base;
+        fresh = left != 0;
+        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+      } else if (team_leaf<T, PROFILE, KIND>(v, e, r, k, c, mask, base, r.tmax)) {
+        hit = true;
+        if (KIND == BVHGPU_ANY) break;
+      }
+      if (!fresh) {
+        if (sp == 0) break;
+        const typename W::T g = stack[(sp - 1) * stride];
+        node = W::node(g);
+        left = W::left(g);
+      }
+      e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, node, left, fresh, sp);
+    }
+  }
+  if (KIND == BVHGPU_ANY && c == 0) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
 }
 
 }  // namespace dev

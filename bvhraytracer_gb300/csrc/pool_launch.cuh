@@ -39,12 +39,42 @@ template <int NM> cudaError_t launch_many_scenes(ManyScenes& p, const PackedCfg&
 #endif
 inline bool pool_wants_queue(uint64_t n) { return n > BVHGPU_POOL_MIN_RAYS; }
 constexpr int kSoloBlock = 64;
+// Batches of up to so many rays run with a team of lanes per ray (closest-hit /
+// any-hit). Solo / team, us, of a call from Python, which itself takes 15-17
+// (251k triangles): N8 primary rays 1k 25 / 25, 4k 60 / 36, 16k 58 / 43, 33k
+// 60 / 61; N8 ambient-occlusion rays 1k 46 / 21, 4k 47 / 24, 16k 56 / 39, 33k
+// 82 / 60, 66k 84 / 82; N16 primary rays 16k 57 / 41, 33k 59 / 76, any-hit rays
+// 16k 61 / 37, 33k 86 / 61, 66k 97 / 91.
+#ifndef BVHGPU_TEAM_MAX_CLOSEST
+#define BVHGPU_TEAM_MAX_CLOSEST 16384
+#endif
+#ifndef BVHGPU_TEAM_MAX_ANY
+#define BVHGPU_TEAM_MAX_ANY 32768
+#endif
+// Warps per SM that the teams are spread over (N16 ambient-occlusion rays, 4k:
+// 16 warps 25.6 us, 32 24.3; N4 8k 47.0 / 42.5).
+#ifndef BVHGPU_TEAM_WARPS
+#define BVHGPU_TEAM_WARPS 32
+#endif
+constexpr int kTeamBlock = 64;
 
-// The traces of one launch: one thread per ray, pools, or both with the rays'
-// own choice between them. ordered: the rays are in direction order.
+// The traces of one launch: a team per ray, one thread per ray, pools, or both
+// of these with the rays' own choice between them.
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
 inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cudaStream_t s) {
   cudaError_t e;
+  if (p.n <= (KIND == BVHGPU_ANY ? BVHGPU_TEAM_MAX_ANY : BVHGPU_TEAM_MAX_CLOSEST)) {
+    auto k = trace_team_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
+    constexpr int kMost = 32 / kTeam<NM>;
+    // As few rays per warp as keep the warps resident.
+    const uint64_t warps = (uint64_t)sm_count * BVHGPU_TEAM_WARPS;
+    const uint64_t per = (p.n + warps - 1) / warps;
+    p.slots = per > kMost ? kMost : (int)per;
+    const uint64_t need = (p.n + p.slots - 1) / p.slots;
+    const size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * kTeamBlock;
+    k<<<(unsigned)((need * 32 + kTeamBlock - 1) / kTeamBlock), kTeamBlock, smem, s>>>(p);
+    return cudaGetLastError();
+  }
   const bool large = pool_wants_queue(p.n) && p.queue != nullptr;
   // Rays in direction order are for the pool; otherwise the rays themselves
   // decide.

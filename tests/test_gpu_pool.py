@@ -64,6 +64,18 @@ def test_pool_equals_counting_kernel(n, l, fmt):
     _same(scene, rays[:LINE])        # one thread per ray
 
 
+@pytest.mark.parametrize("n,l,fmt", [(3, 2, "fp32"), (4, 16, "fp32"), (8, 8, "q8"), (8, 3, "fp32"),
+                                     (12, 12, "fp32"), (16, 16, "q8")])
+@pytest.mark.parametrize("rays", [1, 5, 4865, 16384, 16385, 32768, 32769])
+def test_team_and_solo_sizes(n, l, fmt, rays):
+    """Around the sizes where a team per ray gives way to a thread per ray
+    (16,384 closest-hit rays, 32,768 any-hit rays) and where a warp takes
+    another team."""
+    tris = S.clutter(20, 3)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    _same(scene, _rays(tris, rays, rays + n, extreme=rays > 50))
+
+
 @pytest.mark.parametrize("n", [LINE + 1, LINE + 31, 1000003])
 def test_rays_that_stay_together(n):
     tris = S.clutter(30, 2)
