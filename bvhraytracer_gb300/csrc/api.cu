@@ -259,12 +259,12 @@ static cudaError_t pack_scene(bvhgpu_scene* s) {
 // step logs, save-distance closest hits, a capped traversal stack (their
 // stacks hold one entry per pushed child, which is what the cap counts), the
 // staging wait of the failure-detection tests, node records whose boxes are
-// not ordered (imported trees), trees too deep or large for its stack words,
-// and more than 2^32 - 1 rays.
+// not ordered, Q8 ones whose boxes are not nested (imported trees), trees too
+// deep or large for its stack words, and more than 2^32 - 1 rays.
 static bool scene_uses_pool(const bvhgpu_scene* s) {
   const DeviceLayout& L = s->layout;
   return stack_cap(s) >= s->max_stack && s->stall_bytes == 0 &&
-         (L.node_format != BVHGPU_NODES_FP32 || L.boxes_ordered) &&
+         (L.node_format == BVHGPU_NODES_FP32 ? L.boxes_ordered : L.boxes_nested) &&
          L.n_inner < dev::pool_max_inner(L.node_stride) && L.inner_levels <= kPoolMaxLevels &&
          L.leaf_block[L.n_leaves] <= dev::kMaxBlocks;
 }
@@ -327,7 +327,8 @@ struct PoolQueue {
 };
 
 static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
-  return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root, s->layout.gang};
+  return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root,
+                       (int16_t)s->layout.gang, (int16_t)(s->layout.boxes_nested ? 1 : 0)};
 }
 
 // A trace on the packed scene.

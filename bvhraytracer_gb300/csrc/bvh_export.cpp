@@ -345,6 +345,23 @@ int build_device_layout(const Bvh& bvh, int gang, int leaf_memory, int node_form
     out.inner_levels = std::max(out.inner_levels, level[id] + 1);
     for (uint32_t j = 0; j < c.child_count; ++j) level[c.child_begin + j] = level[id] + 1;
   }
+  out.boxes_nested = true;
+  for (size_t id = 0; id < n && out.boxes_nested; ++id) {
+    const CompactNode& c = bvh.nodes[id];
+    for (int k = 0; k < 3; ++k) {
+      for (uint32_t j = 0; j < c.child_count; ++j) {
+        const CompactNode& ch = bvh.nodes[c.child_begin + j];
+        // (the root's own box is never tested)
+        if (id != 0 && !(ch.bmin[k] >= c.bmin[k] && ch.bmax[k] <= c.bmax[k]))
+          out.boxes_nested = false;
+      }
+      for (uint32_t i = 0; c.child_count == 0 && id != 0 && i < c.prim_count; ++i)
+        for (int v = 0; v < 3; ++v) {
+          const float x = bvh.tris[bvh.prims[c.prim_begin + i]].p[v][k];
+          if (!(x >= c.bmin[k] && x <= c.bmax[k])) out.boxes_nested = false;
+        }
+    }
+  }
   return BVHGPU_OK;
 }
 

@@ -76,6 +76,8 @@ struct DeviceLayout {
   std::vector<uint8_t> leaf_count;
   std::vector<uint32_t> leaf_block;
   int inner_levels = 0;               // inner nodes on the longest path from the root
+  // Every box lies in its parent's and every triangle in its leaf's box.
+  bool boxes_nested = true;
   uint32_t n_inner = 0, n_leaves = 0;
   uint32_t root_entry = 0;            // stack entry of the root
   uint32_t top_nodes = 0;             // inner nodes laid out first

@@ -60,8 +60,10 @@ __global__ void __launch_bounds__(128) pack_nodes_kernel(SceneDev sc, uint32_t n
         s |= (uint32_t)(k < count ? (fwd >> (4 * k)) & 15u : (uint64_t)k) << (4 * k);
       seq[a] = s;
     } else {
-      seq[2 * a] = (uint32_t)inv;
-      seq[2 * a + 1] = (uint32_t)(inv >> 32);
+      seq[2 * a] = (uint32_t)fwd;
+      seq[2 * a + 1] = (uint32_t)(fwd >> 32);
+      seq[6 + 2 * a] = (uint32_t)inv;
+      seq[6 + 2 * a + 1] = (uint32_t)(inv >> 32);
     }
   }
   *reinterpret_cast<uint32_t*>(dst + D::COUNT) = (uint32_t)count;

@@ -20,8 +20,8 @@ namespace dev {
 //   Q8:   float origin[3], int8 exp[3], uint8 count | uint8 q[6][N]
 //   uint32 entry[N]       stack entry of each child
 //   uint32 sorted[3][N]   the entries in the push sequence of each axis
-//   N <= 8: uint32 seq[3], the child at each position (nibbles);
-//         N > 8: uint64 inv[3], the position of each child (nibbles)
+//   uint32 (N > 8: uint64) seq[3]   the child at each position (nibbles)
+//   N > 8: uint64 inv[3]            the position of each child (nibbles)
 //   uint32 count
 template <int N, int FMT>
 struct PackFmt {
@@ -29,7 +29,8 @@ struct PackFmt {
   static constexpr int ENTRY = FMT == kFmtFP32 ? 24 * N : (16 + 6 * N + 15) / 16 * 16;
   static constexpr int SORTED = ENTRY + 4 * N;
   static constexpr int SEQ = SORTED + 12 * N;
-  static constexpr int COUNT = SEQ + (N <= 8 ? 12 : 24);
+  static constexpr int INV = SEQ + 24;  // N > 8
+  static constexpr int COUNT = SEQ + (N <= 8 ? 12 : 48);
   static constexpr int WORDS = (COUNT + 4 + 15) / 16;
   static constexpr int REC = (WORDS | 1) * 16;
 };

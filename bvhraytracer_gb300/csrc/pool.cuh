@@ -52,9 +52,14 @@ constexpr int kPoolWarps = 4;  // per block
 #define BVHGPU_POOL_REFILL 32
 #endif
 
-#ifndef BVHGPU_SOLO_MIN_BLOCKS
-#define BVHGPU_SOLO_MIN_BLOCKS 4
-#endif
+// Blocks of 128 threads per SM that the solo kernel's registers allow (2.1M
+// primary / shadow rays, ms, 4 / 6 / 7 / 8 blocks): N4 0.46 0.46 0.46 0.47 /
+// 0.31 0.32 0.31 0.33 (terrain 0.27 0.28 0.28 0.28); N8 0.47 0.46 0.45 0.44 / 0.32 0.31 0.30 0.29; N8 Q8 1.38
+// 1.36 1.33 1.39 / 0.45 0.43 0.45 0.47; N16 0.65 0.56 0.55 0.55 / 0.46 0.40
+// 0.40 0.40.
+template <int NM, int FMT>
+constexpr int kSoloBlocks =
+    NM == 4 ? 4 : (FMT == kFmtQ8 ? 6 : (NM == 8 ? 8 : 7));
 
 // What a ray's visits need of its scene, and where its result goes.
 struct PackView {
@@ -62,7 +67,8 @@ struct PackView {
   const float4* blocks;  // leaf blocks
   void* out;             // hits or occlusion bytes
   uint32_t root;         // stack entry of the root
-  int gang;
+  int16_t gang;
+  int16_t nested;        // every box lies in its parent's, every triangle in its leaf's
 };
 
 // Common arguments of a launch.
@@ -162,11 +168,12 @@ BVHGPU_DEV float min3f(float a, float b, float c) {
 
 struct PoolRay {
   float o[3], inv[3], tmax;
-  uint32_t bits;  // code | reverse << 2 | exact << 3 | job << 4
+  uint32_t bits;  // code | reverse << 2 | exact << 3 | job << 4 | hit << 12 (closest-hit rays)
 };
 
 // The traversal's view of a ray record; c: its leaf constants and result slot.
-template <int PROFILE>
+constexpr float kMaxInv = 1152921504606846976.0f;  // 2^60
+template <int PROFILE, bool LOOSE = false>
 BVHGPU_DEV PoolRay pool_ray(const bvhgpu_ray_t& in, uint32_t slot, float4& c) {
   const Ray q = make_ray<PROFILE>(in);
   PoolRay r;
@@ -175,7 +182,14 @@ BVHGPU_DEV PoolRay pool_ray(const bvhgpu_ray_t& in, uint32_t slot, float4& c) {
   r.tmax = q.tmax;
   // 1 / direction = 0 (an infinite direction) takes the exact form too: it
   // would make NaNs of the empty slots' rows.
-  const bool exact = q.exact || q.inv[0] == 0.0f || q.inv[1] == 0.0f || q.inv[2] == 0.0f;
+  bool exact = q.exact || q.inv[0] == 0.0f || q.inv[1] == 0.0f || q.inv[2] == 0.0f;
+  if (LOOSE) {
+    // So does one whose 1 / direction is clamped (q8_axis) where the planes
+    // are not moved apart by more than the ray's length there.
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      exact = exact || (fabsf(q.inv[a]) > kMaxInv && !(fabsf(q.o[a]) * 1.0e12f > 2.0f * fabsf(q.tmax)));
+  }
   r.bits = (uint32_t)q.code | ((q.reverse ? 1u : 0u) << 2) | ((exact ? 1u : 0u) << 3);
   c = PROFILE == BVHGPU_PROFILE_INSTRUMENTED
           ? make_float4(q.sx, q.sy, q.sz, __uint_as_float(slot))
@@ -189,6 +203,15 @@ BVHGPU_DEV PoolRay pool_ray(const bvhgpu_ray_t& in, uint32_t slot, float4& c) {
 // t0 <= t1 taken from the sign of t1 - t0 (t1 is at most tMax, which is finite,
 // and t0 at least 0, so the difference is no NaN; the +inf / -inf rows of empty
 // slots give a miss).
+BVHGPU_DEV uint32_t miss2(const float2& nx, const float2& ny, const float2& nz, const float2& fx,
+                          const float2& fy, const float2& fz, float tmax, uint32_t miss) {
+  const float t0x = fmaxf(max3f(nx.x, ny.x, nz.x), 0.0f), t0y = fmaxf(max3f(nx.y, ny.y, nz.y), 0.0f);
+  const float t1x = fminf(min3f(fx.x, fy.x, fz.x), tmax), t1y = fminf(min3f(fx.y, fy.y, fz.y), tmax);
+  // + 0 turns the -0 of t1 = -0, t0 = 0 (a hit) into +0.
+  const float2 s = f2unpack(f2add(f2sub(f2pack(t1x, t1y), f2pack(t0x, t0y)), 0ull));
+  miss = __funnelshift_l(__float_as_uint(s.y), miss, 1);
+  return __funnelshift_l(__float_as_uint(s.x), miss, 1);
+}
 BVHGPU_DEV uint32_t miss4(const float4& nx, const float4& ny, const float4& nz, const float4& fx,
                           const float4& fy, const float4& fz, const PoolRay& r, uint32_t miss) {
   const uint64_t ox = f2splat(r.o[0]), oy = f2splat(r.o[1]), oz = f2splat(r.o[2]);
@@ -196,18 +219,12 @@ BVHGPU_DEV uint32_t miss4(const float4& nx, const float4& ny, const float4& nz, 
 #pragma unroll
   for (int p = 1; p >= 0; --p) {
     const int k = 2 * p;
-    const float2 a = f2plane(f4get(nx, k), f4get(nx, k + 1), ox, ix);
-    const float2 b = f2plane(f4get(ny, k), f4get(ny, k + 1), oy, iy);
-    const float2 c = f2plane(f4get(nz, k), f4get(nz, k + 1), oz, iz);
-    const float2 d = f2plane(f4get(fx, k), f4get(fx, k + 1), ox, ix);
-    const float2 e = f2plane(f4get(fy, k), f4get(fy, k + 1), oy, iy);
-    const float2 f = f2plane(f4get(fz, k), f4get(fz, k + 1), oz, iz);
-    const float t0x = fmaxf(max3f(a.x, b.x, c.x), 0.0f), t0y = fmaxf(max3f(a.y, b.y, c.y), 0.0f);
-    const float t1x = fminf(min3f(d.x, e.x, f.x), r.tmax), t1y = fminf(min3f(d.y, e.y, f.y), r.tmax);
-    // + 0 turns the -0 of t1 = -0, t0 = 0 (a hit) into +0.
-    const float2 s = f2unpack(f2add(f2sub(f2pack(t1x, t1y), f2pack(t0x, t0y)), 0ull));
-    miss = __funnelshift_l(__float_as_uint(s.y), miss, 1);
-    miss = __funnelshift_l(__float_as_uint(s.x), miss, 1);
+    miss = miss2(f2plane(f4get(nx, k), f4get(nx, k + 1), ox, ix),
+                 f2plane(f4get(ny, k), f4get(ny, k + 1), oy, iy),
+                 f2plane(f4get(nz, k), f4get(nz, k + 1), oz, iz),
+                 f2plane(f4get(fx, k), f4get(fx, k + 1), ox, ix),
+                 f2plane(f4get(fy, k), f4get(fy, k + 1), oy, iy),
+                 f2plane(f4get(fz, k), f4get(fz, k + 1), oz, iz), r.tmax, miss);
   }
   return miss;
 }
@@ -222,8 +239,42 @@ BVHGPU_DEV bool slab_exact(float lx, float ly, float lz, float hx, float hy, flo
   return slab(lx, ly, lz, hx, hy, hz, q, r.tmax);
 }
 
+// 1 / direction up to 2^60 in size.
+BVHGPU_DEV float clamp_inv(float inv) { return fminf(fmaxf(inv, -kMaxInv), kMaxInv); }
+
+// One axis of a Q8 node for q8_planes4: t = f * c + d for a byte q placed in
+// f = 1 + q / 2^15; c = 2^15 step / direction, d for the near and the far
+// planes moved apart by more than every rounding error between them and the
+// exact chain (decoded plane - origin) / direction: each error is below 2^-22
+// of one of the terms in s.
+struct Q8Axis {
+  uint64_t c, dn, df;
+};
+BVHGPU_DEV Q8Axis q8_axis(float org, float step, float o, float inv) {
+  inv = clamp_inv(inv);
+  const float b = (org - o) * inv, c = step * 32768.0f * inv;
+  const float s = (fabsf(b) + fabsf(o * inv) + fabsf(c)) * 9.5367431640625e-7f;  // 2^-20
+  const float d = b - c;
+  return Q8Axis{f2splat(c), f2splat(d - s), f2splat(d + s)};
+}
+// Four bytes of a row, two planes per pair.
+BVHGPU_DEV void q8_planes4(uint32_t w, uint64_t c, uint64_t d, float2& p01, float2& p23) {
+  p01 = f2unpack(f2fma(f2pack(__uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u)),
+                              __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7614u))), c, d));
+  p23 = f2unpack(f2fma(f2pack(__uint_as_float(__byte_perm(w, 0x3F800000u, 0x7624u)),
+                              __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7634u))), c, d));
+}
+
 // Children of node e that the ray hits, bit c for child c.
-template <int NM, int FMT>
+//
+// LOOSE (Q8 records, any-hit rays of the instrumented profile): one fused
+// multiply-add per plane instead of the decode and the slab's subtract and
+// multiply, with the planes moved outward, so that some children are visited
+// that the ray misses. That changes no result: a triangle counts only if the
+// ray hits its own bounds (the leaf's pre-test), and then it hits every box
+// around it, whose t0 and t1 enclose the triangle's (rounding is monotonic)
+// with the same tMax. The scene's boxes must be nested.
+template <int NM, int FMT, bool LOOSE>
 BVHGPU_DEV uint32_t pool_node_hits(const uint8_t* rec, const PoolRay& r) {
   using F = PackFmt<NM, FMT>;
   const int nx = r.inv[0] >= 0.0f ? 0 : 3, ny = r.inv[1] >= 0.0f ? 1 : 4;
@@ -267,6 +318,25 @@ BVHGPU_DEV uint32_t pool_node_hits(const uint8_t* rec, const PoolRay& r) {
       return hit;
     }
     const uint8_t* qb = rec + F::BOX;
+    if constexpr (LOOSE) {
+      const Q8Axis ax = q8_axis(org[0], st[0], r.o[0], r.inv[0]);
+      const Q8Axis ay = q8_axis(org[1], st[1], r.o[1], r.inv[1]);
+      const Q8Axis az = q8_axis(org[2], st[2], r.o[2], r.inv[2]);
+#pragma unroll
+      for (int q = NM / 4 - 1; q >= 0; --q) {
+        float2 n[3][2], f[3][2];
+        q8_planes4(ldgu(qb + nx * NM + 4 * q), ax.c, ax.dn, n[0][0], n[0][1]);
+        q8_planes4(ldgu(qb + ny * NM + 4 * q), ay.c, ay.dn, n[1][0], n[1][1]);
+        q8_planes4(ldgu(qb + nz * NM + 4 * q), az.c, az.dn, n[2][0], n[2][1]);
+        q8_planes4(ldgu(qb + fx * NM + 4 * q), ax.c, ax.df, f[0][0], f[0][1]);
+        q8_planes4(ldgu(qb + fy * NM + 4 * q), ay.c, ay.df, f[1][0], f[1][1]);
+        q8_planes4(ldgu(qb + fz * NM + 4 * q), az.c, az.df, f[2][0], f[2][1]);
+#pragma unroll
+        for (int k = 1; k >= 0; --k)
+          miss = miss2(n[0][k], n[1][k], n[2][k], f[0][k], f[1][k], f[2][k], r.tmax, miss);
+      }
+      return ~miss & ((1u << count) - 1u);
+    }
 #pragma unroll
     for (int q = NM / 4 - 1; q >= 0; --q) {
       float4 near[3], far[3];
@@ -302,8 +372,8 @@ BVHGPU_DEV uint32_t pool_positions(const uint8_t* rec, uint32_t code, uint32_t h
     }
     return pm;
   }
-  const uint64_t inv = (uint64_t)ldgu(rec + F::SEQ + 8 * code) |
-                       ((uint64_t)ldgu(rec + F::SEQ + 8 * code + 4) << 32);
+  const uint64_t inv = (uint64_t)ldgu(rec + F::INV + 8 * code) |
+                       ((uint64_t)ldgu(rec + F::INV + 8 * code + 4) << 32);
   uint32_t pm = 0;
   while (hit) {
     const int c = __ffs(hit) - 1;
@@ -330,27 +400,77 @@ struct Pool {
   }
 };
 
-// A ray's next entry: the first of `left` (children of `node` still to visit,
-// non-empty), the others back on the ray's stack (level l at stack[l *
-// stride]). fresh: node is not on the stack yet.
-template <int NM, int FMT, bool ORDERED>
-BVHGPU_DEV uint32_t pool_take(const PackView& v, typename PoolWord<NM>::T* stack, int stride,
-                              uint32_t bits, uint32_t node, uint32_t left, bool fresh,
-                              uint32_t& sp) {
+// Whether the child at push position k of a node lies behind the ray's tMax:
+// its entry distance t0, as the slab test computes it.
+template <int NM, int FMT>
+BVHGPU_DEV bool pool_behind(const uint8_t* rec, const PoolRay& r, int k) {
   using F = PackFmt<NM, FMT>;
-  int k;
-  if (ORDERED && ((bits >> 2) & 1u)) k = 31 - __clz(left);
-  else k = __ffs(left) - 1;
-  left &= ~(1u << k);
-  if (fresh) {
-    if (left) stack[sp++ * stride] = PoolWord<NM>::make(node, left);
-  } else if (left) {
-    stack[(sp - 1) * stride] = PoolWord<NM>::make(node, left);
-  } else {
-    --sp;
+  const uint32_t code = r.bits & 3u;
+  const uint32_t w = NM <= 8 ? ldgu(rec + F::SEQ + 4 * code) >> (4 * k)
+                             : ldgu(rec + F::SEQ + 8 * code + (k >= 8 ? 4 : 0)) >> (4 * (k & 7));
+  const int c = (int)(w & 15u);
+  float t[3];
+  uint4 h = make_uint4(0u, 0u, 0u, 0u);
+  if (FMT == kFmtQ8) h = ldgu4(rec);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const bool neg = !(r.inv[a] >= 0.0f);
+    const int row = neg ? 3 + a : a;
+    float x;
+    if (FMT == kFmtFP32) {
+      x = __ldg(reinterpret_cast<const float*>(rec) + row * NM + c);
+    } else {
+      const float org = __uint_as_float(a == 0 ? h.x : (a == 1 ? h.y : h.z));
+      const float q = (float)__ldg(rec + F::BOX + row * NM + c) * exp2i((int)(int8_t)(h.w >> (8 * a)));
+      x = neg ? __fadd_ru(org, q) : __fadd_rd(org, q);
+    }
+    t[a] = (x - r.o[a]) * r.inv[a];
   }
-  const uint8_t* rec = v.nodes + (size_t)node * F::REC;
-  return ldgu(rec + (ORDERED ? F::SORTED + (bits & 3u) * (4 * NM) : F::ENTRY) + 4 * k);
+  return max3f(t[0], t[1], t[2]) > r.tmax;
+}
+
+// A ray's next entry: the first of `left` (children of `node` still to visit),
+// the others back on the ray's stack (level l at stack[l * stride]). fresh:
+// node is not on the stack yet; otherwise its word is the stack's top, and
+// with left = 0 the top is read here. Returns false when nothing is left.
+//
+// CULL (closest-hit rays of the instrumented profile that have a hit, nested
+// boxes): children behind tMax are dropped. A visit would find nothing there:
+// every box and triangle inside starts at the same t0 or later (rounding is
+// monotonic) and tMax does not change during the visit. 1M-triangle N8L8 tree,
+// primary rays: 18.8 -> 13.9 node visits per ray, solo kernel 0.53 -> 0.47 ms
+// (2.1M rays); N16 0.76 -> 0.65 ms; N4, whose visits cost little more than the
+// check, 0.46 -> 0.47. Pool kernel, bounced rays: N16 1.13 -> 1.06 ms, N8 1.15
+// -> 1.19.
+template <int NM, int FMT, bool ORDERED, bool CULL>
+BVHGPU_DEV bool pool_take(const PackView& v, typename PoolWord<NM>::T* stack, int stride,
+                          const PoolRay& r, uint32_t node, uint32_t left, bool fresh,
+                          uint32_t& sp, uint32_t& e) {
+  using F = PackFmt<NM, FMT>;
+  using W = PoolWord<NM>;
+  const bool cull = CULL && ((r.bits >> 12) & 1u) && !((r.bits >> 3) & 1u) && v.nested;
+  while (true) {
+    if (!fresh) {
+      if (sp == 0) return false;
+      const typename W::T g = stack[(sp - 1) * stride];
+      node = W::node(g);
+      left = W::left(g);
+    }
+    int k;
+    if (ORDERED && ((r.bits >> 2) & 1u)) k = 31 - __clz(left);
+    else k = __ffs(left) - 1;
+    left &= ~(1u << k);
+    const uint8_t* rec = v.nodes + (size_t)node * F::REC;
+    if (fresh) {
+      if (left) stack[sp++ * stride] = W::make(node, left);
+    } else {
+      if (left) stack[(sp - 1) * stride] = W::make(node, left);
+      else --sp;
+      if (CULL && cull && pool_behind<NM, FMT>(rec, r, k)) continue;
+    }
+    e = ldgu(rec + (ORDERED ? F::SORTED + (r.bits & 3u) * (4 * NM) : F::ENTRY) + 4 * k);
+    return true;
+  }
 }
 
 template <bool MM>
@@ -501,6 +621,10 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
   using F = PackFmt<NM, FMT>;
   constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int K = kPoolRays;
+  constexpr bool kLoose = FMT == kFmtQ8 && PROFILE == BVHGPU_PROFILE_INSTRUMENTED &&
+                          KIND == BVHGPU_ANY;
+  constexpr bool kCull =
+      PROFILE == BVHGPU_PROFILE_INSTRUMENTED && KIND == BVHGPU_CLOSEST && NM >= 12;
   extern __shared__ __align__(16) uint8_t pool_smem[];
   if (p.planned && p.queue[1] != kPlanPool) return;
   const unsigned lane = threadIdx.x & 31u;
@@ -547,7 +671,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
           static_cast<float4*>(v.out)[slot] = make_float4(__int_as_float(-1), in.tmax, 0.f, 0.f);
         if (!isnan(in.ox)) {
           float4 c;
-          PoolRay r = pool_ray<PROFILE>(in, slot, c);
+          PoolRay r = pool_ray<PROFILE, kLoose>(in, slot, c);
           r.bits |= job << 4;
           P.a[j] = make_float4(r.o[0], r.o[1], r.o[2], r.tmax);
           P.b[j] = make_float4(r.inv[0], r.inv[1], r.inv[2], __uint_as_float(r.bits));
@@ -564,23 +688,15 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
       if ((int)lane < m) {
         j = P.list[n_node + (int)lane];
         const PoolRay r = P.ray(j);
-        const PackView& v = p.view(r.bits >> 4);
+        const PackView& v = p.view((r.bits >> 4) & 0xFFu);
         const uint2 st = P.state[j];
-        uint32_t node = st.x, sp = st.y;
-        const uint8_t* rec = v.nodes + (size_t)node * F::REC;
-        uint32_t left = pool_node_hits<NM, FMT>(rec, r);
+        uint32_t sp = st.y, e;
+        const uint8_t* rec = v.nodes + (size_t)st.x * F::REC;
+        uint32_t left = pool_node_hits<NM, FMT, kLoose>(rec, r);
         const bool fresh = left != 0;
-        if (fresh) {
-          if (ORDERED) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
-        } else if (sp > 0) {
-          const typename W::T g = P.stack[(sp - 1) * K + j];
-          node = W::node(g);
-          left = W::left(g);
-        }
+        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
         next = 2;
-        if (left) {
-          const uint32_t e = pool_take<NM, FMT, ORDERED>(v, P.stack + j, K, r.bits, node, left,
-                                                         fresh, sp);
+        if (pool_take<NM, FMT, ORDERED, kCull>(v, P.stack + j, K, r, st.x, left, fresh, sp, e)) {
           P.state[j] = make_uint2(e, sp);
           next = (int)(e >> 31);
         } else if (KIND == BVHGPU_ANY) {
@@ -592,22 +708,24 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
       n_leaf -= m;
       if ((int)lane < m) {
         j = P.list[K + n_leaf + (int)lane];
-        const PoolRay r = P.ray(j);
-        const PackView& v = p.view(r.bits >> 4);
+        PoolRay r = P.ray(j);
+        const PackView& v = p.view((r.bits >> 4) & 0xFFu);
         const float4 c = P.c[j];
         const uint2 st = P.state[j];
-        uint32_t sp = st.y;
+        uint32_t sp = st.y, e;
         float tmax = r.tmax;
         const bool hit = pool_leaf<PROFILE, KIND>(v, st.x, r, c, tmax);
+        if (KIND == BVHGPU_CLOSEST && hit) {
+          r.tmax = tmax;
+          r.bits |= 1u << 12;
+          P.a[j].w = tmax;
+          P.b[j].w = __uint_as_float(r.bits);
+        }
         next = 2;
         if (KIND == BVHGPU_ANY && hit) {
           static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 1;
-        } else if (sp > 0) {
-          const typename W::T g = P.stack[(sp - 1) * K + j];
-          const uint32_t e = pool_take<NM, FMT, ORDERED>(v, P.stack + j, K, r.bits, W::node(g),
-                                                         W::left(g), false, sp);
+        } else if (pool_take<NM, FMT, ORDERED, kCull>(v, P.stack + j, K, r, 0u, 0u, false, sp, e)) {
           P.state[j] = make_uint2(e, sp);
-          if (KIND == BVHGPU_CLOSEST && hit) P.a[j].w = tmax;
           next = (int)(e >> 31);
         } else if (KIND == BVHGPU_ANY) {
           static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 0;
@@ -681,10 +799,14 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // One thread per ray on the packed scene, its stack in shared memory
 // ([level][thread]).
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
-__global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
+__global__ void __launch_bounds__(128, kSoloBlocks<NM, FMT>)
     trace_solo_kernel(const __grid_constant__ SRC p) {
   using F = PackFmt<NM, FMT>;
   using W = PoolWord<NM>;
+  constexpr bool kLoose = FMT == kFmtQ8 && PROFILE == BVHGPU_PROFILE_INSTRUMENTED &&
+                          KIND == BVHGPU_ANY;
+  constexpr bool kCull =
+      PROFILE == BVHGPU_PROFILE_INSTRUMENTED && KIND == BVHGPU_CLOSEST && NM >= 8;
   extern __shared__ __align__(16) uint8_t pool_smem[];
   if (p.planned && p.queue[1] != kPlanSolo) return;
   typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
@@ -699,39 +821,26 @@ __global__ void __launch_bounds__(128, BVHGPU_SOLO_MIN_BLOCKS)
   bool hit = false;
   if (!isnan(in.ox)) {
     float4 c;
-    PoolRay r = pool_ray<PROFILE>(in, slot, c);
+    PoolRay r = pool_ray<PROFILE, kLoose>(in, slot, c);
     uint32_t e = v.root, sp = 0;
-    while (true) {
-      uint32_t node = 0, left = 0;
-      bool fresh = false;
-      bool end = false;
-      while (!(e & kLeafBit)) {
-        node = e;
-        const uint8_t* rec = v.nodes + (size_t)node * F::REC;
-        left = pool_node_hits<NM, FMT>(rec, r);
-        fresh = left != 0;
-        if (fresh) {
-          if (ORDERED) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
-        } else if (sp > 0) {
-          const typename W::T g = stack[(sp - 1) * stride];
-          node = W::node(g);
-          left = W::left(g);
-        } else {
-          end = true;
-          break;
-        }
-        e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, node, left, fresh, sp);
+    bool more = true;
+    while (more) {
+      while (more && !(e & kLeafBit)) {
+        const uint8_t* rec = v.nodes + (size_t)e * F::REC;
+        uint32_t left = pool_node_hits<NM, FMT, kLoose>(rec, r);
+        const bool fresh = left != 0;
+        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        more = pool_take<NM, FMT, ORDERED, kCull>(v, stack, stride, r, e, left, fresh, sp, e);
       }
-      if (end) break;
+      if (!more) break;
       float tmax = r.tmax;
       if (pool_leaf<PROFILE, KIND>(v, e, r, c, tmax)) {
         hit = true;
         if (KIND == BVHGPU_ANY) break;
         r.tmax = tmax;
+        r.bits |= 1u << 12;
       }
-      if (sp == 0) break;
-      const typename W::T g = stack[(sp - 1) * stride];
-      e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, W::node(g), W::left(g), false, sp);
+      more = pool_take<NM, FMT, ORDERED, kCull>(v, stack, stride, r, 0u, 0u, false, sp, e);
     }
   }
   if (KIND == BVHGPU_ANY) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
@@ -911,7 +1020,8 @@ __global__ void __launch_bounds__(128) trace_team_kernel(const __grid_constant__
     PoolRay r = pool_ray<PROFILE>(in, slot, k);
     uint32_t e = v.root, sp = 0;
     while (true) {
-      uint32_t node = e, left = 0;
+      const uint32_t node = e;
+      uint32_t left = 0;
       bool fresh = false;
       if (!(e & kLeafBit)) {
         const uint8_t* rec = v.nodes + (size_t)node * F::REC;
@@ -923,13 +1033,7 @@ __global__ void __launch_bounds__(128) trace_team_kernel(const __grid_constant__
         hit = true;
         if (KIND == BVHGPU_ANY) break;
       }
-      if (!fresh) {
-        if (sp == 0) break;
-        const typename W::T g = stack[(sp - 1) * stride];
-        node = W::node(g);
-        left = W::left(g);
-      }
-      e = pool_take<NM, FMT, ORDERED>(v, stack, stride, r.bits, node, left, fresh, sp);
+      if (!pool_take<NM, FMT, ORDERED, false>(v, stack, stride, r, node, left, fresh, sp, e)) break;
     }
   }
   if (KIND == BVHGPU_ANY && c == 0) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
