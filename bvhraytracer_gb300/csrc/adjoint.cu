@@ -295,6 +295,27 @@ __global__ void __launch_bounds__(128) adjoint_hits_kernel(SceneDev sc, AdjointA
   scatter_grads(sc, a, valid, prim, g);
 }
 
+// Hit records to four arrays in one pass (32 bytes per ray moved); as four
+// strided copies by the caller each one reads every record's 32-byte sector.
+__global__ void __launch_bounds__(256) unpack_hits_kernel(const float4* hits, uint64_t n,
+                                                          int32_t* prim, float* t, float* u,
+                                                          float* v) {
+  const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;
+  if (i >= n) return;
+  const float4 h = __ldg(hits + i);
+  prim[i] = __float_as_int(h.x);
+  t[i] = h.y;
+  u[i] = h.z;
+  v[i] = h.w;
+}
+
+cudaError_t launch_unpack_hits(const float4* hits, uint64_t n, int32_t* prim, float* t, float* u,
+                               float* v, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  unpack_hits_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(hits, n, prim, t, u, v);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_adjoint(const SceneDev& sc, int nm, const AdjointArgs& a, cudaStream_t s) {
   if (a.n == 0) return cudaSuccess;
   const int bs = 128;

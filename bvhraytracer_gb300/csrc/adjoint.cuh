@@ -29,6 +29,8 @@ struct AdjointArgs {
   const float* grad_v = nullptr;
 };
 
+cudaError_t launch_unpack_hits(const float4* hits, uint64_t n, int32_t* prim, float* t, float* u,
+                               float* v, cudaStream_t s);
 cudaError_t launch_adjoint(const SceneDev& sc, int nm, const AdjointArgs& a, cudaStream_t s);
 
 }  // namespace dev

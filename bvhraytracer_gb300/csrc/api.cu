@@ -1400,6 +1400,18 @@ int bvhgpu_adjoint_vertices(bvhgpu_scene_t s, const bvhgpu_ray_t* rays, uint64_t
   return BVHGPU_OK;
 }
 
+int bvhgpu_unpack_hits(const bvhgpu_hit_t* hits, uint64_t n, int32_t* prim, float* t, float* u,
+                       float* v, void* stream) {
+  if (n == 0) return BVHGPU_OK;
+  if (!hits || !prim || !t || !u || !v || ((uintptr_t)hits & 15) || ((uintptr_t)prim & 3) ||
+      ((uintptr_t)t & 3) || ((uintptr_t)u & 3) || ((uintptr_t)v & 3))
+    return set_error(BVHGPU_ERR_BAD_ARG, "unpack hits: null or misaligned buffer");
+  if (n > (1ull << 38)) return set_error(BVHGPU_ERR_BAD_ARG, "unpack hits: at most 2^38 records");
+  cudaError_t e = dev::launch_unpack_hits(reinterpret_cast<const float4*>(hits), n, prim, t, u, v,
+                                          (cudaStream_t)stream);
+  return e == cudaSuccess ? BVHGPU_OK : cuda_error(e, "unpack hits");
+}
+
 int bvhgpu_adjoint_hits(bvhgpu_scene_t s, const bvhgpu_ray_t* rays, const bvhgpu_hit_t* hits,
                         uint64_t n, const float* grad_t, const float* grad_u,
                         const float* grad_v, const int32_t* faces, uint64_t n_faces,

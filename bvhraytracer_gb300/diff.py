@@ -33,9 +33,17 @@ class _RayHit(torch.autograd.Function):
             ctx.save_for_backward(rc, faces32)  # the backward re-traces: no hits kept
         else:
             ctx.save_for_backward(rc, faces32, res)
-        prim = res.view(torch.int32)[:, 0].clone()
+        # One pass over the hit records instead of four strided copies; outputs
+        # without a gradient give the backward None, not an array of zeros.
+        n = rc.shape[0]
+        t, u, v = (torch.empty(n, dtype=torch.float32, device=rc.device) for _ in range(3))
+        prim = torch.empty(n, dtype=torch.int32, device=rc.device)
+        N.check(N.lib().bvhgpu_unpack_hits(
+            res.data_ptr(), n, prim.data_ptr(), t.data_ptr(), u.data_ptr(), v.data_ptr(),
+            C.c_void_p(torch.cuda.current_stream(rc.device).cuda_stream)))
         ctx.mark_non_differentiable(prim)
-        return res[:, 1].clone(), res[:, 2].clone(), res[:, 3].clone(), prim
+        ctx.set_materialize_grads(False)
+        return t, u, v, prim
 
     @staticmethod
     def backward(ctx, gt, gu, gv, _gprim):

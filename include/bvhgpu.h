@@ -429,6 +429,12 @@ int bvhgpu_adjoint_hits(bvhgpu_scene_t scene, const bvhgpu_ray_t* rays, const bv
                         uint64_t n_verts, float* grad_verts, float* grad_tri9, float* grad_rays,
                         void* stream);
 
+/* The fields of n closest-hit records as four arrays (16-byte aligned hits,
+ * 4-byte aligned arrays). No reference counterpart: the outputs of the
+ * differentiable hit distance. */
+int bvhgpu_unpack_hits(const bvhgpu_hit_t* hits, uint64_t n, int32_t* prim, float* t, float* u,
+                       float* v, void* stream);
+
 /* ---- tracing without allocation --------------------------------------- */
 /* No counterpart in the reference (its renderer allocates nothing on a GPU).
  * For callers that must not allocate GPU memory while they trace (a plugin
