@@ -27,10 +27,12 @@
 
 // Streams (and staging regions) of the host-buffer pipeline: a chunk's copy
 // in waits until the chunk this many places earlier has been traced and
-// copied out. 1M-triangle frame, median step: 2 streams 8.63 ms, 3 streams
-// 8.38 ms, 4 streams 8.39 ms.
+// copied out, and that many traces share the GPU, so that one's end overlaps
+// the next one's start. 1M-triangle 1080p frame / 251k-triangle 640x360 frame,
+// median step: 3 streams 5.22 / 0.89 ms, 4 streams 5.14 / 0.84, 5 streams 5.14 /
+// 0.84, 6 streams 5.16 / 0.84.
 #ifndef BVHGPU_HOST_STREAMS
-#define BVHGPU_HOST_STREAMS 3
+#define BVHGPU_HOST_STREAMS 4
 #endif
 
 namespace bvhgpu {
@@ -822,7 +824,7 @@ int bvhgpu_trace_steps(bvhgpu_scene_t s, const bvhgpu_ray_t* rays, uint64_t n,
 // median step 8.74-8.75 ms doubling up to 8 Mi, 8.84-9.15 ms in quarters.
 // (With the scratch allocated per launch from the pool, growing chunks
 // alternated between 8.75 and 10.25 ms per step from run to run.)
-// Three streams, median step by growth / cap (three runs on three GPUs):
+// With three streams, median step by growth / cap (three runs on three GPUs):
 // 200 % / 8 Mi 8.33-8.39 ms, 200 % / 4 Mi 8.36, 175 % / 3 Mi 8.30,
 // 150 % / 8, 6, 4, 3, 2 Mi 8.25, 8.27, 8.03, 8.27, 7.95-8.27,
 // 135 % / 4 Mi 8.06, 125 % / 6, 4, 3, 2 Mi 9.05, 7.88 (twice), 7.91, 7.93,
@@ -830,7 +832,7 @@ int bvhgpu_trace_steps(bvhgpu_scene_t s, const bvhgpu_ray_t* rays, uint64_t n,
 // 125 % / 4 Mi: 7.98 / 7.88 / 7.87. With the kernels of a 6.99 ms frame:
 // 125 % / 4 Mi 7.21 ms, 125 % / 2 Mi 7.24, 110 % / 4 Mi 7.39, 150 % / 4 Mi
 // 7.38. A chunk's copy in waits for the copy out
-// of the chunk three before it (same stream, same staging region), so
+// of the chunk four before it (same stream, same staging region), so
 // chunks that grow slowly keep the copies ahead of the traces without
 // leaving one large chunk to trace after the last copy.
 #ifndef BVHGPU_HOST_GROW

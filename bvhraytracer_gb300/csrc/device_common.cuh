@@ -346,6 +346,19 @@ BVHGPU_DEV float4 ldg4(const void* p) { return __ldg(reinterpret_cast<const floa
 BVHGPU_DEV uint4 ldgu4(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 BVHGPU_DEV uint32_t ldgu(const void* p) { return __ldg(reinterpret_cast<const uint32_t*>(p)); }
 
+// Two 16-byte words of a 32-byte aligned record with one 256-bit access
+// (sm_100 family).
+BVHGPU_DEV void ldg32(const void* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+BVHGPU_DEV void stg32(void* p, const float4& a, const float4& b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x),
+               "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+
 BVHGPU_DEV float f4get(const float4& v, int k) {
   return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
 }

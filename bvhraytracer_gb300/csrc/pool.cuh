@@ -19,13 +19,14 @@
 //
 // What bounds them. Pool, ambient-occlusion rays in direction order (3.7M rays,
 // 251k triangles, N8L8): the L1 data pipe is busy 82 % of the time (a node
-// visit gathers 192 bytes of boxes), 21 lanes per instruction, issue 66 %;
-// 0.81 ms, against 1.18 ms of the persistent kernel (17.4 lanes, and 16 of 100
-// L1 cycles lost to bank conflicts of the leaf bounds' 192-byte stride).
-// 8.3M such rays of the 1M-triangle frame: 3.13 -> 2.04 ms; unordered, from
-// the per-ray kernel (6.7 lanes): 4.5M rays, N4L8, 2.97 -> 1.33 ms. Solo, 2.1M
-// primary rays of that frame 0.62 -> 0.51 ms, shadow rays 0.41 -> 0.31 ms
-// (latency: 20 % of the warps resident at the end of a launch).
+// visit gathers 192 bytes of boxes, 40 of the 57 L1 cycles of a ray), issue
+// 66 %; steps have 29 of 32 rays at nodes and 26 at leaves. 1.18 ms on the
+// persistent kernel (17.4 lanes per instruction, a fifth of the L1 cycles lost
+// to bank conflicts), 0.81 ms here; 8.3M such rays of the 1M-triangle frame
+// 3.13 -> 2.04 ms; unordered, from the per-ray kernel (6.7 lanes), 4.5M rays,
+// N4L8, 2.97 -> 1.33 ms. Solo, 2.1M primary rays of that frame 0.62 -> 0.44 ms,
+// shadow rays 0.41 -> 0.29 ms: latency and the longest rays (a fifth of the
+// warps resident on average).
 #pragma once
 #include "pack.cuh"
 #include "traverse.cuh"
@@ -151,7 +152,7 @@ constexpr uint32_t pool_max_inner(int nm) { return nm <= 8 ? 1u << 24 : kLeafBit
 template <int NM>
 __host__ __device__ inline size_t pool_warp_bytes(int levels) {
   return (size_t)kPoolRays * (3 * 16 + 8 + sizeof(typename PoolWord<NM>::T) * (size_t)levels) +
-         (3 * kPoolRays + 15) / 16 * 16;
+         64 + (3 * kPoolRays + 15) / 16 * 16;
 }
 
 // max / min of three.
@@ -389,6 +390,7 @@ struct Pool {
   float4 *a, *b, *c;  // origin, tMax | 1 / direction, bits | leaf constants, result slot
   uint2* state;       // next entry, stack words in use
   typename PoolWord<NM>::T* stack;  // [level][ray]
+  uint16_t* pairs;    // pool_pairs: 32
   uint8_t* list;      // node rays, leaf rays, free slots: kPoolRays each
   BVHGPU_DEV PoolRay ray(int j) const {
     const float4 x = a[j], y = b[j];
@@ -499,74 +501,25 @@ BVHGPU_DEV bool mt_rejects(float n1, float div) {
   return an > ad * (neg ? 1e-30f : 1.0001f);
 }
 
-// One leaf visit: returns whether any triangle was hit. Closest-hit rays
-// lower tmax and write their hit record. First a cheap test of every triangle
-// of the leaf, four at a time (the stored bounds, or the first barycentric
-// without its division), then the full test of the few that pass, so that a
-// warp runs as many full tests as one of its rays needs at most.
-template <int PROFILE, int KIND>
-BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const float4 c,
-                          float& tmax) {
-  const int cnt = (int)((e >> kLeafCountShift) & 15u) + 1;
-  const float4* blk = v.blocks + (size_t)(e & kLeafIndexMask) * kBlockWords;
-  const uint32_t slot = __float_as_uint(c.w);
-  Ray r;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) { r.o[a] = pr.o[a]; r.inv[a] = pr.inv[a]; }
-  r.code = (int)(pr.bits & 3u);
-  r.kx = r.code == 2 ? 0 : r.code + 1;
-  r.ky = r.code == 0 ? 2 : r.code - 1;
-  bool any = false;
-  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
-    r.sx = c.x; r.sy = c.y; r.sz = c.z;
-    const bool exact = (pr.bits >> 3) & 1u;
-    uint32_t pass = (1u << cnt) - 1u;
-    if (!exact) {
-      const int nx = pr.inv[0] >= 0.0f ? 0 : 3, ny = pr.inv[1] >= 0.0f ? 1 : 4;
-      const int nz = pr.inv[2] >= 0.0f ? 2 : 5;
-      const int fx = 3 - nx, fy = 5 - ny, fz = 7 - nz;
-      uint32_t miss = 0;
-      for (int g = (cnt - 1) >> 2; g >= 0; --g) {
-        const float4* b = blk + g * kBlockWords;
-        miss = miss4(__ldg(b + nx), __ldg(b + ny), __ldg(b + nz), __ldg(b + fx), __ldg(b + fy),
-                     __ldg(b + fz), pr, miss);
-      }
-      pass &= ~miss;
-    }
-    while (pass) {
-      const int i = __ffs(pass) - 1;
-      pass &= pass - 1u;
-      const float4* b = blk + (i >> 2) * kBlockWords;
-      if (KIND == BVHGPU_CLOSEST && !exact && tmax != pr.tmax) {
-        // tMax fell in this leaf: the pre-test's tMax condition again.
-        const float* bf = reinterpret_cast<const float*>(b) + (i & 3);
-        float m[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          const float lo = (__ldg(bf + 4 * a) - r.o[a]) * r.inv[a];
-          const float hi = (__ldg(bf + 4 * (3 + a)) - r.o[a]) * r.inv[a];
-          m[a] = fminf(lo, hi);
-        }
-        if (tmax < fmaxf(fmaxf(m[0], m[1]), m[2])) continue;
-      }
-      const float4* tri = b + kBlockTris + 3 * (i & 3);
-      const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
-      float t, b1, b2;
-      const bool h = exact ? pool_watertight<false>(t0, t1, t2, r, tmax, t, b1, b2)
-                           : pool_watertight<true>(t0, t1, t2, r, tmax, t, b1, b2);
-      if (!h) continue;
-      any = true;
-      if (KIND == BVHGPU_ANY) break;
-      // Each accepted triangle overwrites the hit (triangle.cpp:243).
-      tmax = t;
-      static_cast<float4*>(v.out)[slot] = make_float4(t2.y, t, b1, b2);
-    }
-    return any;
-  }
-  // Fast profile: Moller-Trumbore on every triangle; the tie rule of
-  // triIntersect{L} as in visit_leaf_points.
-  r.d[0] = c.x; r.d[1] = c.y; r.d[2] = c.z;
+// The triangles of a leaf that a cheap test does not rule out, four at a time:
+// the stored bounds (instrumented profile; all of them for rays that take the
+// exact forms), or the first barycentric without its division.
+template <int PROFILE>
+BVHGPU_DEV uint32_t leaf_candidates(const float4* blk, int cnt, const PoolRay& r, const float4& c) {
+  const uint32_t all = (1u << cnt) - 1u;
   uint32_t miss = 0;
+  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+    if ((r.bits >> 3) & 1u) return all;
+    const int nx = r.inv[0] >= 0.0f ? 0 : 3, ny = r.inv[1] >= 0.0f ? 1 : 4;
+    const int nz = r.inv[2] >= 0.0f ? 2 : 5;
+    const int fx = 3 - nx, fy = 5 - ny, fz = 7 - nz;
+    for (int g = (cnt - 1) >> 2; g >= 0; --g) {
+      const float4* b = blk + g * kBlockWords;
+      miss = miss4(__ldg(b + nx), __ldg(b + ny), __ldg(b + nz), __ldg(b + fx), __ldg(b + fy),
+                   __ldg(b + fz), r, miss);
+    }
+    return ~miss & all;
+  }
   for (int g = (cnt - 1) >> 2; g >= 0; --g) {
     const float4* tri = blk + g * kBlockWords + kBlockTris;
 #pragma unroll
@@ -575,28 +528,98 @@ BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const
       // moller_trumbore()'s divisor and numerator of b1.
       const float e1x = t0.w - t0.x, e1y = t1.x - t0.y, e1z = t1.y - t0.z;
       const float e2x = t1.z - t0.x, e2y = t1.w - t0.y, e2z = t2.x - t0.z;
-      const float s1x = r.d[1] * e2z - r.d[2] * e2y;
-      const float s1y = r.d[2] * e2x - r.d[0] * e2z;
-      const float s1z = r.d[0] * e2y - r.d[1] * e2x;
+      const float s1x = c.y * e2z - c.z * e2y;
+      const float s1y = c.z * e2x - c.x * e2z;
+      const float s1z = c.x * e2y - c.y * e2x;
       const float div = s1x * e1x + s1y * e1y + s1z * e1z;
       const float n1 = (r.o[0] - t0.x) * s1x + (r.o[1] - t0.y) * s1y + (r.o[2] - t0.z) * s1z;
       miss = (miss << 1) | (mt_rejects(n1, div) ? 1u : 0u);
     }
   }
-  uint32_t pass = ~miss & ((1u << cnt) - 1u);
+  return ~miss & all;
+}
+
+// What the full triangle tests read of a ray.
+template <int PROFILE>
+BVHGPU_DEV Ray leaf_ray(const PoolRay& pr, const float4& c) {
+  Ray r;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) { r.o[a] = pr.o[a]; r.inv[a] = pr.inv[a]; }
+  r.code = (int)(pr.bits & 3u);
+  r.kx = r.code == 2 ? 0 : r.code + 1;
+  r.ky = r.code == 0 ? 2 : r.code - 1;
+  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+    r.sx = c.x; r.sy = c.y; r.sz = c.z;
+  } else {
+    r.d[0] = c.x; r.d[1] = c.y; r.d[2] = c.z;
+  }
+  return r;
+}
+
+// The full test of one triangle.
+template <int PROFILE>
+BVHGPU_DEV bool leaf_test(const float4* tri, const Ray& r, bool exact, float tmax, float& t,
+                          float& b1, float& b2, float& prim) {
+  const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
+  prim = t2.y;
+  if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED)
+    return exact ? pool_watertight<false>(t0, t1, t2, r, tmax, t, b1, b2)
+                 : pool_watertight<true>(t0, t1, t2, r, tmax, t, b1, b2);
+  const float q[3][3] = {{t0.x, t0.y, t0.z}, {t0.w, t1.x, t1.y}, {t1.z, t1.w, t2.x}};
+  return moller_trumbore(q, r, tmax, t, b1, b2);
+}
+
+BVHGPU_DEV const float4* leaf_blocks(const PackView& v, uint32_t e) {
+  return v.blocks + (size_t)(e & kLeafIndexMask) * kBlockWords;
+}
+BVHGPU_DEV int leaf_count(uint32_t e) { return (int)((e >> kLeafCountShift) & 15u) + 1; }
+BVHGPU_DEV const float4* leaf_tri(const float4* blk, int i) {
+  return blk + (i >> 2) * kBlockWords + kBlockTris + 3 * (i & 3);
+}
+
+// One leaf visit: returns whether any triangle was hit. Closest-hit rays
+// lower tmax and write their hit record. First the cheap test of every
+// triangle, then the full test of the few that pass, so that a warp runs as
+// many full tests as one of its rays needs at most.
+template <int PROFILE, int KIND>
+BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const float4 c,
+                          float& tmax) {
+  const float4* blk = leaf_blocks(v, e);
+  const uint32_t slot = __float_as_uint(c.w);
+  const bool exact = PROFILE == BVHGPU_PROFILE_INSTRUMENTED && ((pr.bits >> 3) & 1u);
+  uint32_t pass = leaf_candidates<PROFILE>(blk, leaf_count(e), pr, c);
+  const Ray r = leaf_ray<PROFILE>(pr, c);
+  bool any = false;
+  // Fast profile: the tie rule of triIntersect{L} as in visit_leaf_points.
   float leaf_best = 1000000.0f, wu = 0.f, wv = 0.f, wprim = 0.f;
   int winner = -1;
   uint32_t lanes_at_best = 0;
   while (pass) {
     const int i = __ffs(pass) - 1;
     pass &= pass - 1u;
-    const float4* tri = blk + (i >> 2) * kBlockWords + kBlockTris + 3 * (i & 3);
-    const float4 t0 = __ldg(tri), t1 = __ldg(tri + 1), t2 = __ldg(tri + 2);
-    const float q[3][3] = {{t0.x, t0.y, t0.z}, {t0.w, t1.x, t1.y}, {t1.z, t1.w, t2.x}};
-    float t, b1, b2;
-    if (!moller_trumbore(q, r, tmax, t, b1, b2)) continue;
+    if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED && KIND == BVHGPU_CLOSEST && !exact &&
+        tmax != pr.tmax) {
+      // tMax fell in this leaf: the pre-test's tMax condition again.
+      const float* bf = reinterpret_cast<const float*>(blk + (i >> 2) * kBlockWords) + (i & 3);
+      float m[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float lo = (__ldg(bf + 4 * a) - r.o[a]) * r.inv[a];
+        const float hi = (__ldg(bf + 4 * (3 + a)) - r.o[a]) * r.inv[a];
+        m[a] = fminf(lo, hi);
+      }
+      if (tmax < fmaxf(fmaxf(m[0], m[1]), m[2])) continue;
+    }
+    float t, b1, b2, prim;
+    if (!leaf_test<PROFILE>(leaf_tri(blk, i), r, exact, tmax, t, b1, b2, prim)) continue;
     any = true;
     if (KIND == BVHGPU_ANY) break;
+    if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
+      // Each accepted triangle overwrites the hit (triangle.cpp:243).
+      tmax = t;
+      static_cast<float4*>(v.out)[slot] = make_float4(prim, t, b1, b2);
+      continue;
+    }
     const uint32_t lane_bit = 1u << (i % v.gang);
     if (t < leaf_best || (winner >= 0 && t == leaf_best && !(lanes_at_best & lane_bit))) {
       // (a tie keeps the first one's t: it may be a zero of the other sign)
@@ -605,14 +628,64 @@ BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const
       winner = i;
       wu = b1;
       wv = b2;
-      wprim = t2.y;
+      wprim = prim;
     }
   }
-  if (KIND == BVHGPU_CLOSEST && winner >= 0) {
+  if (PROFILE == BVHGPU_PROFILE_FAST && KIND == BVHGPU_CLOSEST && winner >= 0) {
     tmax = leaf_best;
     static_cast<float4*>(v.out)[slot] = make_float4(wprim, leaf_best, wu, wv);
   }
   return any;
+}
+
+// The full tests of a pool's any-hit leaf step: the (ray, triangle) pairs that
+// passed the cheap test, 32 at a time, one per lane, whichever ray they belong
+// to. About one triangle per leaf visit passes, so the step's up to 32 rays
+// have about as many pairs, where a loop per ray runs as long as the ray with
+// most of them (three to four, with 8 of 32 lanes busy). pass: the lane's
+// candidates of pool ray j. Every lane of the warp calls it; returns whether
+// the lane's ray was hit. Instrumented profile: 1M-triangle frame 4.54 -> 4.50
+// ms, 12 scenes 711 -> 700 us, Q8 frame 3.03 -> 2.92 ms. The fast profile keeps
+// the loop per ray (per-ray calls 1.55 against 1.59 ms: its cheap test leaves
+// more triangles, and the pairs read every triangle a second time).
+template <int PROFILE, typename SRC, typename POOL>
+BVHGPU_DEV bool pool_pairs(const SRC& p, const POOL& P, int j, uint32_t pass, int lane) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  const int mine = __popc(pass);
+  int incl = mine;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int x = __shfl_up_sync(FULL, incl, d);
+    if (lane >= d) incl += x;
+  }
+  const int total = __shfl_sync(FULL, incl, 31), first = incl - mine;
+  int at = first;
+  bool hit = false;
+  for (int base = 0; base < total; base += 32) {
+    while (pass && at < base + 32) {
+      const int i = __ffs(pass) - 1;
+      pass &= pass - 1u;
+      P.pairs[at - base] = (uint16_t)(j | (i << 8));
+      ++at;
+    }
+    __syncwarp();
+    bool h = false;
+    if (base + lane < total) {
+      const int q = P.pairs[lane];
+      const PoolRay pr = P.ray(q & 0xFF);
+      const float4 c = P.c[q & 0xFF];
+      const PackView& v = p.view((pr.bits >> 4) & 0xFFu);
+      const float4* blk = leaf_blocks(v, P.state[q & 0xFF].x);
+      const bool exact = PROFILE == BVHGPU_PROFILE_INSTRUMENTED && ((pr.bits >> 3) & 1u);
+      float t, b1, b2, prim;
+      h = leaf_test<PROFILE>(leaf_tri(blk, q >> 8), leaf_ray<PROFILE>(pr, c), exact, pr.tmax, t, b1,
+                             b2, prim);
+    }
+    const unsigned hits = __ballot_sync(FULL, h);
+    const int lo = max(first - base, 0), hi = min(first + mine - base, 32);
+    if (lo < hi && ((hits >> lo) & (FULL >> (32 - (hi - lo))))) hit = true;
+  }
+  return hit;
 }
 
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
@@ -621,6 +694,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
   using F = PackFmt<NM, FMT>;
   constexpr unsigned FULL = 0xFFFFFFFFu;
   constexpr int K = kPoolRays;
+  constexpr bool kPairs = KIND == BVHGPU_ANY && PROFILE == BVHGPU_PROFILE_INSTRUMENTED;
   constexpr bool kLoose = FMT == kFmtQ8 && PROFILE == BVHGPU_PROFILE_INSTRUMENTED &&
                           KIND == BVHGPU_ANY;
   constexpr bool kCull =
@@ -638,7 +712,8 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
     P.c = P.b + K;
     P.state = reinterpret_cast<uint2*>(P.c + K);
     P.stack = reinterpret_cast<typename W::T*>(P.state + K);
-    P.list = reinterpret_cast<uint8_t*>(P.stack + (size_t)p.levels * K);
+    P.pairs = reinterpret_cast<uint16_t*>(P.stack + (size_t)p.levels * K);
+    P.list = reinterpret_cast<uint8_t*>(P.pairs + 32);
   }
   // Lists 0 node rays, 1 leaf rays, 2 free slots; each grows and shrinks at
   // its end, so rays that went together last stay together.
@@ -706,29 +781,42 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
     } else if (n_leaf > 0) {
       m = min(32, n_leaf);
       n_leaf -= m;
-      if ((int)lane < m) {
-        j = P.list[K + n_leaf + (int)lane];
+      const bool on = (int)lane < m;
+      uint32_t pass = 0;
+      bool hit = false;
+      if (on) j = P.list[K + n_leaf + (int)lane];
+      if (kPairs) {
+        if (on) {
+          const PoolRay r = P.ray(j);
+          const uint32_t e = P.state[j].x;
+          pass = leaf_candidates<PROFILE>(leaf_blocks(p.view((r.bits >> 4) & 0xFFu), e),
+                                          leaf_count(e), r, P.c[j]);
+        }
+        hit = pool_pairs<PROFILE>(p, P, j, pass, (int)lane);
+      }
+      if (on) {
         PoolRay r = P.ray(j);
         const PackView& v = p.view((r.bits >> 4) & 0xFFu);
-        const float4 c = P.c[j];
         const uint2 st = P.state[j];
         uint32_t sp = st.y, e;
-        float tmax = r.tmax;
-        const bool hit = pool_leaf<PROFILE, KIND>(v, st.x, r, c, tmax);
-        if (KIND == BVHGPU_CLOSEST && hit) {
-          r.tmax = tmax;
-          r.bits |= 1u << 12;
-          P.a[j].w = tmax;
-          P.b[j].w = __uint_as_float(r.bits);
+        if (!kPairs) {
+          float tmax = r.tmax;
+          hit = pool_leaf<PROFILE, KIND>(v, st.x, r, P.c[j], tmax);
+          if (KIND == BVHGPU_CLOSEST && hit) {
+            r.tmax = tmax;
+            r.bits |= 1u << 12;
+            P.a[j].w = tmax;
+            P.b[j].w = __uint_as_float(r.bits);
+          }
         }
         next = 2;
         if (KIND == BVHGPU_ANY && hit) {
-          static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 1;
+          static_cast<uint8_t*>(v.out)[__float_as_uint(P.c[j].w)] = 1;
         } else if (pool_take<NM, FMT, ORDERED, kCull>(v, P.stack + j, K, r, 0u, 0u, false, sp, e)) {
           P.state[j] = make_uint2(e, sp);
           next = (int)(e >> 31);
         } else if (KIND == BVHGPU_ANY) {
-          static_cast<uint8_t*>(v.out)[__float_as_uint(c.w)] = 0;
+          static_cast<uint8_t*>(v.out)[__float_as_uint(P.c[j].w)] = 0;
         }
       }
     } else if (drained) {

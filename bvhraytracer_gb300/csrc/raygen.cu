@@ -38,19 +38,32 @@ __device__ __forceinline__ V3 cross(V3 x, V3 y) {
 // glm::normalize: v * inversesqrt(dot(v, v)), inversesqrt(x) = 1 / sqrt(x)
 __device__ __forceinline__ V3 normalize(V3 v) { return mul(v, 1.0f / sqrtf(dot(v, v))); }
 
-__device__ __forceinline__ void store_ray(bvhgpu_ray_t* out, uint64_t i, V3 o, float tmax, V3 d) {
+// One ray record. A pixel's rays lie next to one another, so the lanes of a
+// warp store 32 ao_samples bytes apart: as two 16-byte stores every 32-byte
+// sector goes to L2 twice, half filled. WIDE: the buffer is 32-byte aligned.
+template <bool WIDE>
+__device__ __forceinline__ void store_record(bvhgpu_ray_t* out, uint64_t i, float4 a, float4 b) {
+  if (WIDE) {
+    stg32(out + i, a, b);
+    return;
+  }
   float4* q = reinterpret_cast<float4*>(out + i);
-  q[0] = make_float4(o.x, o.y, o.z, tmax);
-  q[1] = make_float4(d.x, d.y, d.z, 0.0f);
+  q[0] = a;
+  q[1] = b;
 }
 
+template <bool WIDE>
+__device__ __forceinline__ void store_ray(bvhgpu_ray_t* out, uint64_t i, V3 o, float tmax, V3 d) {
+  store_record<WIDE>(out, i, make_float4(o.x, o.y, o.z, tmax), make_float4(d.x, d.y, d.z, 0.0f));
+}
+
+template <bool WIDE>
 __device__ __forceinline__ void store_inactive(bvhgpu_ray_t* out, uint64_t i) {
   const float nan = __int_as_float(0x7FC00000);
-  float4* q = reinterpret_cast<float4*>(out + i);
-  q[0] = make_float4(nan, nan, nan, 0.0f);
-  q[1] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+  store_record<WIDE>(out, i, make_float4(nan, nan, nan, 0.0f), make_float4(1.0f, 1.0f, 1.0f, 0.0f));
 }
 
+template <bool WIDE>
 __global__ void camera_rays_kernel(CameraArgs c, bvhgpu_ray_t* out) {
   const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= c.n) return;
@@ -96,7 +109,7 @@ __global__ void camera_rays_kernel(CameraArgs c, bvhgpu_ray_t* out) {
   t.z = (m[2] * ox + m[6] * oy) + (m[10] * oz + m[14] * ow);
   const V3 pos = v3(c.pos[0], c.pos[1], c.pos[2]);
   const V3 target = add(pos, t);
-  store_ray(out, p, pos, c.tmax, sub(target, pos));
+  store_ray<WIDE>(out, p, pos, c.tmax, sub(target, pos));
 }
 
 // FNV-1a, 64 bit, over the 8 little-endian bytes of x: std::hash<size_t> of
@@ -122,6 +135,7 @@ __device__ __forceinline__ float unit24(uint64_t h) {
   return (float)(uint32_t)(h >> 40) * (1.0f / 16777216.0f);
 }
 
+template <bool WIDE>
 __global__ void secondary_rays_kernel(SceneDev sc, SecondaryArgs a) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -131,8 +145,8 @@ __global__ void secondary_rays_kernel(SceneDev sc, SecondaryArgs a) {
   if (prim < 0 || (uint32_t)prim >= a.n_prims || a.prim_slot[prim] == 0xFFFFFFFFu) {
     // Missed primary ray: inactive secondaries (NaN origin), like
     // rays[j].pos = NaN in cameraFast.h:524-528.
-    if (a.shadow) store_inactive(a.shadow, i);
-    for (int k = 0; k < S; ++k) store_inactive(a.ao, i * S + k);
+    if (a.shadow) store_inactive<WIDE>(a.shadow, i);
+    for (int k = 0; k < S; ++k) store_inactive<WIDE>(a.ao, i * S + k);
     return;
   }
   const uint32_t slot = a.prim_slot[prim];
@@ -154,7 +168,7 @@ __global__ void secondary_rays_kernel(SceneDev sc, SecondaryArgs a) {
   if (a.shadow) {
     const V3 v = sub(v3(a.light[0], a.light[1], a.light[2]), org);
     const float dist = sqrtf(dot(v, v));
-    store_ray(a.shadow, i, org, dist, mul(v, 1.0f / dist));
+    store_ray<WIDE>(a.shadow, i, org, dist, mul(v, 1.0f / dist));
   }
   if (S == 0) return;
   if (a.sampling == BVHGPU_AO_REFERENCE) {
@@ -170,7 +184,7 @@ __global__ void secondary_rays_kernel(SceneDev sc, SecondaryArgs a) {
       const float theta = (float)(2.0 * 3.14159265358979323846 * (double)v);
       V3 r = v3(sinf(phi) * cosf(theta), sinf(phi) * sinf(theta), cosf(phi));
       if (dot(r, nrm) <= 0.0f) r = v3(-r.x, -r.y, -r.z);
-      store_ray(a.ao, i * S + k, org, a.ao_length, r);
+      store_ray<WIDE>(a.ao, i * S + k, org, a.ao_length, r);
     }
     return;
   }
@@ -185,7 +199,7 @@ __global__ void secondary_rays_kernel(SceneDev sc, SecondaryArgs a) {
     const float ph = 6.2831853071795864769f * u2;
     const float lx = rr * cosf(ph), ly = rr * sinf(ph), lz = sqrtf(fmaxf(0.0f, 1.0f - u1));
     const V3 dir = add(add(mul(tg, lx), mul(bt, ly)), mul(nrm, lz));
-    store_ray(a.ao, i * S + k, org, a.ao_length, dir);
+    store_ray<WIDE>(a.ao, i * S + k, org, a.ao_length, dir);
   }
 }
 
@@ -201,13 +215,16 @@ __global__ void ao_factor_kernel(const uint8_t* occluded, uint64_t n, int sample
 
 cudaError_t launch_camera_rays(const CameraArgs& c, bvhgpu_ray_t* out, cudaStream_t s) {
   if (c.n == 0) return cudaSuccess;
-  camera_rays_kernel<<<(unsigned)((c.n + 255) / 256), 256, 0, s>>>(c, out);
+  auto k = ((uintptr_t)out & 31) ? camera_rays_kernel<false> : camera_rays_kernel<true>;
+  k<<<(unsigned)((c.n + 255) / 256), 256, 0, s>>>(c, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_secondary_rays(const SceneDev& sc, const SecondaryArgs& a, cudaStream_t s) {
   if (a.n == 0) return cudaSuccess;
-  secondary_rays_kernel<<<(unsigned)((a.n + 127) / 128), 128, 0, s>>>(sc, a);
+  auto k = (((uintptr_t)a.shadow | (uintptr_t)a.ao) & 31) ? secondary_rays_kernel<false>
+                                                           : secondary_rays_kernel<true>;
+  k<<<(unsigned)((a.n + 127) / 128), 128, 0, s>>>(sc, a);
   return cudaGetLastError();
 }
 

@@ -19,6 +19,8 @@
 // results to slot perm[i].
 #include "reorder.cuh"
 
+#include "device_common.cuh"
+
 namespace bvhgpu {
 namespace dev {
 
@@ -77,6 +79,44 @@ __device__ __forceinline__ uint32_t dir_bin(float ox, float dx, float dy, float 
   return (uint32_t)((face * k + cell(u, aw, k)) * k + cell(v, aw, k));
 }
 
+// A ray's record; wide: the buffer is 32-byte aligned.
+__device__ __forceinline__ void load_record(const bvhgpu_ray_t* r, bool wide, float4& a, float4& b) {
+  if (wide) {
+    ldg32(r, a, b);
+  } else {
+    a = __ldg(reinterpret_cast<const float4*>(r));
+    b = __ldg(reinterpret_cast<const float4*>(r) + 1);
+  }
+}
+
+// Bins and counts of one chunk. The loads of eight rays per thread are in
+// flight at once.
+__device__ __forceinline__ void bin_chunk(const bvhgpu_ray_t* rays, uint64_t begin, int count, int k,
+                                          uint16_t* bins, uint32_t* hist) {
+  const bool wide = ((uintptr_t)rays & 31) == 0;
+  constexpr int U = 8;
+  for (int i0 = (int)threadIdx.x; i0 < count; i0 += U * kThreads) {
+    float ox[U];
+    float4 b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kThreads;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      b[u] = a;
+      if (i < count) load_record(rays + begin + i, wide, a, b[u]);
+      ox[u] = a.x;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * kThreads;
+      if (i >= count) break;
+      const uint32_t bin = dir_bin(ox[u], b[u].x, b[u].y, b[u].z, k);
+      bins[begin + i] = (uint16_t)bin;
+      atomicAdd(&hist[bin], 1u);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kThreads) bin_count_kernel(const bvhgpu_ray_t* rays, uint64_t n,
                                                              int k, Scratch s, uint64_t blocks) {
   extern __shared__ uint32_t hist[];
@@ -84,14 +124,7 @@ __global__ void __launch_bounds__(kThreads) bin_count_kernel(const bvhgpu_ray_t*
   for (int i = threadIdx.x; i < nb; i += kThreads) hist[i] = 0;
   __syncthreads();
   const uint64_t begin = (uint64_t)blockIdx.x * kChunk;
-  const uint64_t end = begin + kChunk < n ? begin + kChunk : n;
-  for (uint64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-    const float4* p = reinterpret_cast<const float4*>(rays + i);
-    const float4 a = __ldg(p), b = __ldg(p + 1);
-    const uint32_t bin = dir_bin(a.x, b.x, b.y, b.z, k);
-    s.bins[i] = (uint16_t)bin;
-    atomicAdd(&hist[bin], 1u);
-  }
+  bin_chunk(rays, begin, (int)(n - begin < kChunk ? n - begin : kChunk), k, s.bins, hist);
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += kThreads)
     s.counts[(uint64_t)i * blocks + blockIdx.x] = hist[i];
@@ -143,19 +176,79 @@ __global__ void __launch_bounds__(kThreads) scan_totals_kernel(Scratch s, int nb
   block_scan_inplace(s.base, (uint64_t)nb);
 }
 
+// Writes the input indices begin .. begin + count - 1 of one chunk to their
+// positions: the chunk is sorted by bin in shared memory first, so that a
+// warp's stores fall into the few runs of its bins instead of 32 sectors.
+// start[bin] (shared, nb words) holds the global position of the chunk's first
+// ray of each bin; work: nb + 2 kChunk / 4 words of shared memory after it.
+__device__ __forceinline__ void scatter_chunk(const uint16_t* bins, uint32_t begin, int count,
+                                              int nb, uint32_t* start, uint32_t* perm) {
+  uint32_t* first = start + nb;  // the bins' first places in the chunk
+  uint16_t* sorted = reinterpret_cast<uint16_t*>(first + nb);
+  uint16_t* bin_at = sorted + kChunk;
+  constexpr int kPer = kChunk / kThreads;
+  __shared__ uint32_t warp_sums[kThreads / 32];
+  for (int i = threadIdx.x; i < nb; i += kThreads) first[i] = 0;
+  __syncthreads();
+  uint16_t bin[kPer], rank[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = k * kThreads + (int)threadIdx.x;
+    bin[k] = i < count ? bins[begin + i] : (uint16_t)0;
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = k * kThreads + (int)threadIdx.x;
+    if (i < count) rank[k] = (uint16_t)atomicAdd(&first[bin[k]], 1u);
+  }
+  __syncthreads();
+  // Exclusive scan of the counts: each thread a run of bins.
+  const int per = (nb + kThreads - 1) / kThreads;
+  const int lo = min((int)threadIdx.x * per, nb), hi = min(lo + per, nb);
+  uint32_t sum = 0;
+  for (int i = lo; i < hi; ++i) sum += first[i];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = sum;
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+    if (lane >= d) incl += y;
+  }
+  if (lane == 31) warp_sums[warp] = incl;
+  __syncthreads();
+  uint32_t at = incl - sum;
+  for (int w = 0; w < warp; ++w) at += warp_sums[w];
+  for (int i = lo; i < hi; ++i) {
+    const uint32_t c = first[i];
+    first[i] = at;
+    at += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = k * kThreads + (int)threadIdx.x;
+    if (i < count) {
+      const uint32_t pos = first[bin[k]] + rank[k];
+      sorted[pos] = (uint16_t)i;
+      bin_at[pos] = bin[k];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < count; i += kThreads) {
+    const uint32_t b = bin_at[i];
+    perm[start[b] + (uint32_t)i - first[b]] = begin + sorted[i];
+  }
+}
+constexpr size_t scatter_smem(int nb) { return (size_t)nb * 8 + (size_t)kChunk * 4; }
+
 __global__ void __launch_bounds__(kThreads) scatter_kernel(uint64_t n, int k, Scratch s,
                                                            uint64_t blocks, uint32_t* perm) {
-  extern __shared__ uint32_t cursor[];
+  extern __shared__ uint32_t start[];
   const int nb = bins_for(k);
   for (int i = threadIdx.x; i < nb; i += kThreads)
-    cursor[i] = s.base[i] + s.counts[(uint64_t)i * blocks + blockIdx.x];
-  __syncthreads();
+    start[i] = s.base[i] + s.counts[(uint64_t)i * blocks + blockIdx.x];
   const uint64_t begin = (uint64_t)blockIdx.x * kChunk;
-  const uint64_t end = begin + kChunk < n ? begin + kChunk : n;
-  for (uint64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-    const uint32_t pos = atomicAdd(&cursor[s.bins[i]], 1u);
-    perm[pos] = (uint32_t)i;
-  }
+  scatter_chunk(s.bins, (uint32_t)begin, (int)(n - begin < kChunk ? n - begin : kChunk), nb, start,
+                perm);
 }
 
 // Job of grid chunk c: the last job whose first chunk is <= c.
@@ -177,14 +270,7 @@ __global__ void __launch_bounds__(kThreads) seg_bin_count_kernel(const __grid_co
   for (int i = threadIdx.x; i < nb; i += kThreads) hist[i] = 0;
   __syncthreads();
   const uint64_t begin = (uint64_t)chunk * kChunk;
-  const uint64_t end = begin + kChunk < J.n ? begin + kChunk : J.n;
-  for (uint64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-    const float4* p = reinterpret_cast<const float4*>(J.rays + i);
-    const float4 a = __ldg(p), b = __ldg(p + 1);
-    const uint32_t bin = dir_bin(a.x, b.x, b.y, b.z, t.k);
-    J.bins[i] = (uint16_t)bin;
-    atomicAdd(&hist[bin], 1u);
-  }
+  bin_chunk(J.rays, begin, (int)(J.n - begin < kChunk ? J.n - begin : kChunk), t.k, J.bins, hist);
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += kThreads)
     J.counts[(uint64_t)i * J.nchunks + chunk] = hist[i];
@@ -204,19 +290,15 @@ __global__ void __launch_bounds__(kThreads) seg_scan_totals_kernel(const __grid_
 }
 
 __global__ void __launch_bounds__(kThreads) seg_scatter_kernel(const __grid_constant__ SegTable t) {
-  extern __shared__ uint32_t cursor[];
+  extern __shared__ uint32_t start[];
   const int nb = bins_for(t.k);
   const SegJob& J = t.jobs[seg_job_of(t, blockIdx.x)];
   const uint32_t chunk = blockIdx.x - J.first_chunk;
   for (int i = threadIdx.x; i < nb; i += kThreads)
-    cursor[i] = J.base[i] + J.counts[(uint64_t)i * J.nchunks + chunk];
-  __syncthreads();
-  const uint64_t begin = (uint64_t)chunk * kChunk;
-  const uint64_t end = begin + kChunk < J.n ? begin + kChunk : J.n;
-  for (uint64_t i = begin + threadIdx.x; i < end; i += kThreads) {
-    const uint32_t pos = atomicAdd(&cursor[J.bins[i]], 1u);
-    J.perm[pos] = (uint32_t)i;
-  }
+    start[i] = J.base[i] + J.counts[(uint64_t)i * J.nchunks + chunk];
+  const uint32_t begin = chunk * kChunk;
+  scatter_chunk(J.bins, begin, (int)(J.n - begin < kChunk ? J.n - begin : kChunk), nb, start,
+                J.perm);
 }
 
 }  // namespace
@@ -248,18 +330,16 @@ cudaError_t reorder_jobs(const SegTable& t, cudaStream_t st) {
   const int nb = bins_for(t.k);
   const size_t smem = (size_t)nb * 4;
   cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(seg_bin_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
+  const size_t sort_smem = scatter_smem(nb);
+  if (sort_smem > 48 * 1024) {
+    e = cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sort_smem);
     if (e != cudaSuccess) return e;
   }
   seg_bin_count_kernel<<<t.total_chunks, kThreads, smem, st>>>(t);
   seg_scan_bins_kernel<<<dim3(nb, t.n_jobs), kThreads, 0, st>>>(t);
   seg_scan_totals_kernel<<<t.n_jobs, kThreads, 0, st>>>(t);
-  seg_scatter_kernel<<<t.total_chunks, kThreads, smem, st>>>(t);
+  seg_scatter_kernel<<<t.total_chunks, kThreads, sort_smem, st>>>(t);
   return cudaGetLastError();
 }
 
@@ -277,18 +357,16 @@ cudaError_t reorder_rays(const bvhgpu_ray_t* rays, uint64_t n, int k, uint32_t* 
   const Scratch s = carve(scratch, n, k);
   const size_t smem = (size_t)nb * 4;
   cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(bin_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
+  const size_t sort_smem = scatter_smem(nb);
+  if (sort_smem > 48 * 1024) {
+    e = cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sort_smem);
     if (e != cudaSuccess) return e;
   }
   bin_count_kernel<<<(unsigned)blocks, kThreads, smem, st>>>(rays, n, k, s, blocks);
   scan_bins_kernel<<<nb, kThreads, 0, st>>>(s, blocks);
   scan_totals_kernel<<<1, kThreads, 0, st>>>(s, nb);
-  scatter_kernel<<<(unsigned)blocks, kThreads, smem, st>>>(n, k, s, blocks, perm);
+  scatter_kernel<<<(unsigned)blocks, kThreads, sort_smem, st>>>(n, k, s, blocks, perm);
   return cudaGetLastError();
 }
 

@@ -158,3 +158,23 @@ def test_many_scenes_on_the_packed_kernels(profile, reorder, any_order, each):
         else:
             assert torch.equal(got, ref)
         scene.status()
+
+
+@pytest.mark.parametrize("n", [2, 31, 4095, 4096, 4097, 12289])
+@pytest.mark.parametrize("k", [1, 10, 32])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_direction_order_chunks(n, k, offset):
+    """The direction sort at its chunk size (4,096 rays), few and many bins,
+    rays on 32-byte and on 16-byte boundaries, alone and as jobs."""
+    tris = S.clutter(20, 3)
+    scene = pkg.Scene(pkg.Bvh(tris, 8, 8))
+    flat = torch.zeros(8 * n + 4, dtype=torch.float32, device="cuda")
+    rays = flat[offset:offset + 8 * n].view(n, 8)
+    rays.copy_(_rays(tris, n, n + k, extreme=n > 100))
+    want = scene.trace(rays, kind="any", counters=True)["occluded"]
+    assert torch.equal(scene.trace(rays, kind="any", reorder=k)["occluded"], want)
+    out = [torch.full_like(want, 9) for _ in range(3)]
+    pkg.trace_jobs([(scene, rays, "any", o, k) for o in out])
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in out)
+    scene.status()
