@@ -257,8 +257,8 @@ static cudaError_t pack_scene(bvhgpu_scene* s) {
 
 // Whether a launch runs on the ray-pool kernel, which traces without counters
 // every ray kind, profile and scheme (results do not depend on the scheme).
-// The kernels of the schemes themselves run what it does not: counters and
-// step logs, save-distance closest hits, a capped traversal stack (their
+// The kernels of the schemes themselves run what it does not: counters (but
+// see counts_packed) and step logs, save-distance closest hits, a capped traversal stack (their
 // stacks hold one entry per pushed child, which is what the cap counts), the
 // staging wait of the failure-detection tests, node records whose boxes are
 // not ordered, Q8 ones whose boxes are not nested (imported trees), trees too
@@ -272,6 +272,14 @@ static bool scene_uses_pool(const bvhgpu_scene* s) {
 }
 static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
   return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&
+         scene_uses_pool(s);
+}
+// Counting traces that have a kernel on the packed scene: per-ray scheme,
+// instrumented profile. (The other schemes count in their own kernels, which
+// is what their step logs and tests are about.)
+static bool counts_packed(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
+  return c.count && c.scheme == BVHGPU_PER_RAY && c.profile == BVHGPU_PROFILE_INSTRUMENTED &&
+         !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&
          scene_uses_pool(s);
 }
 
@@ -336,7 +344,8 @@ static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
 // A trace on the packed scene.
 static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
                                cudaStream_t st) {
-  PoolQueue queue(s->device, a.n, c.pool_queue, st);
+  // Counting traces need no queue.
+  PoolQueue queue(s->device, c.count ? 0 : a.n, c.pool_queue, st);
   dev::OneScene p{};
   p.n = a.n;
   p.levels = std::max(1, s->layout.inner_levels);
@@ -347,6 +356,14 @@ static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const d
   const dev::PackedCfg cfg{s->layout.node_stride, s->layout.node_format, c.kind, c.profile,
                            c.any_order, a.out_index != nullptr, s->sm_count};
   cudaError_t e;
+  if (c.count) {
+    switch (cfg.nm) {
+      case 4: return dev::launch_counting<4>(p, a, cfg, st);
+      case 8: return dev::launch_counting<8>(p, a, cfg, st);
+      case 12: return dev::launch_counting<12>(p, a, cfg, st);
+      default: return dev::launch_counting<16>(p, a, cfg, st);
+    }
+  }
   switch (cfg.nm) {
     case 4: e = dev::launch_one_scene<4>(p, cfg, st); break;
     case 8: e = dev::launch_one_scene<8>(p, cfg, st); break;
@@ -373,7 +390,7 @@ static int launch(bvhgpu_scene_t s, const dev::TraceArgs& a, dev::LaunchCfg cfg,
   if (cfg.scheme == BVHGPU_STREAM && cfg.fmt != BVHGPU_NODES_FP32)
     return set_error(BVHGPU_ERR_UNSUPPORTED, "the stream scheme traverses FP32 nodes only");
   cudaError_t e;
-  if (uses_pool(s, a, cfg)) {
+  if (uses_pool(s, a, cfg) || counts_packed(s, a, cfg)) {
     e = launch_pool(s, a, cfg, st);
     return e == cudaSuccess ? BVHGPU_OK : cuda_error(e, "trace launch");
   }

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(128) pack_nodes_kernel(SceneDev sc, uint32_t n
       seq[6 + 2 * a + 1] = (uint32_t)(inv >> 32);
     }
   }
-  *reinterpret_cast<uint32_t*>(dst + D::COUNT) = (uint32_t)count;
+  *reinterpret_cast<uint32_t*>(dst + D::COUNT) = (uint32_t)count | (meta[2] >> 24) << 8;
 }
 
 struct LeafSource {
@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(128) pack_leaves_kernel(SceneDev sc, uint32_t 
     t[2] = make_float4(v[8], __uint_as_float(prim), 0.0f, 0.0f);
   }
   for (int k = 0; k < 4 && first == 0; ++k) b[6 * L + k] = 0.0f;
-  if (out) out[kBlockWords - 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (out)
+    out[kBlockWords - 1] = make_float4(
+        __uint_as_float(first == 0 ? (uint32_t)sc.leaf_depth[leaf] : 0u), 0.f, 0.f, 0.f);
 }
 
 template <int N, int FMT>

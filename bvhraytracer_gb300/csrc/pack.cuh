@@ -22,7 +22,7 @@ namespace dev {
 //   uint32 sorted[3][N]   the entries in the push sequence of each axis
 //   uint32 (N > 8: uint64) seq[3]   the child at each position (nibbles)
 //   N > 8: uint64 inv[3]            the position of each child (nibbles)
-//   uint32 count
+//   uint32 count         child count | depth << 8
 template <int N, int FMT>
 struct PackFmt {
   static constexpr int BOX = FMT == kFmtFP32 ? 0 : 16;
@@ -41,7 +41,7 @@ struct PackFmt {
 // before the bounds and the triangles themselves.
 //   words 0-5    bounds of the four triangles: lo.x lo.y lo.z hi.x hi.y hi.z
 //   words 6-17   triangle i at 6 + 3 i: 9 floats (p0 p1 p2), input id, 0, 0
-//   word 18      0
+//   word 18      first block: the leaf's depth (uint32), 0, 0, 0
 constexpr int kBlockWords = 19;
 constexpr int kBlockTris = 6;  // first triangle word
 constexpr uint32_t kMaxBlocks = 1u << kLeafCountShift;

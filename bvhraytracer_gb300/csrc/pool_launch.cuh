@@ -19,6 +19,8 @@ struct PackedCfg {
 // Width NM of one scene or many (pool_n*.cu, pool_jobs_n*.cu).
 template <int NM> cudaError_t launch_one_scene(OneScene& p, const PackedCfg& c, cudaStream_t s);
 template <int NM> cudaError_t launch_many_scenes(ManyScenes& p, const PackedCfg& c, cudaStream_t s);
+// The counting kernel for the rays of p, counters and histograms as in a.
+template <int NM> cudaError_t launch_counting(OneScene& p, TraceArgs a, const PackedCfg& c, cudaStream_t s);
 
 // Shared memory of an SM that the pools may take; the rest of its 256 KB is
 // L1, which the node records need.
@@ -132,6 +134,31 @@ inline cudaError_t launch_packed_fmt(SRC& p, const PackedCfg& c, cudaStream_t s)
   if (c.profile == F) return launch_packed<NM, F, A, FMT, false>(p, d, sms, s);
   return c.any_order ? launch_packed<NM, I, A, FMT, false>(p, d, sms, s)
                      : launch_packed<NM, I, A, FMT, true>(p, d, sms, s);
+}
+
+template <int NM, int KIND, int FMT>
+inline cudaError_t launch_count(OneScene& p, TraceArgs& a, cudaStream_t s) {
+  constexpr int kBlock = 128;  // 64: 329 us against 326
+  size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * kBlock;
+  a.block_hist = a.depth_hist != nullptr;
+  if (a.block_hist) smem += kHistBins * sizeof(uint32_t);
+  auto k = trace_count_kernel<NM, KIND, FMT>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  k<<<(unsigned)((p.n + kBlock - 1) / kBlock), kBlock, smem, s>>>(p, a);
+  return cudaGetLastError();
+}
+template <int NM>
+inline cudaError_t launch_count_width(OneScene& p, TraceArgs& a, const PackedCfg& c, cudaStream_t s) {
+  if (p.n == 0) return cudaSuccess;
+  if (c.kind == BVHGPU_CLOSEST)
+    return c.fmt == kFmtQ8 ? launch_count<NM, BVHGPU_CLOSEST, kFmtQ8>(p, a, s)
+                           : launch_count<NM, BVHGPU_CLOSEST, kFmtFP32>(p, a, s);
+  return c.fmt == kFmtQ8 ? launch_count<NM, BVHGPU_ANY, kFmtQ8>(p, a, s)
+                         : launch_count<NM, BVHGPU_ANY, kFmtFP32>(p, a, s);
 }
 
 template <int NM, typename SRC>

@@ -808,8 +808,9 @@ constexpr int kHistBins = 128 + 34;
 // Counting launches: one node visit (depth_count = depth | child count << 8,
 // as node_step returns it) into the per-depth histogram and childFullness
 // (compactNode.cpp:714-716), one leaf visit into the per-depth histogram and
-// primitiveFullness (compactNode.cpp:653-656). hist: the block's own
-// histogram in shared memory, or null: straight to global memory.
+// primitiveFullness (compactNode.cpp:653-656; leaf_depth: where the leaf's
+// depth is). hist: the block's own histogram in shared memory, or null:
+// straight to global memory.
 BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count, uint32_t* hist) {
   const int depth = min(depth_count & 0xFF, 63), fill = 128 + min(depth_count >> 8, 16);
   if (hist != nullptr) {
@@ -820,15 +821,15 @@ BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count, uint32_t* hist) 
   if (a.depth_hist) atomicAdd(a.depth_hist + depth, 1ull);
   if (a.fullness) atomicAdd(a.fullness + fill - 128, 1ull);
 }
-BVHGPU_DEV void count_leaf(const SceneDev& sc, const TraceArgs& a, uint32_t e, uint32_t* hist) {
+BVHGPU_DEV void count_leaf(const TraceArgs& a, const uint8_t* leaf_depth, uint32_t e,
+                           uint32_t* hist) {
   const int fill = 128 + 17 + (int)((e >> kLeafCountShift) & 15u) + 1;
   if (hist != nullptr) {
-    atomicAdd(hist + 64 + min((int)sc.leaf_depth[e & kLeafIndexMask], 63), 1u);
+    atomicAdd(hist + 64 + min((int)*leaf_depth, 63), 1u);
     atomicAdd(hist + fill, 1u);
     return;
   }
-  if (a.depth_hist)
-    atomicAdd(a.depth_hist + 64 + min((int)sc.leaf_depth[e & kLeafIndexMask], 63), 1ull);
+  if (a.depth_hist) atomicAdd(a.depth_hist + 64 + min((int)*leaf_depth, 63), 1ull);
   if (a.fullness) atomicAdd(a.fullness + fill - 128, 1ull);
 }
 
@@ -836,9 +837,9 @@ BVHGPU_DEV void count_leaf(const SceneDev& sc, const TraceArgs& a, uint32_t e, u
 // 64-bit atomics on global memory queue up behind one another in L2. A block
 // adds to its own copy in shared memory (32-bit: a block has at most 256 rays)
 // and to global memory once per bin at its end: 640 x 360 primary and shadow
-// rays on a 251k-triangle N16L16 tree 4.31 -> 0.36 ms, now bound by the
-// traversal itself. The persistent kernel, whose blocks take any number of
-// rays, keeps the 64-bit atomics on global memory.
+// rays on a 251k-triangle N16L16 tree 4.31 -> 0.36 ms. The persistent kernel,
+// whose blocks take any number of rays, keeps the 64-bit atomics on global
+// memory.
 BVHGPU_DEV void hist_clear(uint32_t* hist) {
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0u;
   __syncthreads();
@@ -862,10 +863,9 @@ BVHGPU_DEV bvhgpu_ray_t load_ray(const bvhgpu_ray_t* rays, uint64_t i) {
   return r;
 }
 
-template <bool COUNT>
-BVHGPU_DEV void flush_counters(const TraceArgs& a, uint64_t rid, const Counters& c) {
-  if (!COUNT || a.counters == nullptr) return;
-  uint32_t* o = a.counters + out_slot(a, rid) * BVHGPU_COUNTERS_PER_RAY;
+BVHGPU_DEV void store_counters(const TraceArgs& a, uint64_t slot, const Counters& c) {
+  if (a.counters == nullptr) return;
+  uint32_t* o = a.counters + slot * BVHGPU_COUNTERS_PER_RAY;
   o[0] = c.node_visits;
   o[1] = c.leaf_visits;
   o[2] = c.box_tests;
@@ -874,6 +874,10 @@ BVHGPU_DEV void flush_counters(const TraceArgs& a, uint64_t rid, const Counters&
   o[5] = c.tri_hits;
   o[6] = c.max_stack;
   o[7] = 0;
+}
+template <bool COUNT>
+BVHGPU_DEV void flush_counters(const TraceArgs& a, uint64_t rid, const Counters& c) {
+  if (COUNT) store_counters(a, out_slot(a, rid), c);
 }
 
 template <int KIND>
@@ -927,7 +931,7 @@ BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t r
     const uint32_t e = stack[sp * stride];
     if (DIST && dstack[sp * stride] > tmax) continue;
     if (e & kLeafBit) {
-      if (COUNT) count_leaf(sc, a, e, hist);
+      if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, hist);
       bool h = leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr);
       if (h) {
         hit = true;
@@ -1190,7 +1194,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
       if (log && set_insert(set, 2 * P, e))
         atomicAdd(is_node ? &ctl->unique_nodes : &ctl->unique_leaves, 1);
       auto leaf_visit = [&](uint32_t le) {
-        if (COUNT) count_leaf(sc, a, le, hist);
+        if (COUNT) count_leaf(a, sc.leaf_depth + (le & kLeafIndexMask), le, hist);
         Best best;
         best.leaf = best_leaf[ray];
         best.lane = (int)(int8_t)(misc & 0xFF);
@@ -1674,7 +1678,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
       if (active && sp > 0) {
         --sp;
         const uint32_t e = stack[sp * stride];
-        if (COUNT) count_leaf(sc, a, e, nullptr);
+        if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, nullptr);
         if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
           hit = true;
           if (KIND == BVHGPU_ANY) sp = 0;
@@ -1685,7 +1689,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
         --sp;
         const uint32_t e = stack[sp * stride];
         if (e & kLeafBit) {
-          if (COUNT) count_leaf(sc, a, e, nullptr);
+          if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, nullptr);
           if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
             hit = true;
             if (KIND == BVHGPU_ANY) sp = 0;

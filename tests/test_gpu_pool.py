@@ -40,7 +40,8 @@ def _same(scene, rays, **kw):
     for kind in ("closest", "any"):
         key = "hits" if kind == "closest" else "occluded"
         for profile in ("instrumented", "fast"):
-            want = scene.trace(rays, kind=kind, profile=profile, counters=True)[key]
+            want = scene.trace(rays, kind=kind, profile=profile, scheme="persistent",
+                               counters=True)[key]
             for order in ({}, {"any_order": True}) if kind == "any" else ({},):
                 got = scene.trace(rays, kind=kind, profile=profile, **kw, **order)[key]
                 a, b = got.view(torch.uint8), want.view(torch.uint8)
@@ -177,4 +178,32 @@ def test_direction_order_chunks(n, k, offset):
     pkg.trace_jobs([(scene, rays, "any", o, k) for o in out])
     torch.cuda.synchronize()
     assert all(torch.equal(o, want) for o in out)
+    scene.status()
+
+
+@pytest.mark.parametrize("n,l,fmt", [(2, 1, "fp32"), (4, 16, "fp32"), (5, 7, "q8"), (8, 8, "fp32"),
+                                     (9, 13, "fp32"), (12, 5, "q8"), (16, 16, "fp32"),
+                                     (16, 16, "q8")])
+@pytest.mark.parametrize("rays", [1, 127, 129, 30001])
+def test_counting_traces(n, l, fmt, rays):
+    """Counters, histograms and results of the packed counting kernel against
+    the persistent kernel's, which reads the general records: all equal, with
+    and without histograms, in any ray order."""
+    tris = S.clutter(20, 4)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    d = _rays(tris, rays, rays + l, extreme=rays > 200)
+    for kind in ("closest", "any"):
+        key = "hits" if kind == "closest" else "occluded"
+        want = scene.trace(d, kind=kind, scheme="persistent", counters=True, depth_hist=True)
+        for opts in ({"depth_hist": True}, {"depth_hist": True, "reorder": 3}, {}):
+            got = scene.trace(d, kind=kind, counters=True, **opts)
+            for k in ("counters", "depth_hist", "fullness") if "depth_hist" in opts else ("counters",):
+                assert torch.equal(got[k], want[k]), (kind, opts, k)
+            a, b = got[key], want[key]
+            if kind == "closest":  # a NaN of a degenerate ray matches any NaN
+                assert torch.equal(a[:, 0].contiguous().view(torch.int32), b[:, 0].contiguous().view(torch.int32))
+                a, b = a[:, 1:], b[:, 1:]
+                assert torch.equal(torch.isnan(a), torch.isnan(b))
+                a, b = (torch.where(torch.isnan(x), 0.0, x).view(torch.int32) for x in (a, b))
+            assert torch.equal(a, b), (kind, opts)
     scene.status()
