@@ -649,9 +649,11 @@ def run_ours(a):
                     "matches_device_results": bool(e2e_ok)},
             "cpu_baseline": cpu,
             "clocks": clocks,
-            # per trace call: one traversal launch, plus four reorder passes
-            # (bin, scan, scan, scatter) when the plan groups the rays first
-            "gpu_launches": sum(1 + (4 if o.get("reorder") else 0) for _, o in chosen) * a.steps,
+            # per trace call: four reorder passes (bin, scan, scan, scatter) and the
+            # trace when the plan groups the rays first; else one launch, or for
+            # more than 2^18 rays the plan kernel and the two kernels it chooses from
+            "gpu_launches": sum(5 if o.get("reorder") else 3 if int(r.shape[0]) > 1 << 18 else 1
+                                for (_, o), r in zip(chosen, (primary, shadow, ao))) * a.steps,
         }
         print(json.dumps(line))
     if world > 1:

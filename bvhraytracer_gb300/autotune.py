@@ -9,7 +9,9 @@ persistent with its refill threshold and divergence policy), stack placement
 (reorder), node format (FP32 / Q8) and how many top levels are staged in
 shared memory. Every
 candidate gives the same hits (the kernels are bit-exact with one another and
-Q8 keeps hit sets identical), so the choice only changes speed.
+Q8 keeps hit sets identical), so the choice only changes speed. Scenes that
+trace on the packed records run the same kernels in every scheme, policy and
+stack placement; there reorder, any_order, the node format and (N, L) decide.
 """
 from __future__ import annotations
 
@@ -37,7 +39,7 @@ DEFAULT_OPTIONS = (
     # any-hit batches only: child-index push order
     {"scheme": "persistent", "policy": 2, "refill": 24, "reorder": 10, "any_order": True},
     {"scheme": "persistent", "policy": 2, "refill": 16, "any_order": True},
-    # any-hit batches only: two leaves set aside per lane, tested per lane / warp-wide
+    # any-hit batches only: two leaves set aside per lane
     {"scheme": "persistent", "policy": 3, "refill": 16, "reorder": 10, "any_order": True},
     {"scheme": "persistent", "policy": 4, "refill": 24, "reorder": 10, "any_order": True},
 )

@@ -204,8 +204,7 @@ static int check_smem_fit(const dev::LaunchCfg& cfg, int cap) {
       dev::stream_smem_bytes(cfg.packet, cap, cfg.count) > 227 * 1024)
     return set_error(BVHGPU_ERR_UNSUPPORTED,
                      "stream packet does not fit shared memory for this tree depth");
-  // persistent scheme: plus up to 8 KB of staged top levels and 6 KB of ray
-  // records (policy 3)
+  // persistent scheme: plus up to 8 KB of staged top levels and 6 KB kept free
   const size_t extra = cfg.scheme == BVHGPU_PERSISTENT ? 8192 + 128 * 48 : 0;
   if (cfg.scheme != BVHGPU_STREAM &&
       (size_t)cap * 128 * 4 * (cfg.save_distance ? 2 : 1) + extra > 227 * 1024)

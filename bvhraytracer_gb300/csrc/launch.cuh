@@ -15,8 +15,7 @@ struct LaunchCfg {
   int block = 128;      // per-ray scheme threads per block
   int packet = 256;     // stream scheme rays per block
   int policy = 0;       // persistent scheme: 0 while-while, 1 if-if, 2 speculative any-hit,
-                        // 3 the same with two leaves per lane, 4 as 3 with the leaves
-                        // tested warp-wide
+                        // 3 and 4 the same with two leaves per lane
   int refill_min = 8;   // persistent scheme: idle lanes that trigger a refill
   unsigned long long* queue = nullptr;  // persistent scheme: queue head
   bool queue_cleared = false;  // true: the caller zeroed the head already
@@ -28,12 +27,10 @@ struct LaunchCfg {
   uint32_t top_nodes = 0;       // persistent scheme: inner records staged in shared memory
   uint32_t stall_bytes = 0;     // failure-detection tests (see bvhgpu_scene_inject_stall)
   bool save_distance = false;   // per-ray scheme: save-distance traversal (closest hits)
+  bool stack_local = false;     // accepted and checked; the stacks are in shared memory always
   int reorder = 0;              // > 0: group rays into 6 reorder^2 direction bins first
-  bool stack_local = false;     // per-ray scheme: stacks in local memory (cap <= kLocalStack)
   bool any_order = false;       // any-hit rays without counters: child-index push order
 };
-
-constexpr int kLocalStack = 64;  // entries of the local-memory stack variant
 
 template <typename K>
 inline cudaError_t set_smem(K kernel, size_t bytes) {
@@ -59,32 +56,27 @@ inline cudaError_t launch_one(const SceneDev& sc, TraceArgs a, const LaunchCfg& 
     // never dropped: save-distance any-hit traversal is the plain one.
     constexpr bool kDist = KIND == BVHGPU_CLOSEST;
     const bool dist = kDist && cfg.save_distance;
-    const bool local = cfg.stack_local && !dist && !COUNT && a.stack_cap <= kLocalStack;
-    const size_t smem =
-        local ? 0 : add_block_hist(a, COUNT, (size_t)a.stack_cap * bs * 4 * (dist ? 2 : 1));
+    const size_t smem = add_block_hist(a, COUNT, (size_t)a.stack_cap * bs * 4 * (dist ? 2 : 1));
     auto k = dist ? trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, kDist>
-             : local ? trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false, (COUNT ? 0 : kLocalStack)>
-                     : trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false>;
+                  : trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false>;
     cudaError_t e = set_smem(k, smem);
     if (e != cudaSuccess) return e;
     const uint64_t grid = (a.n + bs - 1) / bs;
     k<<<(unsigned)grid, bs, smem, s>>>(sc, a);
   } else if (cfg.scheme == BVHGPU_PERSISTENT) {
     const int bs = 128;
-    // Policies 2 to 4 change the order of leaf tests, which only any-hit
+    // Policies 2 to 4 (4 is 3: testing the set-aside leaves of a warp together
+    // was the slower form) change the order of leaf tests, which only any-hit
     // rays without counters may do; the others fall back to policy 0.
     constexpr bool kSpec = KIND == BVHGPU_ANY && !COUNT;
-    const bool coop = cfg.policy == 4 && kSpec;
     const size_t smem = (size_t)a.stack_cap * bs * 4 +
-                        ((size_t)cfg.top_nodes * NodeFmt<NM, FMT>::REC + 15) / 16 * 16 +
-                        (coop ? (size_t)bs * kRayRecWords * 4 : 0);
+                        ((size_t)cfg.top_nodes * NodeFmt<NM, FMT>::REC + 15) / 16 * 16;
     auto k = cfg.policy == 1 ? trace_persistent_kernel<NM, PROFILE, KIND, COUNT, 1, FMT>
              : (cfg.policy == 2 && kSpec)
                  ? trace_persistent_kernel<NM, PROFILE, KIND, COUNT, (kSpec ? 2 : 0), FMT>
-             : (cfg.policy == 3 && kSpec)
+             : (cfg.policy >= 3 && kSpec)
                  ? trace_persistent_kernel<NM, PROFILE, KIND, COUNT, (kSpec ? 3 : 0), FMT>
-             : coop ? trace_persistent_kernel<NM, PROFILE, KIND, COUNT, (kSpec ? 4 : 0), FMT>
-                    : trace_persistent_kernel<NM, PROFILE, KIND, COUNT, 0, FMT>;
+                 : trace_persistent_kernel<NM, PROFILE, KIND, COUNT, 0, FMT>;
     cudaError_t e = set_smem(k, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

@@ -197,15 +197,19 @@ typedef struct {
 
 typedef struct {
   int32_t kind;      /* BVHGPU_CLOSEST / BVHGPU_ANY */
-  int32_t scheme;    /* BVHGPU_PER_RAY / BVHGPU_STREAM */
+  int32_t scheme;    /* BVHGPU_PER_RAY / BVHGPU_STREAM / BVHGPU_PERSISTENT. The results do
+                        not depend on it. Traces without counters of a scene whose boxes
+                        are ordered (Q8: and nested), without a stack limit, run on the
+                        packed scene in every scheme, and workgroup, block, policy, refill
+                        and stack_local then change nothing; the scheme's own kernel
+                        records counters (per-ray: on the packed scene too) and step
+                        logs, and runs every other scene. */
   int32_t profile;   /* BVHGPU_PROFILE_* */
   int32_t workgroup; /* stream scheme: packet = workgroup^2 rays (8, 16); 0 = 16 */
   int32_t block;     /* per-ray scheme: threads per block (32, 64, 128; 0 = 128) */
   int32_t policy;    /* persistent scheme: 0 while-while, 1 if-if, 2 while-while with
-                        one leaf per lane set aside, 3 the same with up to two leaves per
-                        lane, 4 as 3 with the warp's set-aside leaves tested as one pool
-                        of (ray, triangle) pairs, 32 at a time (2 to 4: any-hit rays
-                        without counters; else 0) */
+                        one leaf per lane set aside, 3 and 4 the same with up to two
+                        leaves per lane (2 to 4: any-hit rays without counters; else 0) */
   int32_t refill;    /* persistent scheme: idle lanes of a warp that trigger a refill
                         (1..32; 0 = 8) */
   int32_t save_distance; /* per-ray scheme, nonzero: the save-distance traversal of
@@ -222,9 +226,9 @@ typedef struct {
                         slot; at most 2^32 - 1 rays per call. Results are identical
                         either way; incoherent rays (ambient occlusion) run faster
                         grouped. */
-  int32_t stack_local; /* per-ray scheme, nonzero: each thread's traversal stack in local
-                        memory (when the tree needs at most 64 entries; else shared
-                        memory, the default placement). Same results. */
+  int32_t stack_local; /* per-ray scheme: asks for the traversal stacks in local memory.
+                        Accepted; the stacks are in shared memory either way (the packed
+                        scene needs one word per tree level). Same results. */
   int32_t any_order; /* 0: any-hit rays push the hit children of a node in the reference's
                         order (instrumented profile: traverseOrderEachAxis of the ray's
                         major axis; fast profile: child-index order). Nonzero: any-hit

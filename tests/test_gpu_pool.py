@@ -108,6 +108,23 @@ def test_unordered_boxes_take_the_general_kernels():
     _same(scene, _rays(tris, LINE + 1, 4))
 
 
+@pytest.mark.parametrize("fmt", ["fp32", "q8"])
+def test_boxes_that_are_not_nested(fmt):
+    """Imported trees whose inner boxes are smaller than what they hold: nothing
+    is dropped behind tMax, and Q8 records stay with the general kernels."""
+    tris, bvh, _ = TS.bvh("clutter120", 8, 4)
+    arrays = bvh.export_compact()
+    inner = np.flatnonzero(arrays["child_count"] > 0)[1::3]
+    lo, hi = arrays["lo3"].copy(), arrays["hi3"].copy()
+    hi[inner] = lo[inner] + 0.8 * (hi[inner] - lo[inner])
+    arrays["lo3"], arrays["hi3"] = lo, hi
+    scene = pkg.Scene(pkg.Bvh.from_compact(arrays, 8, 4), node_format=fmt)
+    rays = _rays(tris, LINE + 1, 6)
+    _same(scene, rays)
+    _same(scene, rays[:40000])
+    _same(scene, rays[:3000])
+
+
 def test_captured_and_concurrent_traces():
     tris = S.clutter(60, 2)
     scene = pkg.Scene(pkg.Bvh(tris, 8, 8))
