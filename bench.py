@@ -818,7 +818,11 @@ def run_batch(a):
     clocks = clk.summary()
     ms_batched = timed(batched, a.steps)
     per_kind_launches = len({(k, s_.bvh_info["branching"]) for s_, _, k, _ in jobs_plain})
-    launches = (1 if one_form else per_kind_launches) + (4 if a.job_reorder else 0)
+    # Per group of one kind, width and ray order (every group of the packed
+    # scenes has more than 2^18 rays): one launch for reordered rays, else the
+    # plan and the two kernels it chooses from; one_launch takes the same path.
+    groups = {(j[2], j[0].bvh_info["branching"], any(j[4:5])) for j in jobs_batched}
+    launches = sum(1 if g_[2] else 3 for g_ in groups) + (4 if a.job_reorder else 0)
     ms_seq = timed(sequential, a.steps)
     for s_ in {id(j[0]): j[0] for j in jobs_plain}.values():
         s_.status()
@@ -847,8 +851,8 @@ def run_batch(a):
             "speedup_vs_sequential": ms_seq / ms_head, "results_identical": bool(same),
             "autotuned_nl": bool(a.tune_nl), "scenes": scenes, "setup_s": round(setup_s, 1),
         },
-        # per step the batched launch(es) of the chosen form plus the four
-        # segmented reorder passes
+        # per step the launches of the groups plus the four segmented reorder
+        # passes
         "clocks": clocks, "gpu_launches": a.steps * launches,
     }
     print(json.dumps(line))

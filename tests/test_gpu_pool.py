@@ -224,3 +224,27 @@ def test_counting_traces(n, l, fmt, rays):
                 a, b = (torch.where(torch.isnan(x), 0.0, x).view(torch.int32) for x in (a, b))
             assert torch.equal(a, b), (kind, opts)
     scene.status()
+
+
+def test_captured_jobs():
+    """Reordered and plain jobs of one captured call, enough rays for the pool."""
+    tris = S.clutter(40, 2)
+    scene = pkg.Scene(pkg.Bvh(tris, 8, 8))
+    rays = _rays(tris, LINE + 77, 8)
+    want = {k: scene.trace(rays, kind=k, scheme="persistent", counters=True) for k in ("closest", "any")}
+    want = {"closest": want["closest"]["hits"], "any": want["any"]["occluded"]}
+    jobs = [(scene, rays, kind, torch.full_like(want[kind], 5), k, k > 0)
+            for kind in ("closest", "any") for k in (0, 4)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        pkg.trace_jobs(jobs)
+    for _ in range(2):
+        for j in jobs:
+            j[3].fill_(5)
+        graph.replay()
+        torch.cuda.synchronize()
+        for _, _, kind, out, _, _ in jobs:
+            assert torch.equal(out.view(torch.uint8), want[kind].view(torch.uint8)), kind
+    scene.status()
