@@ -308,18 +308,19 @@ int bvhgpu_trace_host_batches(bvhgpu_scene_t scene, const bvhgpu_host_batch_t* b
 /* ---- many scenes in one launch ---------------------------------------- */
 /* A job: one ray batch traced in one scene. bvhgpu_trace_jobs traces up to
  * BVHGPU_MAX_JOBS jobs (scenes of any N, L and node format, closest or any
- * hit, uneven sizes) in one persistent launch per group of jobs with the same
- * ray kind, node width and node format (each kernel compiled for its kind)
- * that pulls rays from a global queue spanning the group's jobs, scenes of
- * any size mixed (the GPU form of the reference's
+ * hit, uneven sizes) together, per group of jobs with the same ray kind, node
+ * width and node format (on packed scenes also the same push and ray order),
+ * each kernel compiled for what its jobs share: the rays of the group's jobs
+ * are one batch, scenes of any size mixed (the GPU form of the reference's
  * workgroup refill, fastNodeManager.h:92-156, 277-450, extended across
  * scenes). Results per ray
  * equal bvhgpu_trace's. All scenes must live on the stream's device; the
  * options' profile and policy (0 or 2) apply to every job. Stream-ordered, no
- * synchronisation (so it can be recorded in a CUDA graph); no allocation
- * unless a job is reordered, whose scratch (about 6 bytes per ray) comes from
+ * synchronisation (so it can be recorded in a CUDA graph). Scratch comes from
  * the stream-ordered allocator (cudaMallocAsync / cudaFreeAsync on the
- * stream, which graph capture records as memory nodes). */
+ * stream): about 6 bytes per ray of reordered jobs, which graph capture
+ * records as memory nodes, and in calls without one, outside a capture, 16
+ * bytes per group of more than 2^18 rays. */
 #define BVHGPU_MAX_JOBS 192
 typedef struct {
   bvhgpu_scene_t scene;
@@ -444,9 +445,8 @@ int bvhgpu_unpack_hits(const bvhgpu_hit_t* hits, uint64_t n, int32_t* prim, floa
  * For callers that must not allocate GPU memory while they trace (a plugin
  * whose host application owns the memory budget, a frame loop that cannot
  * take the synchronisation an allocation may cause): traces up to 64 ray
- * batches with the persistent kernel, whose scratch (one ray-queue head per
- * batch) lives in a fixed 512-byte device array inside the library instead of
- * being allocated. More than 64 batches -> BVHGPU_ERR_BAD_ARG. The first call
+ * batches with kernels whose scratch (two queue words per batch) lives in a
+ * fixed 1 KB device array inside the library instead of being allocated. More than 64 batches -> BVHGPU_ERR_BAD_ARG. The first call
  * on a device, and the first after that device's context was destroyed and
  * re-created (cudaDeviceReset), looks up that array's address: make it before
  * any stream capture. The first call with a given kind, profile, policy and
@@ -455,8 +455,7 @@ int bvhgpu_unpack_hits(const bvhgpu_hit_t* hits, uint64_t n, int32_t* prim, floa
  * change of free device memory may be seen. All calls share the array: calls
  * that overlap on the GPU race. opts: profile, policy, refill and any_order
  * are used; scheme is always persistent; reorder, save_distance and
- * stack_local -> BVHGPU_ERR_UNSUPPORTED. The top levels are staged in shared
- * memory as in the regular persistent launches. */
+ * stack_local -> BVHGPU_ERR_UNSUPPORTED. */
 typedef struct {
   const bvhgpu_ray_t* rays; /* device, 16-byte aligned */
   uint64_t n;
