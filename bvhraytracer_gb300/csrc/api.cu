@@ -218,20 +218,25 @@ constexpr uint32_t kTopStageBytes = 8192;
 // Deepest trees of the ray-pool kernel: their stacks leave two blocks per SM.
 constexpr int kPoolMaxLevels = 48;
 
-// The packed scene, made on the device. The caller's streams may not be
-// ordered after the default stream, so this waits for it.
+// Whether the kernels on the packed scene can trace the tree at all.
+static bool packable(const DeviceLayout& L) {
+  return (L.node_format == BVHGPU_NODES_FP32 ? L.boxes_ordered : L.boxes_nested) &&
+         L.n_inner < dev::pool_max_inner(L.node_stride) && L.inner_levels <= kPoolMaxLevels &&
+         L.leaf_block[L.n_leaves] <= dev::kMaxBlocks;
+}
+
+// The packed scene, made on the device, and the general kernels' leaf bounds.
+// Without room for the packed scene the general kernels trace everything. The
+// caller's streams may not be ordered after the default stream, so this waits
+// for it.
 static cudaError_t pack_scene(bvhgpu_scene* s) {
   const DeviceLayout& L = s->layout;
   const size_t node = dev::pack_node_bytes(L.node_stride, L.node_format);
   const size_t blocks = L.leaf_block[L.n_leaves];
   uint32_t* d_block = nullptr;
   uint8_t* d_count = nullptr;
-  cudaError_t e = cudaMalloc((void**)&s->d_pack_nodes, std::max<size_t>(L.n_inner * node, 16));
-  if (e == cudaSuccess)
-    e = cudaMalloc((void**)&s->d_pack_blocks, blocks * dev::kBlockWords * sizeof(float4));
-  if (e == cudaSuccess)
-    e = cudaMalloc((void**)&s->d_leaf_bounds, (size_t)L.n_leaves * sizeof(float) *
-                                                  dev::leaf_bounds_floats(L.leaf_memory));
+  cudaError_t e = cudaMalloc((void**)&s->d_leaf_bounds, (size_t)L.n_leaves * sizeof(float) *
+                                                            dev::leaf_bounds_floats(L.leaf_memory));
   if (e == cudaSuccess) e = cudaMalloc((void**)&d_block, L.leaf_block.size() * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc((void**)&d_count, L.leaf_count.size());
   if (e == cudaSuccess)
@@ -239,8 +244,17 @@ static cudaError_t pack_scene(bvhgpu_scene* s) {
                    cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(d_count, L.leaf_count.data(), L.leaf_count.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && packable(L) &&
+      (cudaMalloc((void**)&s->d_pack_nodes, std::max<size_t>(L.n_inner * node, 16)) != cudaSuccess ||
+       cudaMalloc((void**)&s->d_pack_blocks, blocks * dev::kBlockWords * sizeof(float4)) !=
+           cudaSuccess)) {
+    cudaGetLastError();
+    cudaFree(s->d_pack_nodes);
+    s->d_pack_nodes = nullptr;
+    s->d_pack_blocks = nullptr;
+  }
   const dev::SceneDev sc = s->dev_view();
-  if (e == cudaSuccess)
+  if (e == cudaSuccess && s->d_pack_nodes != nullptr)
     e = dev::pack_nodes(sc, L.node_stride, L.node_format, L.n_inner, d_block, s->d_pack_nodes,
                         nullptr);
   if (e == cudaSuccess)
@@ -261,13 +275,9 @@ static cudaError_t pack_scene(bvhgpu_scene* s) {
 // stacks hold one entry per pushed child, which is what the cap counts), the
 // staging wait of the failure-detection tests, node records whose boxes are
 // not ordered, Q8 ones whose boxes are not nested (imported trees), trees too
-// deep or large for its stack words, and more than 2^32 - 1 rays.
+// deep or large for its stack words (packable), and more than 2^32 - 1 rays.
 static bool scene_uses_pool(const bvhgpu_scene* s) {
-  const DeviceLayout& L = s->layout;
-  return stack_cap(s) >= s->max_stack && s->stall_bytes == 0 &&
-         (L.node_format == BVHGPU_NODES_FP32 ? L.boxes_ordered : L.boxes_nested) &&
-         L.n_inner < dev::pool_max_inner(L.node_stride) && L.inner_levels <= kPoolMaxLevels &&
-         L.leaf_block[L.n_leaves] <= dev::kMaxBlocks;
+  return s->d_pack_nodes != nullptr && stack_cap(s) >= s->max_stack && s->stall_bytes == 0;
 }
 static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
   return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&

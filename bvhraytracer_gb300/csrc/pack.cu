@@ -96,8 +96,9 @@ __global__ void __launch_bounds__(128) pack_leaves_kernel(SceneDev sc, uint32_t 
   if (leaf >= n) return;
   const LeafSource l = leaf_source(sc, leaf, leaf_count);
   float* b = bounds + (size_t)leaf * leaf_bounds_floats(L);
-  float4* out = first < l.cnt ? blocks + (size_t)(leaf_block[leaf] + first / 4) * kBlockWords
-                              : nullptr;
+  float4* out = blocks != nullptr && first < l.cnt
+                    ? blocks + (size_t)(leaf_block[leaf] + first / 4) * kBlockWords
+                    : nullptr;
   for (int k = 0; k < 4; ++k) {
     const int i = first + k;
     float v[9];

@@ -58,7 +58,7 @@ int pack_node_bytes(int nm, int fmt);
 // leaf_block: first block of each leaf.
 cudaError_t pack_nodes(const SceneDev& sc, int nm, int fmt, uint32_t n_inner,
                        const uint32_t* leaf_block, uint8_t* out, cudaStream_t s);
-// Fills the leaf blocks and the general kernels' bounds from the leaves.
+// Fills the leaf blocks (null: none) and the general kernels' bounds from the leaves.
 // leaf_count: triangles of each leaf.
 cudaError_t pack_leaves(const SceneDev& sc, uint32_t n_leaves, const uint32_t* leaf_block,
                         const uint8_t* leaf_count, float4* blocks, float* bounds,
