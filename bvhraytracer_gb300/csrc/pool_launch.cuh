@@ -94,7 +94,11 @@ inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cud
     // (2.1M primary rays on 251k triangles, N8 0.442 -> 0.437 ms, shadow rays
     // 0.337 -> 0.335).
     // Blocks of 256 hold their slots until the last warp ends: 0.449 and 0.347.
-    const int block = p.planned ? 2 * kSoloBlock : kSoloBlock;
+    // Closest-hit rays take them at every size (251k triangles, N8, 131k rays 89
+    // -> 84 us; 32k triangles, N4, 262k rays 65 -> 62; 251k, N16, 262k 146 ->
+    // 145), any-hit rays, which end sooner and less evenly, lose by it (N8 131k
+    // rays 57 -> 60, N4 262k 90 -> 92).
+    const int block = p.planned || KIND == BVHGPU_CLOSEST ? 2 * kSoloBlock : kSoloBlock;
     const size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * block;
     const uint64_t grid = (p.n + block - 1) / block;
     k<<<(unsigned)grid, block, smem, s>>>(p);
