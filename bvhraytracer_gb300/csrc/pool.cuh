@@ -689,6 +689,8 @@ BVHGPU_DEV bool pool_pairs(const SRC& p, const POOL& P, int j, uint32_t pass, in
     const unsigned hits = __ballot_sync(FULL, h);
     const int lo = max(first - base, 0), hi = min(first + mine - base, 32);
     if (lo < hi && ((hits >> lo) & (FULL >> (32 - (hi - lo))))) hit = true;
+    // Other lanes write these pairs, and the owners their rays, next.
+    __syncwarp();
   }
   return hit;
 }
@@ -832,6 +834,8 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
     const unsigned mf = (m == 32 ? FULL : (1u << m) - 1u) & ~(mn | ml);
     const unsigned mine = next == 0 ? mn : (next == 1 ? ml : mf);
     const int at = next == 0 ? n_node : (next == 1 ? K + n_leaf : 2 * K + n_free);
+    // Every lane has read its own entry (votes alone order no memory).
+    __syncwarp();
     if (next >= 0) P.list[at + __popc(mine & below)] = (uint8_t)j;
     n_node += __popc(mn);
     n_leaf += __popc(ml);

@@ -1,0 +1,28 @@
+"""Paths of the kernels on the packed scene that ordinary batches seldom take.
+Results equal the counting kernels' bit for bit (tests/test_gpu_pool.py)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import bvhraytracer_gb300 as pkg  # noqa: E402
+from bvhraytracer_gb300 import scenes as S  # noqa: E402
+from tests.test_gpu_pool import LINE, _rays, _same  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("active", ["one_in_32", "one_in_9", "alternate", "all_but_lane_0",
+                                    "last_warp_only"])
+@pytest.mark.parametrize("n,l,fmt", [(8, 8, "fp32"), (16, 4, "q8")])
+def test_pool_refills_among_inactive_rays(active, n, l, fmt):
+    """A refill step reads free slots and, for rays that are inactive, gives
+    slots back in the same step: every slot stays in exactly one list."""
+    tris = S.clutter(30, 2)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    rays = _rays(tris, LINE + 4097, 11)
+    i = torch.arange(rays.shape[0], device="cuda")
+    off = {"one_in_32": i % 32 != 7, "one_in_9": i % 9 != 0, "alternate": i % 2 == 0,
+           "all_but_lane_0": i % 32 == 0, "last_warp_only": i < rays.shape[0] - 33}[active]
+    rays[off, 0] = float("nan")
+    _same(scene, rays)
+    _same(scene, rays, reorder=3)
