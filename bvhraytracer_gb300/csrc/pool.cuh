@@ -61,6 +61,10 @@ constexpr int kPoolWarps = 4;  // per block
 template <int NM, int FMT>
 constexpr int kSoloBlocks =
     NM == 4 ? 4 : (FMT == kFmtQ8 ? 6 : (NM == 8 ? 8 : 7));
+// The same for launches of no more rays than these blocks hold: registers enough
+// (128 and 168) that nothing spills.
+template <int NM>
+constexpr int kSoloFewBlocks = NM <= 8 ? 4 : 3;
 
 // What a ray's visits need of its scene, and where its result goes.
 struct PackView {
@@ -355,14 +359,24 @@ BVHGPU_DEV uint32_t pool_node_hits(const uint8_t* rec, const PoolRay& r) {
   }
 }
 
-// Hit children as positions in the push sequence of the ray's major axis.
+// What pool_positions reads of a node's record: the child at each position of
+// the push sequence of axis `code`, or for more than 8 children the position of
+// each child.
 template <int NM, int FMT>
-BVHGPU_DEV uint32_t pool_positions(const uint8_t* rec, uint32_t code, uint32_t hit) {
+BVHGPU_DEV typename PoolWord<NM>::T pool_sequence(const uint8_t* rec, uint32_t code) {
   using F = PackFmt<NM, FMT>;
-  if (NM <= 8) {
+  if constexpr (NM <= 8)
+    return ldgu(rec + F::SEQ + 4 * code);
+  else
+    return make_uint2(ldgu(rec + F::INV + 8 * code), ldgu(rec + F::INV + 8 * code + 4));
+}
+
+// Hit children as positions in the push sequence of the ray's major axis.
+template <int NM>
+BVHGPU_DEV uint32_t pool_positions(const typename PoolWord<NM>::T seq, uint32_t hit) {
+  if constexpr (NM <= 8) {
     // Each hit bit spread to a byte, the bytes permuted by the sequence (its
     // nibbles are the selectors of the byte permute), and gathered again.
-    const uint32_t seq = ldgu(rec + F::SEQ + 4 * code);
     const uint32_t lo = ((hit & 15u) * 0x00204081u) & 0x01010101u;
     const uint32_t hi = NM > 4 ? ((hit >> 4) * 0x00204081u) & 0x01010101u : 0u;
     const uint32_t p0 = __byte_perm(lo, hi, seq & 0xFFFFu);
@@ -372,16 +386,16 @@ BVHGPU_DEV uint32_t pool_positions(const uint8_t* rec, uint32_t code, uint32_t h
       pm |= ((p1 * 0x01020408u) >> 24) << 4;
     }
     return pm;
+  } else {
+    const uint64_t inv = (uint64_t)seq.x | ((uint64_t)seq.y << 32);
+    uint32_t pm = 0;
+    while (hit) {
+      const int c = __ffs(hit) - 1;
+      hit &= hit - 1u;
+      pm |= 1u << (uint32_t)((inv >> (4 * c)) & 15u);
+    }
+    return pm;
   }
-  const uint64_t inv = (uint64_t)ldgu(rec + F::INV + 8 * code) |
-                       ((uint64_t)ldgu(rec + F::INV + 8 * code + 4) << 32);
-  uint32_t pm = 0;
-  while (hit) {
-    const int c = __ffs(hit) - 1;
-    hit &= hit - 1u;
-    pm |= 1u << (uint32_t)((inv >> (4 * c)) & 15u);
-  }
-  return pm;
 }
 
 // One lane's view of its warp's pool.
@@ -431,6 +445,18 @@ BVHGPU_DEV bool pool_behind(const uint8_t* rec, const PoolRay& r, int k) {
   return max3f(t[0], t[1], t[2]) > r.tmax;
 }
 
+// The first of a node's children `left`, as a position, and where its record
+// holds their entries by position.
+template <bool ORDERED>
+BVHGPU_DEV int pool_first(const PoolRay& r, uint32_t left) {
+  return ORDERED && ((r.bits >> 2) & 1u) ? 31 - __clz(left) : __ffs(left) - 1;
+}
+template <int NM, int FMT, bool ORDERED>
+BVHGPU_DEV uint32_t pool_entries(const PoolRay& r) {
+  using F = PackFmt<NM, FMT>;
+  return ORDERED ? F::SORTED + (r.bits & 3u) * (4 * NM) : F::ENTRY;
+}
+
 // A ray's next entry: the first of `left` (children of `node` still to visit),
 // the others back on the ray's stack (level l at stack[l * stride]). fresh:
 // node is not on the stack yet; otherwise its word is the stack's top, and
@@ -458,9 +484,7 @@ BVHGPU_DEV bool pool_take(const PackView& v, typename PoolWord<NM>::T* stack, in
       node = W::node(g);
       left = W::left(g);
     }
-    int k;
-    if (ORDERED && ((r.bits >> 2) & 1u)) k = 31 - __clz(left);
-    else k = __ffs(left) - 1;
+    const int k = pool_first<ORDERED>(r, left);
     left &= ~(1u << k);
     const uint8_t* rec = v.nodes + (size_t)node * F::REC;
     if (fresh) {
@@ -470,7 +494,7 @@ BVHGPU_DEV bool pool_take(const PackView& v, typename PoolWord<NM>::T* stack, in
       else --sp;
       if (CULL && cull && pool_behind<NM, FMT>(rec, r, k)) continue;
     }
-    e = ldgu(rec + (ORDERED ? F::SORTED + (r.bits & 3u) * (4 * NM) : F::ENTRY) + 4 * k);
+    e = ldgu(rec + pool_entries<NM, FMT, ORDERED>(r) + 4 * k);
     return true;
   }
 }
@@ -776,7 +800,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
         const uint8_t* rec = v.nodes + (size_t)st.x * F::REC;
         uint32_t left = pool_node_hits<NM, FMT, kLoose>(rec, r);
         const bool fresh = left != 0;
-        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        if (ORDERED && fresh) left = pool_positions<NM>(pool_sequence<NM, FMT>(rec, r.bits & 3u), left);
         next = 2;
         if (pool_take<NM, FMT, ORDERED, kCull>(v, P.stack + j, K, r, st.x, left, fresh, sp, e)) {
           P.state[j] = make_uint2(e, sp);
@@ -894,9 +918,16 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 }
 
 // One thread per ray on the packed scene, its stack in shared memory
-// ([level][thread]).
-template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
-__global__ void __launch_bounds__(128, kSoloBlocks<NM, FMT>)
+// ([level][thread]). FEW: for launches whose rays all run at once, where the
+// longest rays' latency counts and not the rate of visits; a visit then loads
+// the push sequence (and the entries of 4 children) together with the boxes
+// instead of after them. 40k unordered closest-hit rays (L8, 251k triangles), us,
+// of the general per-ray kernel / this one without FEW / with it: N4 119 / 125 /
+// 98, N8 103 / 112 / 96, N12 111 / 131 / 114, N16 103 / 116 / 101. Beyond one
+// wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it, N16,
+// 65k rays, 132 / 168.
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, bool FEW, typename SRC>
+__global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks<NM> : kSoloBlocks<NM, FMT>)
     trace_solo_kernel(const __grid_constant__ SRC p) {
   using F = PackFmt<NM, FMT>;
   using W = PoolWord<NM>;
@@ -904,6 +935,7 @@ __global__ void __launch_bounds__(128, kSoloBlocks<NM, FMT>)
                           KIND == BVHGPU_ANY;
   constexpr bool kCull =
       PROFILE == BVHGPU_PROFILE_INSTRUMENTED && KIND == BVHGPU_CLOSEST && NM >= 8;
+  constexpr bool kRow = FEW && NM == 4;
   extern __shared__ __align__(16) uint8_t pool_smem[];
   if (p.planned && p.queue[1] != kPlanSolo) return;
   typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
@@ -924,9 +956,21 @@ __global__ void __launch_bounds__(128, kSoloBlocks<NM, FMT>)
     while (more) {
       while (more && !(e & kLeafBit)) {
         const uint8_t* rec = v.nodes + (size_t)e * F::REC;
+        typename W::T seq{};
+        uint4 row{};
+        if (FEW && ORDERED) seq = pool_sequence<NM, FMT>(rec, r.bits & 3u);
+        if (kRow) row = ldgu4(rec + pool_entries<NM, FMT, ORDERED>(r));
         uint32_t left = pool_node_hits<NM, FMT, kLoose>(rec, r);
         const bool fresh = left != 0;
-        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        if (ORDERED && fresh)
+          left = pool_positions<NM>(FEW ? seq : pool_sequence<NM, FMT>(rec, r.bits & 3u), left);
+        if (kRow && fresh) {
+          const int k = pool_first<ORDERED>(r, left);
+          left &= ~(1u << k);
+          if (left) stack[sp++ * stride] = W::make(e, left);
+          e = (k & 2) ? ((k & 1) ? row.w : row.z) : ((k & 1) ? row.y : row.x);
+          continue;
+        }
         more = pool_take<NM, FMT, ORDERED, kCull>(v, stack, stride, r, e, left, fresh, sp, e);
       }
       if (!more) break;
@@ -990,7 +1034,7 @@ __global__ void __launch_bounds__(128, 6)
           ctr.max_stack = max(ctr.max_stack, held);
           count_node(a, (int)((info >> 8) | (info & 0xFFu) << 8), hist);
           const bool fresh = left != 0;
-          if (fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+          if (fresh) left = pool_positions<NM>(pool_sequence<NM, FMT>(rec, r.bits & 3u), left);
           more = pool_take<NM, FMT, true, false>(v, stack, stride, r, e, left, fresh, sp, e);
           --held;
         }
@@ -1196,7 +1240,7 @@ __global__ void __launch_bounds__(128) trace_team_kernel(const __grid_constant__
         const bool h = team_child_hit<NM, FMT>(rec, r, c);
         left = (__ballot_sync(mask, h) & mask) >> base;
         fresh = left != 0;
-        if (ORDERED && fresh) left = pool_positions<NM, FMT>(rec, r.bits & 3u, left);
+        if (ORDERED && fresh) left = pool_positions<NM>(pool_sequence<NM, FMT>(rec, r.bits & 3u), left);
       } else if (team_leaf<T, PROFILE, KIND>(v, e, r, k, c, mask, base, r.tmax)) {
         hit = true;
         if (KIND == BVHGPU_ANY) break;

@@ -87,7 +87,9 @@ inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cud
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!pool) {
-    auto k = trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
+    auto k = p.n <= (uint64_t)sm_count * kSoloFewBlocks<NM> * 128
+                 ? trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, true, SRC>
+                 : trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, false, SRC>;
     // A planned launch takes blocks of twice the size: if the pool is chosen,
     // its blocks only start and return (half as many: a 1001 x 563 frame with 8
     // random rays per hit 1.54 -> 1.52 ms), and if not, fewer starts are as good

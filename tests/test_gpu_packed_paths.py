@@ -26,3 +26,16 @@ def test_pool_refills_among_inactive_rays(active, n, l, fmt):
     rays[off, 0] = float("nan")
     _same(scene, rays)
     _same(scene, rays, reorder=3)
+
+
+@pytest.mark.parametrize("n,l,fmt", [(2, 1, "fp32"), (4, 4, "q8"), (8, 8, "fp32"), (8, 4, "q8"),
+                                     (12, 9, "fp32"), (16, 16, "q8"), (16, 2, "fp32")])
+def test_solo_kernel_of_one_wave(n, l, fmt):
+    """A launch whose rays all run at once takes the one-thread-per-ray kernel
+    with more registers: its last size, the next one, and a remainder."""
+    tris = S.clutter(30, 5)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * 128 * (4 if n <= 8 else 3)
+    rays = _rays(tris, wave + 1, n + l, extreme=True)
+    for k in (wave - 127, wave, wave + 1):
+        _same(scene, rays[:k])
