@@ -346,8 +346,11 @@ struct PoolQueue {
 };
 
 static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
-  return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root,
-                       (int16_t)s->layout.gang, (int16_t)(s->layout.boxes_nested ? 1 : 0)};
+  const DeviceLayout& L = s->layout;
+  const int leaves = (L.most_leaf <= 2 ? dev::kSmallLeaves : 0) |
+                     (L.most_leaf <= L.node_stride ? dev::kLeavesInTurn : 0);
+  return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root, (int16_t)L.gang,
+                       (int8_t)(L.boxes_nested ? 1 : 0), (int8_t)leaves};
 }
 
 // A trace on the packed scene.

@@ -333,6 +333,7 @@ int build_device_layout(const Bvh& bvh, int gang, int leaf_memory, int node_form
     }
     out.leaf_depth[k] = c.depth;
     out.leaf_count[k] = (uint8_t)c.prim_count;
+    out.most_leaf = std::max(out.most_leaf, (int)c.prim_count);
     out.leaf_block[k + 1] = (c.prim_count + 3) / 4;
   }
   for (uint32_t k = 0; k < nl; ++k) out.leaf_block[k + 1] += out.leaf_block[k];

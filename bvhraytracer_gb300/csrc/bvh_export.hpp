@@ -75,6 +75,7 @@ struct DeviceLayout {
   // (n_leaves + 1 values).
   std::vector<uint8_t> leaf_count;
   std::vector<uint32_t> leaf_block;
+  int most_leaf = 0;                  // triangles of the largest leaf
   int inner_levels = 0;               // inner nodes on the longest path from the root
   // Every box lies in its parent's and every triangle in its leaf's box.
   bool boxes_nested = true;

@@ -53,18 +53,22 @@ constexpr int kPoolWarps = 4;  // per block
 #define BVHGPU_POOL_REFILL 32
 #endif
 
-// Blocks of 128 threads per SM that the solo kernel's registers allow (2.1M
-// primary / shadow rays, ms, 4 / 6 / 7 / 8 blocks): N4 0.46 0.46 0.46 0.47 /
-// 0.31 0.32 0.31 0.33 (terrain 0.27 0.28 0.28 0.28); N8 0.47 0.46 0.45 0.44 / 0.32 0.31 0.30 0.29; N8 Q8 1.38
-// 1.36 1.33 1.39 / 0.45 0.43 0.45 0.47; N16 0.65 0.56 0.55 0.55 / 0.46 0.40
-// 0.40 0.40.
+// Blocks of 128 threads per SM that the solo kernel's registers allow. Closest-hit
+// rays, us: N8L8, primary rays of 12 scenes, 0.46M, 5 / 6 / 7 / 8 blocks 201 197
+// 197 210, of one (251k triangles), 0.5M, 6 / 7 / 8 228 223 226; N16L8, 0.26M
+// unordered, 6 / 7 285 255; N4L4, 131k unordered, 5 / 6 / 7 182 136 137. Q8 nodes,
+// N8, 2.1M rays, ms, 4 / 6 / 7 / 8: primary 1.38 1.36 1.33 1.39, shadow 0.45 0.43
+// 0.45 0.47.
 template <int NM, int FMT>
-constexpr int kSoloBlocks =
-    NM == 4 ? 4 : (FMT == kFmtQ8 ? 6 : (NM == 8 ? 8 : 7));
+constexpr int kSoloBlocks = NM > 4 && FMT == kFmtQ8 ? 6 : 7;
 // The same for launches of no more rays than these blocks hold: registers enough
 // (128 and 168) that nothing spills.
 template <int NM>
 constexpr int kSoloFewBlocks = NM <= 8 ? 4 : 3;
+
+// PackView::leaves: no leaf has more than two triangles; none has more than a
+// node has child slots (see trace_solo_kernel).
+constexpr int kSmallLeaves = 1, kLeavesInTurn = 2;
 
 // What a ray's visits need of its scene, and where its result goes.
 struct PackView {
@@ -73,7 +77,8 @@ struct PackView {
   void* out;             // hits or occlusion bytes
   uint32_t root;         // stack entry of the root
   int16_t gang;
-  int16_t nested;        // every box lies in its parent's, every triangle in its leaf's
+  int8_t nested;         // every box lies in its parent's, every triangle in its leaf's
+  int8_t leaves;         // kSmallLeaves, kLeavesInTurn
 };
 
 // Common arguments of a launch.
@@ -465,7 +470,8 @@ BVHGPU_DEV uint32_t pool_entries(const PoolRay& r) {
 // CULL (closest-hit rays of the instrumented profile that have a hit, nested
 // boxes): children behind tMax are dropped. A visit would find nothing there:
 // every box and triangle inside starts at the same t0 or later (rounding is
-// monotonic) and tMax does not change during the visit. 1M-triangle N8L8 tree,
+// monotonic) and tMax does not change during the visit. Not for leaves of one or
+// two triangles, which cost as much as the check. 1M-triangle N8L8 tree,
 // primary rays: 18.8 -> 13.9 node visits per ray, solo kernel 0.53 -> 0.47 ms
 // (2.1M rays); N16 0.76 -> 0.65 ms; N4, whose visits cost little more than the
 // check, 0.46 -> 0.47. Pool kernel, bounced rays: N16 1.13 -> 1.06 ms, N8 1.15
@@ -476,7 +482,8 @@ BVHGPU_DEV bool pool_take(const PackView& v, typename PoolWord<NM>::T* stack, in
                           uint32_t& sp, uint32_t& e) {
   using F = PackFmt<NM, FMT>;
   using W = PoolWord<NM>;
-  const bool cull = CULL && ((r.bits >> 12) & 1u) && !((r.bits >> 3) & 1u) && v.nested;
+  const bool cull = CULL && ((r.bits >> 12) & 1u) && !((r.bits >> 3) & 1u) && v.nested &&
+                    !(v.leaves & kSmallLeaves);
   while (true) {
     if (!fresh) {
       if (sp == 0) return false;
@@ -528,8 +535,13 @@ BVHGPU_DEV bool mt_rejects(float n1, float div) {
 // The triangles of a leaf that a cheap test does not rule out, four at a time:
 // the stored bounds (instrumented profile; all of them for rays that take the
 // exact forms), or the first barycentric without its division.
+//
+// In the fast profile leaves of one or two triangles go straight to the full
+// test, as the cheap one is half of it (0.26M unordered any-hit rays, N4L1, 149
+// -> 143 us).
 template <int PROFILE>
-BVHGPU_DEV uint32_t leaf_candidates(const float4* blk, int cnt, const PoolRay& r, const float4& c) {
+BVHGPU_DEV uint32_t leaf_candidates(const PackView& v, const float4* blk, int cnt, const PoolRay& r,
+                                    const float4& c) {
   const uint32_t all = (1u << cnt) - 1u;
   uint32_t miss = 0;
   if (PROFILE == BVHGPU_PROFILE_INSTRUMENTED) {
@@ -544,6 +556,7 @@ BVHGPU_DEV uint32_t leaf_candidates(const float4* blk, int cnt, const PoolRay& r
     }
     return ~miss & all;
   }
+  if (v.leaves & kSmallLeaves) return all;
   for (int g = (cnt - 1) >> 2; g >= 0; --g) {
     const float4* tri = blk + g * kBlockWords + kBlockTris;
 #pragma unroll
@@ -612,7 +625,7 @@ BVHGPU_DEV bool pool_leaf(const PackView& v, uint32_t e, const PoolRay pr, const
   const float4* blk = leaf_blocks(v, e);
   const uint32_t slot = __float_as_uint(c.w);
   const bool exact = PROFILE == BVHGPU_PROFILE_INSTRUMENTED && ((pr.bits >> 3) & 1u);
-  uint32_t pass = leaf_candidates<PROFILE>(blk, leaf_count(e), pr, c);
+  uint32_t pass = leaf_candidates<PROFILE>(v, blk, leaf_count(e), pr, c);
   const Ray r = leaf_ray<PROFILE>(pr, c);
   bool any = false;
   // Fast profile: the tie rule of triIntersect{L} as in visit_leaf_points.
@@ -820,8 +833,8 @@ __global__ void __launch_bounds__(kPoolWarps * 32, BVHGPU_POOL_MIN_BLOCKS)
         if (on) {
           const PoolRay r = P.ray(j);
           const uint32_t e = P.state[j].x;
-          pass = leaf_candidates<PROFILE>(leaf_blocks(p.view((r.bits >> 4) & 0xFFu), e),
-                                          leaf_count(e), r, P.c[j]);
+          const PackView& v = p.view((r.bits >> 4) & 0xFFu);
+          pass = leaf_candidates<PROFILE>(v, leaf_blocks(v, e), leaf_count(e), r, P.c[j]);
         }
         hit = pool_pairs<PROFILE>(p, P, j, pass, (int)lane);
       }
@@ -926,6 +939,15 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // 98, N8 103 / 112 / 96, N12 111 / 131 / 114, N16 103 / 116 / 101. Beyond one
 // wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it, N16,
 // 65k rays, 132 / 168.
+//
+// kLeavesInTurn: a lane that reaches a leaf visits it after the warp's current
+// node step, instead of when every lane has a leaf. A leaf of few triangles
+// costs less than a node, so waiting for company only idles lanes (N8L1: 16.4
+// of 32 lanes against 19.8 of the general per-ray kernel). 0.5M primary rays
+// (251k triangles), us, general / waiting / in turn: N4L1 335 / 349 / 235, N8L1 316
+// / 363 / 239, N8L8 301 / 253 / 223. With leaves larger than nodes waiting is
+// better: N4L8, 0.26M unordered any-hit rays of the fast profile, 172 waiting / 190
+// in turn.
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, bool FEW, typename SRC>
 __global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks<NM> : kSoloBlocks<NM, FMT>)
     trace_solo_kernel(const __grid_constant__ SRC p) {
@@ -969,11 +991,13 @@ __global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks<NM> : kSoloBlocks<NM
           left &= ~(1u << k);
           if (left) stack[sp++ * stride] = W::make(e, left);
           e = (k & 2) ? ((k & 1) ? row.w : row.z) : ((k & 1) ? row.y : row.x);
-          continue;
+        } else {
+          more = pool_take<NM, FMT, ORDERED, kCull>(v, stack, stride, r, e, left, fresh, sp, e);
         }
-        more = pool_take<NM, FMT, ORDERED, kCull>(v, stack, stride, r, e, left, fresh, sp, e);
+        if (v.leaves & kLeavesInTurn) break;
       }
       if (!more) break;
+      if (!(e & kLeafBit)) continue;
       float tmax = r.tmax;
       if (pool_leaf<PROFILE, KIND>(v, e, r, c, tmax)) {
         hit = true;

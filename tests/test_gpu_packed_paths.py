@@ -39,3 +39,18 @@ def test_solo_kernel_of_one_wave(n, l, fmt):
     rays = _rays(tris, wave + 1, n + l, extreme=True)
     for k in (wave - 127, wave, wave + 1):
         _same(scene, rays[:k])
+
+
+@pytest.mark.parametrize("n,l", [(2, 1), (3, 2), (4, 2), (4, 3), (4, 4), (4, 5), (8, 1), (8, 8),
+                                 (8, 9), (12, 12), (12, 13), (16, 2), (16, 16)])
+@pytest.mark.parametrize("fmt", ["fp32", "q8"])
+def test_small_leaves_and_leaves_in_turn(n, l, fmt):
+    """The one-thread-per-ray kernel at the leaf sizes where its loop and its
+    cheap tests change, in launches of one wave, of more, and planned ones."""
+    tris = S.clutter(25, 6)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    rays = _rays(tris, LINE + 1, 3 * n + l, extreme=True)
+    for k in (40000, 140001, LINE + 1):
+        _same(scene, rays[:k])
+    cam, target, _ = S.clutter_viewpoints(25, 6)
+    _same(scene, pkg.camera_rays(cam, target, 768, 512))  # stay together: not the pool
