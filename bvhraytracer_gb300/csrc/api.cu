@@ -330,8 +330,10 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
 struct PoolQueue {
   unsigned long long* words = nullptr;
   void* scratch = nullptr;
-  PoolQueue(int device, uint64_t n, unsigned long long* given, cudaStream_t st) : words(given) {
-    if (given || !dev::pool_wants_queue(n)) return;
+  PoolQueue(int device, const dev::PackedCfg& c, uint64_t n, unsigned long long* given,
+            cudaStream_t st)
+      : words(given) {
+    if (given || !dev::pool_wants_queue(c, n)) return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
     if (cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone &&
@@ -345,6 +347,12 @@ struct PoolQueue {
   }
 };
 
+// Bytes of a scene's packed node records.
+static uint64_t pack_bytes(const bvhgpu_scene* s) {
+  return (uint64_t)s->layout.n_inner *
+         dev::pack_node_bytes(s->layout.node_stride, s->layout.node_format);
+}
+
 static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
   const DeviceLayout& L = s->layout;
   const int leaves = (L.most_leaf <= 2 ? dev::kSmallLeaves : 0) |
@@ -356,17 +364,14 @@ static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
 // A trace on the packed scene.
 static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
                                cudaStream_t st) {
-  // Counting traces need no queue.
-  PoolQueue queue(s->device, c.count ? 0 : a.n, c.pool_queue, st);
   dev::OneScene p{};
   p.n = a.n;
   p.levels = std::max(1, s->layout.inner_levels);
-  p.queue = queue.words;
   p.scene = pack_view(s, c.kind == BVHGPU_ANY ? (void*)a.occluded : (void*)a.hits);
   p.rays = a.rays;
   p.out_index = a.out_index;
   const dev::PackedCfg cfg{s->layout.node_stride, s->layout.node_format, c.kind, c.profile,
-                           c.any_order, a.out_index != nullptr, s->sm_count};
+                           c.any_order, a.out_index != nullptr, s->sm_count, pack_bytes(s)};
   cudaError_t e;
   if (c.count) {
     switch (cfg.nm) {
@@ -376,6 +381,8 @@ static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const d
       default: return dev::launch_counting<16>(p, a, cfg, st);
     }
   }
+  PoolQueue queue(s->device, cfg, a.n, c.pool_queue, st);
+  p.queue = queue.words;
   switch (cfg.nm) {
     case 4: e = dev::launch_one_scene<4>(p, cfg, st); break;
     case 8: e = dev::launch_one_scene<8>(p, cfg, st); break;
@@ -1152,7 +1159,7 @@ static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, cons
     if (jobs[i].n == 0) continue;
     const dev::JobDev& d = t.jobs[k++];
     const dev::PackedCfg c{d.nm, d.fmt, d.kind, profile, d.kind == BVHGPU_ANY && d.any_index_order,
-                           d.perm != nullptr, sms};
+                           d.perm != nullptr, sms, 0};
     size_t g = 0;
     while (g < cfg.size() && !(cfg[g].nm == c.nm && cfg[g].fmt == c.fmt && cfg[g].kind == c.kind &&
                                cfg[g].any_order == c.any_order &&
@@ -1165,6 +1172,7 @@ static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, cons
     p->n = 0;
     p->n_jobs = 0;
     p->levels = 1;
+    const bvhgpu_scene* last = nullptr;  // a scene's jobs mostly follow one another
     for (int i = 0, k = 0; i < n_jobs; ++i) {
       if (jobs[i].n == 0) continue;
       const dev::JobDev& d = t.jobs[k];
@@ -1176,8 +1184,10 @@ static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, cons
       j.begin = p->n;
       p->n += d.n;
       p->levels = std::max(p->levels, jobs[i].scene->layout.inner_levels);
+      if (jobs[i].scene != last) cfg[g].node_bytes += pack_bytes(jobs[i].scene);
+      last = jobs[i].scene;
     }
-    PoolQueue queue(device, p->n, words ? words + 2 * g : nullptr, st);
+    PoolQueue queue(device, cfg[g], p->n, words ? words + 2 * g : nullptr, st);
     p->queue = queue.words;
     cudaError_t e;
     switch (cfg[g].nm) {

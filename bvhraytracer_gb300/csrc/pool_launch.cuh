@@ -14,6 +14,7 @@ struct PackedCfg {
   bool any_order;        // any-hit rays push in child-index order
   bool direction_order;  // the rays are sorted by direction
   int sm_count;
+  uint64_t node_bytes;   // packed node records of the scenes together
 };
 
 // Width NM of one scene or many (pool_n*.cu, pool_jobs_n*.cu).
@@ -39,7 +40,19 @@ template <int NM> cudaError_t launch_counting(OneScene& p, TraceArgs a, const Pa
 #ifndef BVHGPU_POOL_MIN_RAYS
 #define BVHGPU_POOL_MIN_RAYS (1u << 18)
 #endif
-inline bool pool_wants_queue(uint64_t n) { return n > BVHGPU_POOL_MIN_RAYS; }
+// FP32 nodes of more than 8 children in trees of more than so many bytes of
+// records: unordered rays have a thread each at every batch size. A pool's 56
+// rays are at as many nodes, 288 or 384 bytes of boxes each, and eight pools per SM
+// leave the L1 too little room for them. Closest-hit rays on 251k triangles, 2M
+// unordered, pool / solo, us: N12L8 (6.6 MB) 2694 / 1670, N16L4 (12 MB) 2013 / 1631,
+// N16L1 (43 MB) 3483 / 1811, but N16L8 (4.9 MB) 1578 / 1641, N16L16 (3.5 MB) 1744 /
+// 1849; N8L4 (7.5 MB) 1119 / 1421, N8L8 of 1M triangles (17 MB), 3.5M rays, 2496 / 2870;
+// N12L8 with Q8 records 2760 / 4057.
+constexpr uint64_t kPoolWideBytes = 5u << 20;
+inline bool pool_wants_queue(const PackedCfg& c, uint64_t n) {
+  return n > BVHGPU_POOL_MIN_RAYS && (c.direction_order || c.nm <= 8 || c.fmt != kFmtFP32 ||
+                                      c.node_bytes <= kPoolWideBytes);
+}
 constexpr int kSoloBlock = 64;
 // Batches of up to so many rays run with a team of lanes per ray (closest-hit /
 // any-hit). Solo / team, us, of a call from Python, which itself takes 15-17
@@ -63,7 +76,8 @@ constexpr int kTeamBlock = 64;
 // The traces of one launch: a team per ray, one thread per ray, pools, or both
 // of these with the rays' own choice between them.
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
-inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cudaStream_t s) {
+inline cudaError_t launch_packed(SRC& p, const PackedCfg& c, cudaStream_t s) {
+  const int sm_count = c.sm_count;
   cudaError_t e;
   if (p.n <= (KIND == BVHGPU_ANY ? BVHGPU_TEAM_MAX_ANY : BVHGPU_TEAM_MAX_CLOSEST)) {
     auto k = trace_team_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
@@ -77,10 +91,10 @@ inline cudaError_t launch_packed(SRC& p, bool direction_order, int sm_count, cud
     k<<<(unsigned)((need * 32 + kTeamBlock - 1) / kTeamBlock), kTeamBlock, smem, s>>>(p);
     return cudaGetLastError();
   }
-  const bool large = pool_wants_queue(p.n) && p.queue != nullptr;
+  const bool large = pool_wants_queue(c, p.n) && p.queue != nullptr;
   // Rays in direction order are for the pool; otherwise the rays themselves
   // decide.
-  const bool pool = large && direction_order;
+  const bool pool = large && c.direction_order;
   p.planned = large && !pool;
   if (p.planned) {
     plan_kernel<SRC><<<1, kPlanWarps * 32, 0, s>>>(p);
@@ -131,15 +145,13 @@ template <int NM, int FMT, typename SRC>
 inline cudaError_t launch_packed_fmt(SRC& p, const PackedCfg& c, cudaStream_t s) {
   constexpr int F = BVHGPU_PROFILE_FAST, I = BVHGPU_PROFILE_INSTRUMENTED;
   constexpr int C = BVHGPU_CLOSEST, A = BVHGPU_ANY;
-  const bool d = c.direction_order;
-  const int sms = c.sm_count;
   if (c.kind == C)
-    return c.profile == F ? launch_packed<NM, F, C, FMT, true>(p, d, sms, s)
-                          : launch_packed<NM, I, C, FMT, true>(p, d, sms, s);
+    return c.profile == F ? launch_packed<NM, F, C, FMT, true>(p, c, s)
+                          : launch_packed<NM, I, C, FMT, true>(p, c, s);
   // Any-hit rays of the fast profile push in child-index order always.
-  if (c.profile == F) return launch_packed<NM, F, A, FMT, false>(p, d, sms, s);
-  return c.any_order ? launch_packed<NM, I, A, FMT, false>(p, d, sms, s)
-                     : launch_packed<NM, I, A, FMT, true>(p, d, sms, s);
+  if (c.profile == F) return launch_packed<NM, F, A, FMT, false>(p, c, s);
+  return c.any_order ? launch_packed<NM, I, A, FMT, false>(p, c, s)
+                     : launch_packed<NM, I, A, FMT, true>(p, c, s);
 }
 
 template <int NM, int KIND, int FMT>

@@ -54,3 +54,26 @@ def test_small_leaves_and_leaves_in_turn(n, l, fmt):
         _same(scene, rays[:k])
     cam, target, _ = S.clutter_viewpoints(25, 6)
     _same(scene, pkg.camera_rays(cam, target, 768, 512))  # stay together: not the pool
+
+
+@pytest.mark.parametrize("n,l,fmt,objects", [(12, 4, "fp32", 800), (16, 1, "fp32", 300),
+                                             (12, 4, "fp32", 300), (16, 1, "q8", 300)])
+def test_wide_trees_on_both_sides_of_the_pool_line(n, l, fmt, objects):
+    """Trees of wide nodes with more records than the pool kernel is good for,
+    with fewer, and on Q8 records, for large unordered and ordered batches and
+    as jobs."""
+    tris = S.clutter(objects, 4)
+    bvh = pkg.Bvh(tris, n, l)
+    wide_bytes = bvh.info["n_inner"] * (560 if n == 12 else 720)
+    assert (wide_bytes > 5 << 20) == (objects == 800 or n == 16)
+    scene = pkg.Scene(bvh, node_format=fmt)
+    rays = _rays(tris, LINE + 1, n + l)
+    _same(scene, rays)
+    _same(scene, rays, reorder=3)
+    for kind in ("closest", "any"):
+        key = "hits" if kind == "closest" else "occluded"
+        want = scene.trace(rays, kind=kind, scheme="persistent", counters=True)[key]
+        jobs = [(scene, rays, kind, torch.full_like(want, 5)) for _ in range(2)]
+        pkg.trace_jobs(jobs)
+        torch.cuda.synchronize()
+        assert all(torch.equal(j[3].view(torch.uint8), want.view(torch.uint8)) for j in jobs)
