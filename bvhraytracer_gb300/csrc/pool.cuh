@@ -61,10 +61,10 @@ constexpr int kPoolWarps = 4;  // per block
 // 0.45 0.47.
 template <int NM, int FMT>
 constexpr int kSoloBlocks = NM > 4 && FMT == kFmtQ8 ? 6 : 7;
-// The same for launches of no more rays than these blocks hold: registers enough
-// (128 and 168) that nothing spills.
-template <int NM>
-constexpr int kSoloFewBlocks = NM <= 8 ? 4 : 3;
+// The same for launches of no more rays than these blocks hold (FEW): up to 128
+// registers. N16L8, 40k / 65k unordered closest-hit rays, us, 3 / 4 / 5 blocks: 92
+// 96 98 / 112 105 108 (3 blocks hold 58k rays).
+constexpr int kSoloFewBlocks = 4;
 
 // PackView::leaves: no leaf has more than two triangles; none has more than a
 // node has child slots (see trace_solo_kernel).
@@ -936,9 +936,8 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // the push sequence (and the entries of 4 children) together with the boxes
 // instead of after them. 40k unordered closest-hit rays (L8, 251k triangles), us,
 // of the general per-ray kernel / this one without FEW / with it: N4 119 / 125 /
-// 98, N8 103 / 112 / 96, N12 111 / 131 / 114, N16 103 / 116 / 101. Beyond one
-// wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it, N16,
-// 65k rays, 132 / 168.
+// 98, N8 103 / 112 / 96, N12 111 / 131 / 108, N16 103 / 116 / 96. Beyond one
+// wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it.
 //
 // kLeavesInTurn: a lane that reaches a leaf visits it after the warp's current
 // node step, instead of when every lane has a leaf. A leaf of few triangles
@@ -949,7 +948,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // better: N4L8, 0.26M unordered any-hit rays of the fast profile, 172 waiting / 190
 // in turn.
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, bool FEW, typename SRC>
-__global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks<NM> : kSoloBlocks<NM, FMT>)
+__global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks : kSoloBlocks<NM, FMT>)
     trace_solo_kernel(const __grid_constant__ SRC p) {
   using F = PackFmt<NM, FMT>;
   using W = PoolWord<NM>;

@@ -101,7 +101,7 @@ inline cudaError_t launch_packed(SRC& p, const PackedCfg& c, cudaStream_t s) {
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!pool) {
-    auto k = p.n <= (uint64_t)sm_count * kSoloFewBlocks<NM> * 128
+    auto k = p.n <= (uint64_t)sm_count * kSoloFewBlocks * 128
                  ? trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, true, SRC>
                  : trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, false, SRC>;
     // A planned launch takes blocks of twice the size: if the pool is chosen,

@@ -35,7 +35,7 @@ def test_solo_kernel_of_one_wave(n, l, fmt):
     with more registers: its last size, the next one, and a remainder."""
     tris = S.clutter(30, 5)
     scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
-    wave = torch.cuda.get_device_properties(0).multi_processor_count * 128 * (4 if n <= 8 else 3)
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * 128 * 4
     rays = _rays(tris, wave + 1, n + l, extreme=True)
     for k in (wave - 127, wave, wave + 1):
         _same(scene, rays[:k])
