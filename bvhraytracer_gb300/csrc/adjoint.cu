@@ -17,6 +17,7 @@
 // then added with atomics per triangle (9 floats, scattered to shared
 // vertices by the caller) or per vertex through the face indices.
 #include "adjoint.cuh"
+#include "smem_limit.cuh"
 
 namespace bvhgpu {
 namespace dev {
@@ -326,9 +327,7 @@ cudaError_t launch_adjoint(const SceneDev& sc, int nm, const AdjointArgs& a, cud
   const size_t smem = (size_t)a.stack_cap * bs * 4;
   const uint64_t grid = (a.n + bs - 1) / bs;
   auto pick = [&](auto k) -> cudaError_t {
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024)
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     k<<<(unsigned)grid, bs, smem, s>>>(sc, a);
     return cudaGetLastError();

@@ -25,6 +25,7 @@
 #define BVHGPU_LEAF_BOUNDS BVHGPU_BATCHED_BOUNDS
 
 #include "batched.cuh"
+#include "smem_limit.cuh"
 
 namespace bvhgpu {
 namespace dev {
@@ -45,9 +46,7 @@ cudaError_t launch_batched(const JobTable& t, int profile, int kmode, int sm_cou
                       : kmode == 2 ? trace_batched_kernel<I, 2>
                       : kmode == 3 ? trace_batched_kernel<I, 3>
                                    : trace_batched_kernel<I, 0>);
-  cudaError_t e = cudaSuccess;
-  if (smem > 48 * 1024)
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "smem_limit.cuh"
 #include "traverse.cuh"
 
 namespace bvhgpu {
@@ -32,12 +33,6 @@ struct LaunchCfg {
   bool any_order = false;       // any-hit rays without counters: child-index push order
 };
 
-template <typename K>
-inline cudaError_t set_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 // Room for the block's visit histogram after `smem` bytes, if it is wanted and
 // fits (else the kernel counts in global memory).
 inline size_t add_block_hist(TraceArgs& a, bool count, size_t smem) {
@@ -59,7 +54,7 @@ inline cudaError_t launch_one(const SceneDev& sc, TraceArgs a, const LaunchCfg& 
     const size_t smem = add_block_hist(a, COUNT, (size_t)a.stack_cap * bs * 4 * (dist ? 2 : 1));
     auto k = dist ? trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, kDist>
                   : trace_dfs_kernel<NM, PROFILE, KIND, COUNT, FMT, false>;
-    cudaError_t e = set_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     const uint64_t grid = (a.n + bs - 1) / bs;
     k<<<(unsigned)grid, bs, smem, s>>>(sc, a);
@@ -77,7 +72,7 @@ inline cudaError_t launch_one(const SceneDev& sc, TraceArgs a, const LaunchCfg& 
              : (cfg.policy >= 3 && kSpec)
                  ? trace_persistent_kernel<NM, PROFILE, KIND, COUNT, (kSpec ? 3 : 0), FMT>
                  : trace_persistent_kernel<NM, PROFILE, KIND, COUNT, 0, FMT>;
-    cudaError_t e = set_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);
@@ -98,7 +93,7 @@ inline cudaError_t launch_one(const SceneDev& sc, TraceArgs a, const LaunchCfg& 
     const size_t smem = add_block_hist(
         a, COUNT, stream_smem_bytes(p, a.stack_cap, COUNT, COUNT && a.step_stats));
     auto k = trace_stream_kernel<NM, PROFILE, KIND, COUNT>;
-    cudaError_t e = set_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     const uint64_t grid = (a.n + p - 1) / p;
     k<<<(unsigned)grid, p, smem, s>>>(sc, a);

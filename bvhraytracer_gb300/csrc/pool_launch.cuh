@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "pool.cuh"
+#include "smem_limit.cuh"
 
 namespace bvhgpu {
 namespace dev {
@@ -122,10 +123,7 @@ inline cudaError_t launch_packed(SRC& p, const PackedCfg& c, cudaStream_t s) {
   }
   auto k = trace_pool_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
   const size_t smem = kPoolWarps * pool_warp_bytes<NM>(p.levels);
-  if (smem > 48 * 1024 &&
-      (e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-          cudaSuccess)
-    return e;
+  if ((e = allow_smem(k, smem)) != cudaSuccess) return e;
   // Resident warps; blocks past them would find the queue empty.
   const size_t fit = BVHGPU_POOL_SMEM / smem;
   const uint64_t per_sm = fit < 1 ? 1 : fit > BVHGPU_POOL_MIN_BLOCKS ? BVHGPU_POOL_MIN_BLOCKS : fit;
@@ -161,11 +159,8 @@ inline cudaError_t launch_count(OneScene& p, TraceArgs& a, cudaStream_t s) {
   a.block_hist = a.depth_hist != nullptr;
   if (a.block_hist) smem += kHistBins * sizeof(uint32_t);
   auto k = trace_count_kernel<NM, KIND, FMT>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem(k, smem);
+  if (e != cudaSuccess) return e;
   k<<<(unsigned)((p.n + kBlock - 1) / kBlock), kBlock, smem, s>>>(p, a);
   return cudaGetLastError();
 }

@@ -20,6 +20,7 @@
 #include "reorder.cuh"
 
 #include "device_common.cuh"
+#include "smem_limit.cuh"
 
 namespace bvhgpu {
 namespace dev {
@@ -329,13 +330,9 @@ cudaError_t reorder_jobs(const SegTable& t, cudaStream_t st) {
   if (t.k < 1 || t.k > kReorderMaxK || t.n_jobs > kSegMaxJobs) return cudaErrorInvalidValue;
   const int nb = bins_for(t.k);
   const size_t smem = (size_t)nb * 4;
-  cudaError_t e = cudaSuccess;
   const size_t sort_smem = scatter_smem(nb);
-  if (sort_smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(seg_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sort_smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem(seg_scatter_kernel, sort_smem);
+  if (e != cudaSuccess) return e;
   seg_bin_count_kernel<<<t.total_chunks, kThreads, smem, st>>>(t);
   seg_scan_bins_kernel<<<dim3(nb, t.n_jobs), kThreads, 0, st>>>(t);
   seg_scan_totals_kernel<<<t.n_jobs, kThreads, 0, st>>>(t);
@@ -356,13 +353,9 @@ cudaError_t reorder_rays(const bvhgpu_ray_t* rays, uint64_t n, int k, uint32_t* 
   const uint64_t blocks = blocks_for(n);
   const Scratch s = carve(scratch, n, k);
   const size_t smem = (size_t)nb * 4;
-  cudaError_t e = cudaSuccess;
   const size_t sort_smem = scatter_smem(nb);
-  if (sort_smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sort_smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem(scatter_kernel, sort_smem);
+  if (e != cudaSuccess) return e;
   bin_count_kernel<<<(unsigned)blocks, kThreads, smem, st>>>(rays, n, k, s, blocks);
   scan_bins_kernel<<<nb, kThreads, 0, st>>>(s, blocks);
   scan_totals_kernel<<<1, kThreads, 0, st>>>(s, nb);
