@@ -805,6 +805,7 @@ static int trace_device(bvhgpu_scene_t s, const bvhgpu_ray_t* rays, uint64_t n,
       return set_error(BVHGPU_ERR_BAD_ARG, "fullness: needs depth_hist (2 x 64 + 2 x 17 entries)");
     a.fullness = a.depth_hist + 128;
   }
+  a.block_hist = s->layout.visits_fit_32(dev::kHistRays);
   a.stack_cap = stack_cap(s);
   if (step_stats) {
     if (cfg.scheme != BVHGPU_STREAM || !cfg.count || !step_count || step_cap < 1 || cfg.reorder)

@@ -85,6 +85,11 @@ struct DeviceLayout {
   // Every child box is finite with lo <= hi on each axis (FP32 records), so
   // a slab test may take the near / far planes by the sign of 1/direction.
   bool boxes_ordered = true;
+  // Whether `rays` rays together visit less than 2^32 nodes and leaves each (a
+  // ray visits each at most once), so that 32 bits count their visits.
+  bool visits_fit_32(uint64_t rays) const {
+    return rays * (n_inner > n_leaves ? n_inner : n_leaves) <= 0xFFFFFFFFull;
+  }
 };
 
 constexpr uint32_t kLeafBit = 0x80000000u;

@@ -33,11 +33,12 @@ struct LaunchCfg {
   bool any_order = false;       // any-hit rays without counters: child-index push order
 };
 
-// Room for the block's visit histogram after `smem` bytes, if it is wanted and
-// fits (else the kernel counts in global memory).
+// Room for the block's visit histogram after `smem` bytes, if it is wanted, its
+// words are wide enough (a.block_hist) and it fits (else the kernel counts in
+// global memory).
 inline size_t add_block_hist(TraceArgs& a, bool count, size_t smem) {
   const size_t bytes = kHistBins * sizeof(uint32_t);
-  a.block_hist = count && a.depth_hist != nullptr && smem + bytes <= 227 * 1024;
+  a.block_hist = a.block_hist && count && a.depth_hist != nullptr && smem + bytes <= 227 * 1024;
   return a.block_hist ? smem + bytes : smem;
 }
 

@@ -111,7 +111,7 @@ struct TraceArgs {
   // visit counts as one step) instead of intersectWideAlternative's.
   bool step_wide = false;
   // With depth_hist: the block has kHistBins words of shared memory for its
-  // own histogram (see hist_flush).
+  // own histogram (see hist_flush). Until the launch: whether it may have.
   bool block_hist = false;
 };
 
@@ -806,6 +806,7 @@ BVHGPU_DEV void record_error(int* status, int code) { atomicCAS(status, 0, code)
 // [64, 128) leaf visits per depth, [128, 145) visits of nodes with c children,
 // [145, 162) of leaves with c triangles.
 constexpr int kHistBins = 128 + 34;
+constexpr int kHistRays = 256;  // rays of a block at most (a stream packet)
 
 // Counting launches: one node visit (depth_count = depth | child count << 8,
 // as node_step returns it) into the per-depth histogram and childFullness
@@ -837,11 +838,11 @@ BVHGPU_DEV void count_leaf(const TraceArgs& a, const uint8_t* leaf_depth, uint32
 
 // The block's histogram: every visit of a launch adds to a few dozen bins, so
 // 64-bit atomics on global memory queue up behind one another in L2. A block
-// adds to its own copy in shared memory (32-bit: a block has at most 256 rays)
-// and to global memory once per bin at its end: 640 x 360 primary and shadow
-// rays on a 251k-triangle N16L16 tree 4.31 -> 0.36 ms. The persistent kernel,
-// whose blocks take any number of rays, keeps the 64-bit atomics on global
-// memory.
+// adds to its own copy in shared memory (32-bit, for trees whose nodes and leaves
+// times the block's rays stay below 2^32) and to global memory once per bin at
+// its end: 640 x 360 primary and shadow rays on a 251k-triangle N16L16 tree 4.31
+// -> 0.36 ms. The persistent kernel, whose blocks take any number of rays, keeps
+// the 64-bit atomics on global memory, and so do the others for larger trees.
 BVHGPU_DEV void hist_clear(uint32_t* hist) {
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0u;
   __syncthreads();
