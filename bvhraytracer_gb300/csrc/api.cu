@@ -361,6 +361,12 @@ static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
                        (int8_t)(L.boxes_nested ? 1 : 0), (int8_t)leaves};
 }
 
+static dev::PackedCfg packed_cfg(const bvhgpu_scene* s, const dev::TraceArgs& a,
+                                 const dev::LaunchCfg& c) {
+  return dev::PackedCfg{s->layout.node_stride, s->layout.node_format, c.kind, c.profile,
+                        c.any_order, a.out_index != nullptr, s->sm_count, pack_bytes(s)};
+}
+
 // A trace on the packed scene.
 static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c,
                                cudaStream_t st) {
@@ -370,8 +376,7 @@ static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const d
   p.scene = pack_view(s, c.kind == BVHGPU_ANY ? (void*)a.occluded : (void*)a.hits);
   p.rays = a.rays;
   p.out_index = a.out_index;
-  const dev::PackedCfg cfg{s->layout.node_stride, s->layout.node_format, c.kind, c.profile,
-                           c.any_order, a.out_index != nullptr, s->sm_count, pack_bytes(s)};
+  const dev::PackedCfg cfg = packed_cfg(s, a, c);
   cudaError_t e;
   if (c.count) {
     switch (cfg.nm) {
@@ -1736,10 +1741,11 @@ int bvhgpu_scene_status(bvhgpu_scene_t s, void* stream) {
 // that device, and again on the first call after the device's context was
 // destroyed and re-created (cudaDeviceReset), since the array then lives at a
 // new address; make that first call before any stream capture. The first call
-// with a given ray kind, profile, policy and node width may also load that
-// kernel variant into the context (CUDA's lazy module loading), which can
-// take device memory for the code itself; a caller that must see no device
-// memory change at all warms up every combination it will use.
+// with a given ray kind, profile, policy, node width and node format may also
+// load kernels into the context (CUDA's lazy module loading), which can take
+// device memory for the code itself: all that such a batch may run on, whatever
+// its size (packed scenes choose the kernel by it). A caller that must see no
+// device memory change at all warms up every combination it will use.
 // Every call shares the array and leaves its contents behind: each call clears
 // the heads it uses before its launches, and calls that overlap on the GPU
 // (different streams of one device) race on the heads, so serialise them.
@@ -1752,6 +1758,7 @@ constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
 unsigned long long* g_noalloc_addr[kNoAllocMaxDevices] = {};
 unsigned long long g_noalloc_ctx[kNoAllocMaxDevices] = {};  // context id of each address
+uint32_t g_noalloc_loaded[kNoAllocMaxDevices] = {};  // kernel sets loaded into that context
 
 // Unique id of the calling thread's current context (ids are never reused
 // within a process, unlike context handles), through the driver entry points
@@ -1793,9 +1800,28 @@ int noalloc_scratch(int device, unsigned long long** out) {
     if (e != cudaSuccess) return cuda_error(e, "no-alloc trace: cudaGetSymbolAddress");
     g_noalloc_addr[device] = static_cast<unsigned long long*>(p);
     g_noalloc_ctx[device] = ctx;
+    g_noalloc_loaded[device] = 0;
   }
   *out = g_noalloc_addr[device];
   return BVHGPU_OK;
+}
+
+// Loads the kernels that a batch may run on, once per device and context
+// (after noalloc_scratch; `device` is current).
+cudaError_t noalloc_load(int device, const dev::PackedCfg& c) {
+  const uint32_t set = 1u << ((c.nm / 4 - 1) * 8 + (c.fmt == BVHGPU_NODES_Q8) * 4 +
+                              (c.profile == BVHGPU_PROFILE_FAST) * 2 + (c.kind == BVHGPU_ANY));
+  std::lock_guard<std::mutex> lock(g_noalloc_mu);
+  if (g_noalloc_loaded[device] & set) return cudaSuccess;
+  cudaError_t e;
+  switch (c.nm) {
+    case 4: e = dev::load_one_scene<4>(c); break;
+    case 8: e = dev::load_one_scene<8>(c); break;
+    case 12: e = dev::load_one_scene<12>(c); break;
+    default: e = dev::load_one_scene<16>(c); break;
+  }
+  if (e == cudaSuccess) g_noalloc_loaded[device] |= set;
+  return e;
 }
 
 }  // namespace
@@ -1865,7 +1891,8 @@ int bvhgpu_trace_batches_noalloc(bvhgpu_scene_t s, const bvhgpu_batch_t* batches
     c.top_nodes = std::min(s->layout.top_nodes, kTopStageBytes / (uint32_t)s->layout.record_bytes);
     c.stall_bytes = s->stall_bytes;
     if (uses_pool(s, a, c)) {
-      e = launch_pool(s, a, c, st);
+      e = noalloc_load(s->device, packed_cfg(s, a, c));
+      if (e == cudaSuccess) e = launch_pool(s, a, c, st);
       if (e != cudaSuccess) return cuda_error(e, "no-alloc trace launch");
       continue;
     }

@@ -21,6 +21,9 @@ struct PackedCfg {
 // Width NM of one scene or many (pool_n*.cu, pool_jobs_n*.cu).
 template <int NM> cudaError_t launch_one_scene(OneScene& p, const PackedCfg& c, cudaStream_t s);
 template <int NM> cudaError_t launch_many_scenes(ManyScenes& p, const PackedCfg& c, cudaStream_t s);
+// Loads the code of every kernel that launch_one_scene may choose for a ray
+// kind, profile and format, whatever the batch's size and push order.
+template <int NM> cudaError_t load_one_scene(const PackedCfg& c);
 // The counting kernel for the rays of p, counters and histograms as in a.
 template <int NM> cudaError_t launch_counting(OneScene& p, TraceArgs a, const PackedCfg& c, cudaStream_t s);
 
@@ -150,6 +153,41 @@ inline cudaError_t launch_packed_fmt(SRC& p, const PackedCfg& c, cudaStream_t s)
   if (c.profile == F) return launch_packed<NM, F, A, FMT, false>(p, c, s);
   return c.any_order ? launch_packed<NM, I, A, FMT, false>(p, c, s)
                      : launch_packed<NM, I, A, FMT, true>(p, c, s);
+}
+
+// A kernel's code is loaded when its attributes are first asked for.
+template <typename K>
+inline void load_kernel(K kernel, cudaError_t& e) {
+  cudaFuncAttributes a;
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+}
+template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED>
+inline void load_order(cudaError_t& e) {
+  load_kernel(trace_team_kernel<NM, PROFILE, KIND, FMT, ORDERED, OneScene>, e);
+  load_kernel(trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, true, OneScene>, e);
+  load_kernel(trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, false, OneScene>, e);
+  load_kernel(trace_pool_kernel<NM, PROFILE, KIND, FMT, ORDERED, OneScene>, e);
+}
+template <int NM, int FMT>
+inline cudaError_t load_fmt(const PackedCfg& c) {
+  constexpr int F = BVHGPU_PROFILE_FAST, I = BVHGPU_PROFILE_INSTRUMENTED;
+  constexpr int C = BVHGPU_CLOSEST, A = BVHGPU_ANY;
+  cudaError_t e = cudaSuccess;
+  load_kernel(plan_kernel<OneScene>, e);
+  if (c.kind == C) {
+    if (c.profile == F) load_order<NM, F, C, FMT, true>(e);
+    else load_order<NM, I, C, FMT, true>(e);
+  } else if (c.profile == F) {
+    load_order<NM, F, A, FMT, false>(e);
+  } else {
+    load_order<NM, I, A, FMT, true>(e);
+    load_order<NM, I, A, FMT, false>(e);
+  }
+  return e;
+}
+template <int NM>
+inline cudaError_t load_width(const PackedCfg& c) {
+  return c.fmt == kFmtQ8 ? load_fmt<NM, kFmtQ8>(c) : load_fmt<NM, kFmtFP32>(c);
 }
 
 template <int NM, int KIND, int FMT>

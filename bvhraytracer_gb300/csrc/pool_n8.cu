@@ -6,6 +6,7 @@ namespace dev {
 template <> cudaError_t launch_one_scene<8>(OneScene& p, const PackedCfg& c, cudaStream_t s) {
   return launch_packed_width<8>(p, c, s);
 }
+template <> cudaError_t load_one_scene<8>(const PackedCfg& c) { return load_width<8>(c); }
 template <> cudaError_t launch_counting<8>(OneScene& p, TraceArgs a, const PackedCfg& c, cudaStream_t s) {
   return launch_count_width<8>(p, a, c, s);
 }

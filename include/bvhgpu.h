@@ -446,16 +446,18 @@ int bvhgpu_unpack_hits(const bvhgpu_hit_t* hits, uint64_t n, int32_t* prim, floa
  * whose host application owns the memory budget, a frame loop that cannot
  * take the synchronisation an allocation may cause): traces up to 64 ray
  * batches with kernels whose scratch (two queue words per batch) lives in a
- * fixed 1 KB device array inside the library instead of being allocated. More than 64 batches -> BVHGPU_ERR_BAD_ARG. The first call
- * on a device, and the first after that device's context was destroyed and
- * re-created (cudaDeviceReset), looks up that array's address: make it before
- * any stream capture. The first call with a given kind, profile, policy and
- * node width may also load that kernel variant (CUDA lazy loading), which can
- * take device memory for its code: warm up each combination once where no
- * change of free device memory may be seen. All calls share the array: calls
- * that overlap on the GPU race. opts: profile, policy, refill and any_order
- * are used; scheme is always persistent; reorder, save_distance and
- * stack_local -> BVHGPU_ERR_UNSUPPORTED. */
+ * fixed 1 KB device array inside the library instead of being allocated. More
+ * than 64 batches -> BVHGPU_ERR_BAD_ARG. The first call on a device, and the
+ * first after that device's context was destroyed and re-created
+ * (cudaDeviceReset), looks up that array's address: make it before any stream
+ * capture. The first call with a given kind, profile, policy, node width and
+ * node format may also load the kernels that such batches of any size run on
+ * (CUDA lazy loading), which can take device memory for their code: warm up
+ * each combination once, with a batch of any size, where no change of free
+ * device memory may be seen. All calls share the array: calls that overlap on
+ * the GPU race. opts: profile, policy, refill and any_order are used; scheme is
+ * always persistent; reorder, save_distance and stack_local ->
+ * BVHGPU_ERR_UNSUPPORTED. */
 typedef struct {
   const bvhgpu_ray_t* rays; /* device, 16-byte aligned */
   uint64_t n;
