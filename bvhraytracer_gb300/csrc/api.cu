@@ -84,6 +84,12 @@ struct bvhgpu_scene {
   unsigned long long* d_queue = nullptr;
   std::atomic<unsigned> queue_next{0};
   unsigned long long* next_queue() { return d_queue + queue_next.fetch_add(1) % kQueueSlots; }
+  // Word pairs for launches recorded into CUDA graphs (see PoolQueue).
+  static constexpr int kGraphSlots = 1024;
+  std::atomic<unsigned> graph_next{0};
+  unsigned long long* next_graph_words() {
+    return d_queue + kQueueSlots + 2 * (graph_next.fetch_add(1) % kGraphSlots);
+  }
   int sm_count = 0;
   // Staging for bvhgpu_trace_host (grown on demand): one region per
   // pipeline stream, and the streams / events that order them.
@@ -324,23 +330,34 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
 }
 
 // Two words of device memory for a large launch on the packed scene: the
-// caller's or stream-ordered scratch, freed behind the launch. A stream that is
-// being captured gets none (an allocation would put memory nodes into the
-// caller's graph), nor does a full device: then every ray has its own thread.
+// caller's or stream-ordered scratch, freed behind the launch. An allocation in a
+// stream that is being captured would put memory nodes into the caller's graph.
+// There a launch of the persistent scheme takes a pair of its scene's, one per
+// recorded launch (as the scheme's own kernel takes its queue head from the
+// scene), so a recorded launch must not run twice at the same time; 4M unordered
+// rays on 250k triangles, us, the scheme's own kernel / a thread per ray /
+// with the words: N8L8 closest-hit 3681 / 4150 / 2795, N4L8 3637 / 4130 / 3300, any-hit
+// rays of the fast profile, Q8 N8L4 2104 / 2465 / 1111. Other schemes, which never had
+// such a limit, get none, nor does a full device: then every ray has its own
+// thread (per-ray kernel / a thread per ray: N8L8 5901 / 4150).
 struct PoolQueue {
   unsigned long long* words = nullptr;
   void* scratch = nullptr;
-  PoolQueue(int device, const dev::PackedCfg& c, uint64_t n, unsigned long long* given,
-            cudaStream_t st)
+  PoolQueue(bvhgpu_scene* s, const dev::PackedCfg& c, uint64_t n, unsigned long long* given,
+            bool persistent, cudaStream_t st)
       : words(given) {
     if (given || !dev::pool_wants_queue(c, n)) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
-    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
-        capture == cudaStreamCaptureStatusNone &&
-        scratch_alloc(device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
-      words = static_cast<unsigned long long*>(scratch);
-    else
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusInvalidated;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
       cudaGetLastError();
+    } else if (capture == cudaStreamCaptureStatusActive) {
+      if (persistent) words = s->next_graph_words();
+    } else if (capture == cudaStreamCaptureStatusNone) {
+      if (scratch_alloc(s->device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
+        words = static_cast<unsigned long long*>(scratch);
+      else
+        cudaGetLastError();
+    }
   }
   cudaError_t free(cudaStream_t st) {
     return scratch ? cudaFreeAsync(scratch, st) : cudaSuccess;
@@ -386,7 +403,7 @@ static cudaError_t launch_pool(bvhgpu_scene* s, const dev::TraceArgs& a, const d
       default: return dev::launch_counting<16>(p, a, cfg, st);
     }
   }
-  PoolQueue queue(s->device, cfg, a.n, c.pool_queue, st);
+  PoolQueue queue(s, cfg, a.n, c.pool_queue, c.scheme == BVHGPU_PERSISTENT, st);
   p.queue = queue.words;
   switch (cfg.nm) {
     case 4: e = dev::launch_one_scene<4>(p, cfg, st); break;
@@ -704,7 +721,8 @@ int bvhgpu_scene_create(bvhgpu_bvh_t h, const bvhgpu_scene_params_t* params, bvh
   }
   if (e == cudaSuccess) e = pack_scene(s);
   if (e == cudaSuccess)
-    e = cudaMalloc((void**)&s->d_queue, sizeof(unsigned long long) * bvhgpu_scene::kQueueSlots);
+    e = cudaMalloc((void**)&s->d_queue, sizeof(unsigned long long) *
+                                       (bvhgpu_scene::kQueueSlots + 2 * bvhgpu_scene::kGraphSlots));
   if (e == cudaSuccess)
     e = cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device);
   if (e != cudaSuccess) {
@@ -1154,8 +1172,8 @@ extern "C" {
 // ambient-occlusion jobs in a CUDA graph 3.96 -> 3.52 ms (a plain call 3.57).
 constexpr int kMaxJobGroups = 4 * 2 * (2 + 4);  // widths, formats, (kind, push order, ray order)
 static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, const dev::JobTable& t,
-                                      int profile, int device, int sms,
-                                      unsigned long long* words, cudaStream_t st) {
+                                      int profile, int sms, unsigned long long* words,
+                                      cudaStream_t st) {
   static_assert(dev::kPoolMaxJobs == dev::kMaxJobs, "job limit");
   std::unique_ptr<dev::ManyScenes> p(new (std::nothrow) dev::ManyScenes());
   if (!p) return cudaErrorMemoryAllocation;
@@ -1178,7 +1196,7 @@ static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, cons
     p->n = 0;
     p->n_jobs = 0;
     p->levels = 1;
-    const bvhgpu_scene* last = nullptr;  // a scene's jobs mostly follow one another
+    bvhgpu_scene *first = nullptr, *last = nullptr;  // a scene's jobs mostly follow one another
     for (int i = 0, k = 0; i < n_jobs; ++i) {
       if (jobs[i].n == 0) continue;
       const dev::JobDev& d = t.jobs[k];
@@ -1192,8 +1210,9 @@ static cudaError_t launch_packed_jobs(const bvhgpu_job_t* jobs, int n_jobs, cons
       p->levels = std::max(p->levels, jobs[i].scene->layout.inner_levels);
       if (jobs[i].scene != last) cfg[g].node_bytes += pack_bytes(jobs[i].scene);
       last = jobs[i].scene;
+      if (!first) first = last;
     }
-    PoolQueue queue(device, cfg[g], p->n, words ? words + 2 * g : nullptr, st);
+    PoolQueue queue(first, cfg[g], p->n, words ? words + 2 * g : nullptr, true, st);
     p->queue = queue.words;
     cudaError_t e;
     switch (cfg[g].nm) {
@@ -1322,7 +1341,7 @@ int bvhgpu_trace_jobs(const bvhgpu_job_t* jobs, int32_t n_jobs, const bvhgpu_tra
   for (int i = 0; i < n_jobs; ++i)
     if (jobs[i].n != 0 && !scene_uses_pool(jobs[i].scene)) packed = false;
   if (packed) {
-    e = launch_packed_jobs(jobs, n_jobs, *t, cfg.profile, device, sms, words, st);
+    e = launch_packed_jobs(jobs, n_jobs, *t, cfg.profile, sms, words, st);
     if (scratch) {
       cudaError_t f = cudaFreeAsync(scratch, st);
       if (e == cudaSuccess) e = f;

@@ -259,7 +259,10 @@ typedef struct {
 
 /* Device pointers. Closest: writes hits[n]. Any: writes occluded[n] (0/1).
  * Rays whose origin x is NaN are skipped (miss / not occluded), like the
- * reference's inactive secondary rays. */
+ * reference's inactive secondary rays. Stream-ordered; can be recorded in a
+ * CUDA graph. A recorded launch of the persistent scheme keeps its queue in the
+ * scene, so it must not run twice at the same time (replays of one executable
+ * graph never do). */
 int bvhgpu_trace(bvhgpu_scene_t scene, const bvhgpu_ray_t* rays, uint64_t n,
                  const bvhgpu_trace_opts_t* opts, bvhgpu_hit_t* hits, uint8_t* occluded,
                  uint32_t* counters, uint64_t* depth_hist, void* stream);
@@ -316,7 +319,8 @@ int bvhgpu_trace_host_batches(bvhgpu_scene_t scene, const bvhgpu_host_batch_t* b
  * scenes). Results per ray
  * equal bvhgpu_trace's. All scenes must live on the stream's device; the
  * options' profile and policy (0 or 2) apply to every job. Stream-ordered, no
- * synchronisation (so it can be recorded in a CUDA graph). Scratch comes from
+ * synchronisation (so it can be recorded in a CUDA graph; without reordered
+ * jobs, see bvhgpu_trace for the persistent scheme). Scratch comes from
  * the stream-ordered allocator (cudaMallocAsync / cudaFreeAsync on the
  * stream): about 6 bytes per ray of reordered jobs, which graph capture
  * records as memory nodes, and in calls without one, outside a capture, 16
