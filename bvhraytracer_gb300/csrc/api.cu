@@ -302,7 +302,9 @@ static bool counts_packed(const bvhgpu_scene* s, const dev::TraceArgs& a, const 
 // the library's own (one per device, created on first use) that keeps freed
 // memory instead of returning it at every synchronisation, so repeated
 // traces reuse it; the process's default pool is left as the caller set it.
-static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
+// optional: the caller does without, so a failure is not an error of the call.
+static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st,
+                         bool optional = false) {
   static std::mutex mu;
   static std::vector<cudaMemPool_t> pools;
   cudaMemPool_t pool = nullptr;
@@ -318,7 +320,7 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
       cudaError_t e = cudaMemPoolCreate(&pools[device], &props);
       if (e != cudaSuccess) {
         pools[device] = nullptr;
-        return cuda_error(e, "scratch memory pool");
+        return optional ? BVHGPU_ERR_CUDA : cuda_error(e, "scratch memory pool");
       }
       uint64_t keep = ~0ull;
       cudaMemPoolSetAttribute(pools[device], cudaMemPoolAttrReleaseThreshold, &keep);
@@ -326,7 +328,8 @@ static int scratch_alloc(int device, void** p, size_t bytes, cudaStream_t st) {
     pool = pools[device];
   }
   cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
-  return e == cudaSuccess ? BVHGPU_OK : set_error(BVHGPU_ERR_OOM, "scratch allocation failed");
+  if (e == cudaSuccess) return BVHGPU_OK;
+  return optional ? BVHGPU_ERR_OOM : set_error(BVHGPU_ERR_OOM, "scratch allocation failed");
 }
 
 // Two words of device memory for a large launch on the packed scene: the
@@ -353,7 +356,7 @@ struct PoolQueue {
     } else if (capture == cudaStreamCaptureStatusActive) {
       if (persistent) words = s->next_graph_words();
     } else if (capture == cudaStreamCaptureStatusNone) {
-      if (scratch_alloc(s->device, &scratch, 2 * sizeof(unsigned long long), st) == BVHGPU_OK)
+      if (scratch_alloc(s->device, &scratch, 2 * sizeof(unsigned long long), st, true) == BVHGPU_OK)
         words = static_cast<unsigned long long*>(scratch);
       else
         cudaGetLastError();
