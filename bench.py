@@ -37,15 +37,15 @@ sys.path.insert(0, str(ROOT))
 METRIC = "Mrays/s"
 
 # DRAM bytes per AO ray (dram__bytes_read.sum + dram__bytes_write.sum) of
-# this workload's AO call (clutter 4,000 objects, N8L8, FP32 nodes;
-# persistent kernel, refill 24, 6 x 10 x 10 direction bins, child-index
-# order), from one ncu capture of `bench.py --workload aolaunch --steps 1
-# --warmup 1` (2,000,000 AO rays, an evenly strided sample of the frame's):
-# the trace kernel 101,412,096 B, the four reorder passes 70,406,912 B. The
+# this workload's AO call (clutter 4,000 objects, N8L8, FP32 nodes; the pool
+# kernel on 6 x 10 x 10 direction bins, child-index order), from one ncu
+# capture of `bench.py --workload aolaunch --steps 1 --warmup 1` (2,000,000 AO
+# rays, an evenly strided sample of the frame's): the trace kernel 90,317,312 B,
+# the four reorder passes 70,942,464 B. The
 # traffic is the ray stream plus the BVH lines that miss L2, so it is scaled
 # to a launch by its ray count.
-NCU_DRAM_BYTES_PER_AO_RAY = {"trace": 101412096 / 2e6,
-                             "with_reorder": (101412096 + 70406912) / 2e6}
+NCU_DRAM_BYTES_PER_AO_RAY = {"trace": 90317312 / 2e6,
+                             "with_reorder": (90317312 + 70942464) / 2e6}
 
 
 def parse():
@@ -118,6 +118,25 @@ def dist_info():
 def workload_name(a):
     return (f"clutter-{a.objects}obj N{a.branching}L{a.leaf} {a.width}x{a.height} primary "
             f"+1 shadow +{a.ao} AO per hit")
+
+
+# Bytes of a packed FP32 node record by child slots.
+PACKED_NODE = {4: 176, 8: 336, 12: 560, 16: 720}
+
+
+def bvh_bytes(scene, bvh, branching):
+    """Device bytes of an FP32 scene: the general records, one 4-byte stack
+    entry per child slot, the triangle bounds (24 bytes per triangle slot and
+    16 per leaf), and the packed records that traces without counters read."""
+    slots = -(-branching // 4) * 4
+    nodes = scene.node_bytes // scene.node_record_bytes
+    compact = bvh.export_compact()
+    tris = compact["prim_count"][compact["child_count"] == 0]
+    return {"nodes_fp32": scene.node_bytes, "leaves": scene.leaf_bytes,
+            "child_entries": nodes * slots * 4,
+            "triangle_bounds": scene.leaf_bytes * 6 // 9 + 16 * len(tris),
+            "packed_nodes": nodes * PACKED_NODE[slots],
+            "packed_leaf_blocks": int(((tris + 3) // 4).sum()) * 304}
 
 
 def make_frame(a, scene_trace=None):
@@ -516,7 +535,15 @@ def run_ours(a):
     per_kernel_ms = [statistics.mean(e[i][0].elapsed_time(e[i][1]) for e in ev)
                      for i in range(len(batches))]
     value = n_rays * world * a.steps / (ms / 1e3) / 1e6
-    ok = torch.equal(out_h.view(torch.int32), hits0.view(torch.int32))
+    # The same batches on the general records: the persistent scheme's counting
+    # kernel (traces without counters run on the packed ones in every scheme).
+    ok = True
+    for rays, kind, out in ((d_primary, "closest", out_h), (d_shadow, "any", out_s),
+                            (d_ao, "any", out_a)):
+        ref = plain.trace(rays, kind=kind, profile=a.profile, scheme="persistent", counters=True)
+        ref = ref["hits" if kind == "closest" else "occluded"]
+        ok = ok and torch.equal(out.view(torch.uint8), ref.view(torch.uint8))
+        del ref
 
     # End to end through the C-ABI host entry point, pinned host buffers.
     h_rays = [torch.from_numpy(x).pin_memory() for x in (primary, shadow, ao)]
@@ -616,12 +643,7 @@ def run_ours(a):
                 "oracle_equal": parity,
                 "l2": "inputs larger than L2 (rays ~%d MB per step); BVH stays L2-resident"
                       % (n_rays * 32 // 2**20),
-                # beside the records: one 4-byte stack entry per child slot and
-                # 6 of the leaf block's 9 floats per triangle slot (bounds)
-                "bvh_bytes": {"nodes_fp32": plain.node_bytes, "leaves": plain.leaf_bytes,
-                              "child_entries": plain.node_bytes // plain.node_record_bytes
-                              * (-(-a.branching // 4) * 4) * 4,
-                              "triangle_bounds": plain.leaf_bytes * 6 // 9},
+                "bvh_bytes": bvh_bytes(plain, bvh, a.branching),
                 "per_kernel_ms": dict(zip(names, per_kernel_ms)),
                 "ms_per_frame_by_method": compare,
                 "setup_s": round(setup_s, 2),
@@ -636,7 +658,7 @@ def run_ours(a):
                                    "(trace kernel + reorder passes), captured on a 2M-ray "
                                    "strided sample and scaled by rays" if traffic else None),
                 "algorithmic_bytes_per_launch": alg[dom]["bytes"],
-                "bytes_rule": "node visits x node record bytes + triangle tests x 36 B",
+                "bytes_rule": "node visits x general node record bytes + triangle tests x 36 B",
                 "l2_peak": l2_peak, "l2_frac": achieved / l2_peak,
                 "l2_peak_source": "measured: bvhgpu_read_bandwidth, 60 MB buffer read 20 times "
                                   "per launch, L1 bypassed, median of 7",
@@ -998,13 +1020,13 @@ def run_adjoint(a):
 
 
 # DRAM bytes per AO ray of the 8M-triangle scene's AO call (trace kernel +
-# the four reorder passes; policy 2, refill 24, 6 x 10 x 10 bins,
-# child-index order), from one ncu capture each of `bench.py --workload
+# the four reorder passes; the pool kernel, 6 x 10 x 10 bins, child-index
+# order), from one ncu capture each of `bench.py --workload
 # aolaunch --objects 32000 --leaf 4 --ao 16 --steps 1 --warmup 1 [--nodes
-# q8]` (2,000,000 strided AO rays): FP32 209,611,008 + 70,400,256 B, Q8
-# 190,471,680 + 70,404,864 B.
-SCALE8M_DRAM_BYTES_PER_AO_RAY = {"fp32": (209611008 + 70400256) / 2e6,
-                                 "q8": (190471680 + 70404864) / 2e6}
+# q8]` (2,000,000 strided AO rays): FP32 214,769,408 + 70,559,744 B, Q8
+# 195,918,080 + 70,812,160 B.
+SCALE8M_DRAM_BYTES_PER_AO_RAY = {"fp32": (214769408 + 70559744) / 2e6,
+                                 "q8": (195918080 + 70812160) / 2e6}
 
 
 def run_scale(a):

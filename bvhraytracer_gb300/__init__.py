@@ -477,9 +477,11 @@ def ao_factor(occluded, samples: int, stream=None):
 
 def trace_jobs(jobs, *, profile: str = "instrumented", policy: int = 2, refill: int = 16,
                one_launch: bool = False, stream=None) -> None:
-    """Traces many (scene, rays) jobs in one persistent launch per ray kind
-    (and node width and format), or with ``one_launch`` in a single launch
-    whose warps trace one ray kind at a time.
+    """Traces many (scene, rays) jobs together: one batch per ray kind, node
+    width and format (and push and ray order), whatever the scenes. If a scene
+    has no packed records, all jobs run on the persistent multi-scene kernel,
+    one launch per kind, width and format, or with ``one_launch`` a single
+    launch whose warps trace one ray kind at a time.
 
     ``jobs``: list of ``(scene, rays, kind, out)``, ``(scene, rays, kind,
     out, reorder)`` or ``(scene, rays, kind, out, reorder, any_order)`` with

@@ -24,9 +24,9 @@
 // persistent kernel (17.4 lanes per instruction, a fifth of the L1 cycles lost
 // to bank conflicts), 0.81 ms here; 8.3M such rays of the 1M-triangle frame
 // 3.13 -> 2.04 ms; unordered, from the per-ray kernel (6.7 lanes), 4.5M rays,
-// N4L8, 2.97 -> 1.33 ms. Solo, 2.1M primary rays of that frame 0.62 -> 0.44 ms,
-// shadow rays 0.41 -> 0.29 ms: latency and the longest rays (a fifth of the
-// warps resident on average).
+// N4L8, 2.97 -> 1.33 ms. Solo, 2.1M primary rays of that frame 0.64 -> 0.46 ms,
+// shadow rays 0.38 -> 0.24 ms: issue (70 %), latency and the longest rays (a
+// third of the warps resident on average).
 #pragma once
 #include "pack.cuh"
 #include "traverse.cuh"

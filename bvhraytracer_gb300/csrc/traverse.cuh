@@ -43,8 +43,8 @@ struct SceneDev {
   // NodeFmt<N>::NM stack entries per inner node, one per child slot (null:
   // computed from the record).
   const uint32_t* child_entry = nullptr;
-  // Packed leaf records (pack.cuh), 6 * leaf_memory + 4 floats per leaf: each
-  // triangle slot's vertex minima (rows 0-2) and maxima (rows 3-5) per axis
+  // Triangle bounds of the leaf pre-test (leaf_bounds_floats in pack.cuh), 6 *
+  // leaf_memory + 4 floats per leaf: each triangle slot's vertex minima (rows 0-2) and maxima (rows 3-5) per axis
   // (read when BVHGPU_LEAF_BOUNDS).
   const float* leaf_bounds = nullptr;
 };

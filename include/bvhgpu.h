@@ -161,7 +161,13 @@ typedef struct {
 int bvhgpu_scene_create(bvhgpu_bvh_t bvh, const bvhgpu_scene_params_t* params,
                         bvhgpu_scene_t* out);
 int bvhgpu_scene_free(bvhgpu_scene_t scene);
-/* Device bytes of the node array and of the leaf array. */
+/* Device bytes of the node array and of the leaf array: the records of the
+ * schemes' own kernels. A scene also holds 4 bytes per child slot (stack
+ * entries), 28 bytes per triangle slot and 17 per leaf (bounds, ids, depth) and,
+ * where its tree allows, the packed records that most traces read: per node
+ * 176 / 336 / 560 / 720 bytes (FP32, 4 / 8 / 12 / 16 child slots) or 144 / 208 /
+ * 368 / 432 (Q8), and 304 bytes per four triangles of a leaf or part of four.
+ * With one or two triangles per leaf those are most of the scene. */
 int bvhgpu_scene_bytes(bvhgpu_scene_t scene, uint64_t* node_bytes, uint64_t* leaf_bytes,
                        uint64_t* node_record_bytes, uint64_t* leaf_record_bytes);
 
@@ -242,12 +248,13 @@ typedef struct {
                         summed over the rays: visits of nodes with c children
                         (entry 128 + c) and of leaves with c triangles (entry 145 + c),
                         c = 0..16. Instrumented and fast profile, every scheme. */
-  int32_t one_launch; /* bvhgpu_trace_jobs: 0 one persistent launch per group of jobs with
-                        one ray kind, node width and node format; nonzero: one launch for
-                        all jobs, the closest-hit jobs' rays queued before the any-hit
-                        jobs', each warp tracing one kind at a time (it takes any-hit
-                        rays once the closest-hit queue is empty and its lanes are done).
-                        Same results. */
+  int32_t one_launch; /* bvhgpu_trace_jobs, calls with a scene that has no packed records
+                        (others run per group either way): 0 one persistent launch per
+                        group of jobs with one ray kind, node width and node format;
+                        nonzero: one launch for all jobs, the closest-hit jobs' rays
+                        queued before the any-hit jobs', each warp tracing one kind at a
+                        time (it takes any-hit rays once the closest-hit queue is empty
+                        and its lanes are done). Same results. */
 } bvhgpu_trace_opts_t;
 
 /* Counters per ray when `counters` is non-null (8 uint32 per ray):
@@ -312,8 +319,9 @@ int bvhgpu_trace_host_batches(bvhgpu_scene_t scene, const bvhgpu_host_batch_t* b
 /* A job: one ray batch traced in one scene. bvhgpu_trace_jobs traces up to
  * BVHGPU_MAX_JOBS jobs (scenes of any N, L and node format, closest or any
  * hit, uneven sizes) together, per group of jobs with the same ray kind, node
- * width and node format (on packed scenes also the same push and ray order),
- * each kernel compiled for what its jobs share: the rays of the group's jobs
+ * width and node format (on packed scenes also the same push and ray order; a
+ * call with one scene that has no packed records runs all its jobs on the
+ * persistent multi-scene kernel), each kernel compiled for what its jobs share: the rays of the group's jobs
  * are one batch, scenes of any size mixed (the GPU form of the reference's
  * workgroup refill, fastNodeManager.h:92-156, 277-450, extended across
  * scenes). Results per ray
