@@ -38,8 +38,9 @@ struct LaunchCfg {
 // global memory).
 inline size_t add_block_hist(TraceArgs& a, bool count, size_t smem) {
   const size_t bytes = kHistBins * sizeof(uint32_t);
-  a.block_hist = a.block_hist && count && a.depth_hist != nullptr && smem + bytes <= 227 * 1024;
-  return a.block_hist ? smem + bytes : smem;
+  const bool fits = a.block_hist && count && a.depth_hist != nullptr && smem + bytes <= 227 * 1024;
+  a.hist_at = fits ? (uint32_t)(smem / 4) : 0u;
+  return fits ? smem + bytes : smem;
 }
 
 template <int NM, int PROFILE, int KIND, bool COUNT, int FMT>

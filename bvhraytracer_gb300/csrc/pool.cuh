@@ -1026,10 +1026,7 @@ __global__ void __launch_bounds__(128, 6)
   extern __shared__ __align__(16) uint8_t pool_smem[];
   const int stride = (int)blockDim.x;
   typename W::T* stack = reinterpret_cast<typename W::T*>(pool_smem) + threadIdx.x;
-  uint32_t* hist = a.block_hist ? reinterpret_cast<uint32_t*>(
-                                      reinterpret_cast<typename W::T*>(pool_smem) + p.levels * stride)
-                                : nullptr;
-  if (hist != nullptr) hist_clear(hist);
+  hist_clear(a);
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < p.n) {
     uint32_t slot, job;
@@ -1055,7 +1052,7 @@ __global__ void __launch_bounds__(128, 6)
           ctr.box_hits += n;
           held += n;
           ctr.max_stack = max(ctr.max_stack, held);
-          count_node(a, (int)((info >> 8) | (info & 0xFFu) << 8), hist);
+          count_node<true>(a, (int)((info >> 8) | (info & 0xFFu) << 8));
           const bool fresh = left != 0;
           if (fresh) left = pool_positions<NM>(pool_sequence<NM, FMT>(rec, r.bits & 3u), left);
           more = pool_take<NM, FMT, true, false>(v, stack, stride, r, e, left, fresh, sp, e);
@@ -1064,7 +1061,7 @@ __global__ void __launch_bounds__(128, 6)
         if (!more) break;
         ctr.leaf_visits++;
         ctr.tri_tests += (uint32_t)leaf_count(e);
-        count_leaf(a, reinterpret_cast<const uint8_t*>(leaf_blocks(v, e) + kBlockWords - 1), e, hist);
+        count_leaf<true>(a, reinterpret_cast<const uint8_t*>(leaf_blocks(v, e) + kBlockWords - 1), e);
         float tmax = r.tmax;
         if (pool_leaf<I, KIND, true>(v, e, r, c, tmax, &ctr.tri_hits)) {
           hit = true;
@@ -1078,7 +1075,7 @@ __global__ void __launch_bounds__(128, 6)
     if (KIND == BVHGPU_ANY) static_cast<uint8_t*>(v.out)[slot] = hit ? 1 : 0;
     store_counters(a, slot, ctr);
   }
-  if (hist != nullptr) hist_flush(a, hist);
+  hist_flush(a);
 }
 
 // A team of lanes per ray, one child or triangle per lane, for batches too

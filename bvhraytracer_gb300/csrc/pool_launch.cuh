@@ -194,8 +194,10 @@ template <int NM, int KIND, int FMT>
 inline cudaError_t launch_count(OneScene& p, TraceArgs& a, cudaStream_t s) {
   constexpr int kBlock = 128;  // 64: 329 us against 326
   size_t smem = sizeof(typename PoolWord<NM>::T) * p.levels * kBlock;
-  a.block_hist = a.block_hist && a.depth_hist != nullptr;
-  if (a.block_hist) smem += kHistBins * sizeof(uint32_t);
+  if (a.block_hist && a.depth_hist != nullptr) {
+    a.hist_at = (uint32_t)(smem / 4);
+    smem += kHistBins * sizeof(uint32_t);
+  }
   auto k = trace_count_kernel<NM, KIND, FMT>;
   const cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;

@@ -110,9 +110,11 @@ struct TraceArgs {
   // Step log of intersectWide's schedule (a node visit followed by a leaf
   // visit counts as one step) instead of intersectWideAlternative's.
   bool step_wide = false;
-  // With depth_hist: the block has kHistBins words of shared memory for its
-  // own histogram (see hist_flush). Until the launch: whether it may have.
+  // With depth_hist: whether 32 bits hold a block's visits, and if the block has
+  // a histogram of its own (see hist_flush), its first word of the dynamic
+  // shared memory (0: none).
   bool block_hist = false;
+  uint32_t hist_at = 0;
 };
 
 BVHGPU_DEV uint64_t out_slot(const TraceArgs& a, uint64_t rid) {
@@ -812,24 +814,31 @@ constexpr int kHistRays = 256;  // rays of a block at most (a stream packet)
 // as node_step returns it) into the per-depth histogram and childFullness
 // (compactNode.cpp:714-716), one leaf visit into the per-depth histogram and
 // primitiveFullness (compactNode.cpp:653-656; leaf_depth: where the leaf's
-// depth is). hist: the block's own histogram in shared memory, or null:
-// straight to global memory.
-BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count, uint32_t* hist) {
+// depth is). BLOCK: into the block's own histogram where it has one, else
+// straight to global memory. (Its place is a kernel argument: kept as a pointer
+// through the traversal it took the fast profile's closest-hit kernels from 96
+// registers to 120, 4 blocks per SM instead of 5, also without histograms.)
+BVHGPU_DEV uint32_t* block_hist(const TraceArgs& a) {
+  extern __shared__ uint32_t hist_words[];
+  return hist_words + a.hist_at;
+}
+template <bool BLOCK>
+BVHGPU_DEV void count_node(const TraceArgs& a, int depth_count) {
   const int depth = min(depth_count & 0xFF, 63), fill = 128 + min(depth_count >> 8, 16);
-  if (hist != nullptr) {
-    atomicAdd(hist + depth, 1u);
-    atomicAdd(hist + fill, 1u);
+  if (BLOCK && a.hist_at != 0) {
+    atomicAdd(block_hist(a) + depth, 1u);
+    atomicAdd(block_hist(a) + fill, 1u);
     return;
   }
   if (a.depth_hist) atomicAdd(a.depth_hist + depth, 1ull);
   if (a.fullness) atomicAdd(a.fullness + fill - 128, 1ull);
 }
-BVHGPU_DEV void count_leaf(const TraceArgs& a, const uint8_t* leaf_depth, uint32_t e,
-                           uint32_t* hist) {
+template <bool BLOCK>
+BVHGPU_DEV void count_leaf(const TraceArgs& a, const uint8_t* leaf_depth, uint32_t e) {
   const int fill = 128 + 17 + (int)((e >> kLeafCountShift) & 15u) + 1;
-  if (hist != nullptr) {
-    atomicAdd(hist + 64 + min((int)*leaf_depth, 63), 1u);
-    atomicAdd(hist + fill, 1u);
+  if (BLOCK && a.hist_at != 0) {
+    atomicAdd(block_hist(a) + 64 + min((int)*leaf_depth, 63), 1u);
+    atomicAdd(block_hist(a) + fill, 1u);
     return;
   }
   if (a.depth_hist) atomicAdd(a.depth_hist + 64 + min((int)*leaf_depth, 63), 1ull);
@@ -843,11 +852,15 @@ BVHGPU_DEV void count_leaf(const TraceArgs& a, const uint8_t* leaf_depth, uint32
 // its end: 640 x 360 primary and shadow rays on a 251k-triangle N16L16 tree 4.31
 // -> 0.36 ms. The persistent kernel, whose blocks take any number of rays, keeps
 // the 64-bit atomics on global memory, and so do the others for larger trees.
-BVHGPU_DEV void hist_clear(uint32_t* hist) {
+BVHGPU_DEV void hist_clear(const TraceArgs& a) {
+  if (a.hist_at == 0) return;
+  uint32_t* hist = block_hist(a);
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) hist[i] = 0u;
   __syncthreads();
 }
-BVHGPU_DEV void hist_flush(const TraceArgs& a, const uint32_t* hist) {
+BVHGPU_DEV void hist_flush(const TraceArgs& a) {
+  if (a.hist_at == 0) return;
+  const uint32_t* hist = block_hist(a);
   __syncthreads();
   for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) {
     if (hist[i] == 0u) continue;
@@ -910,7 +923,7 @@ BVHGPU_DEV void write_result(const SceneDev& sc, const TraceArgs& a, uint64_t ri
 // One ray of the per-ray scheme, from its record to its result.
 template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST>
 BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t rid,
-                              uint32_t* stack, float* dstack, int stride, uint32_t* hist) {
+                              uint32_t* stack, float* dstack, int stride) {
   const bvhgpu_ray_t in = load_ray(a.rays, out_slot(a, rid));
   if (isnan(in.ox)) {
     Best none;
@@ -934,7 +947,7 @@ BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t r
     const uint32_t e = stack[sp * stride];
     if (DIST && dstack[sp * stride] > tmax) continue;
     if (e & kLeafBit) {
-      if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, hist);
+      if (COUNT) count_leaf<true>(a, sc.leaf_depth + (e & kLeafIndexMask), e);
       bool h = leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr);
       if (h) {
         hit = true;
@@ -949,7 +962,7 @@ BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t r
         best = Best();
         break;
       }
-      if (COUNT) count_node(a, depth, hist);
+      if (COUNT) count_node<true>(a, depth);
       if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
     }
   }
@@ -965,24 +978,30 @@ BVHGPU_DEV void trace_dfs_ray(const SceneDev& sc, const TraceArgs& a, uint64_t r
 // every entry also carries its box's entry distance (in a second shared
 // array after the stack), the root enters with 0, and a pop whose distance
 // exceeds the current tMax is dropped before it is visited or counted.
+// Blocks per SM asked of the compiler (0: its own choice): the variants here fit 5
+// blocks (96 registers) with few spills, but left alone it gives them 106 to 128
+// registers and 4 blocks: counting closest-hit rays, fast profile, Q8 N4L4, 0.6M,
+// 1056 us with 5 blocks, 1182 with 4.
+template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST>
+constexpr int dfs_blocks() {
+  constexpr bool kFast = PROFILE == BVHGPU_PROFILE_FAST, kAny = KIND == BVHGPU_ANY;
+  if (!COUNT) return DIST && !kFast && !kAny && FMT == kFmtFP32 ? 5 : 0;
+  if (kFast) return FMT == kFmtQ8 || DIST || (kAny && N <= 12) ? 5 : 0;
+  return kAny && FMT == kFmtQ8 && N <= 8 ? 5 : 0;
+}
+
 template <int N, int PROFILE, int KIND, bool COUNT, int FMT, bool DIST = false>
-__global__ void __launch_bounds__(128) trace_dfs_kernel(SceneDev sc, TraceArgs a) {
+__global__ void __launch_bounds__(128, dfs_blocks<N, PROFILE, KIND, COUNT, FMT, DIST>())
+    trace_dfs_kernel(SceneDev sc, TraceArgs a) {
   extern __shared__ uint32_t smem[];
   const int stride = (int)blockDim.x;
   uint32_t* stack = smem + threadIdx.x;
   float* dstack = DIST ? reinterpret_cast<float*>(smem + (size_t)a.stack_cap * stride) + threadIdx.x
                        : nullptr;
   const uint64_t rid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if constexpr (COUNT) {
-    // After the stacks, where it fits (TraceArgs::block_hist).
-    uint32_t* hist = a.block_hist ? smem + (size_t)a.stack_cap * stride * (DIST ? 2 : 1) : nullptr;
-    if (hist != nullptr) hist_clear(hist);
-    if (rid < a.n)
-      trace_dfs_ray<N, PROFILE, KIND, COUNT, FMT, DIST>(sc, a, rid, stack, dstack, stride, hist);
-    if (hist != nullptr) hist_flush(a, hist);
-  } else if (rid < a.n) {
-    trace_dfs_ray<N, PROFILE, KIND, COUNT, FMT, DIST>(sc, a, rid, stack, dstack, stride, nullptr);
-  }
+  if (COUNT) hist_clear(a);
+  if (rid < a.n) trace_dfs_ray<N, PROFILE, KIND, COUNT, FMT, DIST>(sc, a, rid, stack, dstack, stride);
+  if (COUNT) hist_flush(a);
 }
 
 
@@ -1098,8 +1117,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
   uint16_t* work0 = reinterpret_cast<uint16_t*>(base);  // list c at work0 + c * P
   base += (size_t)P * 4;
   uint32_t* ctrs = reinterpret_cast<uint32_t*>(base);  // [8][P]
-  uint32_t* hist = COUNT && a.block_hist ? ctrs + 8 * P : nullptr;
-  if (COUNT && hist != nullptr) hist_clear(hist);
+  if (COUNT) hist_clear(a);
 
   const uint64_t first = (uint64_t)blockIdx.x * P;
   const uint64_t rid = first + tid;
@@ -1193,7 +1211,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
       if (log && set_insert(set, 2 * P, e))
         atomicAdd(is_node ? &ctl->unique_nodes : &ctl->unique_leaves, 1);
       auto leaf_visit = [&](uint32_t le) {
-        if (COUNT) count_leaf(a, sc.leaf_depth + (le & kLeafIndexMask), le, hist);
+        if (COUNT) count_leaf<true>(a, sc.leaf_depth + (le & kLeafIndexMask), le);
         Best best;
         best.leaf = best_leaf[ray];
         best.lane = (int)(int8_t)(misc & 0xFF);
@@ -1222,7 +1240,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
           done = true;
           sp = 0;
         }
-        if (COUNT) count_node(a, depth, hist);
+        if (COUNT) count_node<true>(a, depth);
         // intersectWide's schedule (compactNode.cpp:118-356, step log only):
         // a ray whose next entry is a leaf visits it in the same step.
         if (log && a.step_wide && !done && sp > 0 && (stacks[(sp - 1) * P + ray] & kLeafBit)) {
@@ -1302,7 +1320,7 @@ __global__ void __launch_bounds__(256, BVHGPU_STREAM_MIN_BLOCKS)
     __syncthreads();
   }
   if (log && tid == 0) a.step_count[blockIdx.x] = (uint32_t)step;
-  if (COUNT && hist != nullptr) hist_flush(a, hist);
+  if (COUNT) hist_flush(a);
 
   // Results of this thread's own ray slot.
   if (rid < a.n) {
@@ -1529,14 +1547,14 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
             best = Best();
             sp = 0;
           }
-          if (COUNT) count_node(a, depth, nullptr);
+          if (COUNT) count_node<false>(a, depth);
           if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
         }
       }
       if (active && sp > 0) {
         --sp;
         const uint32_t e = stack[sp * stride];
-        if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, nullptr);
+        if (COUNT) count_leaf<false>(a, sc.leaf_depth + (e & kLeafIndexMask), e);
         if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
           hit = true;
           if (KIND == BVHGPU_ANY) sp = 0;
@@ -1547,7 +1565,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
         --sp;
         const uint32_t e = stack[sp * stride];
         if (e & kLeafBit) {
-          if (COUNT) count_leaf(a, sc.leaf_depth + (e & kLeafIndexMask), e, nullptr);
+          if (COUNT) count_leaf<false>(a, sc.leaf_depth + (e & kLeafIndexMask), e);
           if (leaf_step<PROFILE, KIND, COUNT>(sc, e, r, tmax, best, ctr)) {
             hit = true;
             if (KIND == BVHGPU_ANY) sp = 0;
@@ -1561,7 +1579,7 @@ __global__ void __launch_bounds__(128, BVHGPU_PERSIST_MIN_BLOCKS)
             best = Best();
             sp = 0;
           }
-          if (COUNT) count_node(a, depth, nullptr);
+          if (COUNT) count_node<false>(a, depth);
           if (COUNT) ctr.max_stack = max(ctr.max_stack, (uint32_t)sp);
         }
       }
