@@ -289,11 +289,12 @@ static bool uses_pool(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev:
   return !c.count && !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&
          scene_uses_pool(s);
 }
-// Counting traces that have a kernel on the packed scene: per-ray scheme,
-// instrumented profile. (The other schemes count in their own kernels, which
+// Counting traces that run on the packed scene: per-ray scheme, instrumented
+// profile, large batches (pool_counts). (The other schemes count in their own kernels, which
 // is what their step logs and tests are about.)
 static bool counts_packed(const bvhgpu_scene* s, const dev::TraceArgs& a, const dev::LaunchCfg& c) {
   return c.count && c.scheme == BVHGPU_PER_RAY && c.profile == BVHGPU_PROFILE_INSTRUMENTED &&
+         dev::pool_counts(s->layout.node_stride, s->layout.node_format, a.n) &&
          !(c.save_distance && c.kind == BVHGPU_CLOSEST) && a.n <= 0xFFFFFFFFull &&
          scene_uses_pool(s);
 }

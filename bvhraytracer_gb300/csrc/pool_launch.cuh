@@ -57,6 +57,18 @@ inline bool pool_wants_queue(const PackedCfg& c, uint64_t n) {
   return n > BVHGPU_POOL_MIN_RAYS && (c.direction_order || c.nm <= 8 || c.fmt != kFmtFP32 ||
                                       c.node_bytes <= kPoolWideBytes);
 }
+// Whether counting traces of n rays run on the packed scene. Smaller batches,
+// whose time is the longest ray's, are faster in the general per-ray kernel, and so
+// are all on Q8 nodes of more than 8 children. General / packed time, least and
+// median over primary, shadow and random rays, 251k and 33k triangles, two leaf
+// sizes, with histograms and without: FP32 1k rays 0.85 (median), 30k 0.90, 130k
+// 0.87 1.01, 250k N4 1.08 1.12, N8 1.02 1.12, N12 0.94 1.03, N16 0.95 1.06, 1M 1.02
+// 1.25; Q8 250k N4 1.03 1.11, N8 0.92 1.06, N12 0.88 0.98, N16 0.81 0.93, 1M N16 0.88
+// 1.00.
+constexpr uint64_t kCountRays = 3u << 16;
+inline bool pool_counts(int nm, int fmt, uint64_t n) {
+  return n > kCountRays && (fmt == kFmtFP32 || nm <= 8);
+}
 constexpr int kSoloBlock = 64;
 // Batches of up to so many rays run with a team of lanes per ray (closest-hit /
 // any-hit). Solo / team, us, of a call from Python, which itself takes 15-17
@@ -207,11 +219,14 @@ inline cudaError_t launch_count(OneScene& p, TraceArgs& a, cudaStream_t s) {
 template <int NM>
 inline cudaError_t launch_count_width(OneScene& p, TraceArgs& a, const PackedCfg& c, cudaStream_t s) {
   if (p.n == 0) return cudaSuccess;
-  if (c.kind == BVHGPU_CLOSEST)
-    return c.fmt == kFmtQ8 ? launch_count<NM, BVHGPU_CLOSEST, kFmtQ8>(p, a, s)
-                           : launch_count<NM, BVHGPU_CLOSEST, kFmtFP32>(p, a, s);
-  return c.fmt == kFmtQ8 ? launch_count<NM, BVHGPU_ANY, kFmtQ8>(p, a, s)
-                         : launch_count<NM, BVHGPU_ANY, kFmtFP32>(p, a, s);
+  if constexpr (NM <= 8) {
+    if (c.fmt == kFmtQ8)
+      return c.kind == BVHGPU_CLOSEST ? launch_count<NM, BVHGPU_CLOSEST, kFmtQ8>(p, a, s)
+                                      : launch_count<NM, BVHGPU_ANY, kFmtQ8>(p, a, s);
+  }
+  if (c.fmt != kFmtFP32) return cudaErrorNotSupported;  // see pool_counts
+  return c.kind == BVHGPU_CLOSEST ? launch_count<NM, BVHGPU_CLOSEST, kFmtFP32>(p, a, s)
+                                  : launch_count<NM, BVHGPU_ANY, kFmtFP32>(p, a, s);
 }
 
 template <int NM, typename SRC>

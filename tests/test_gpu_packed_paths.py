@@ -77,3 +77,25 @@ def test_wide_trees_on_both_sides_of_the_pool_line(n, l, fmt, objects):
         pkg.trace_jobs(jobs)
         torch.cuda.synchronize()
         assert all(torch.equal(j[3].view(torch.uint8), want.view(torch.uint8)) for j in jobs)
+
+
+@pytest.mark.parametrize("n,l,fmt", [(2, 1, "fp32"), (4, 16, "q8"), (8, 8, "fp32"), (8, 5, "q8"),
+                                     (12, 13, "fp32"), (12, 5, "q8"), (16, 16, "fp32"),
+                                     (16, 4, "q8")])
+def test_counting_traces_of_large_batches(n, l, fmt):
+    """Counters, histograms and results on both sides of the size from which
+    counting traces run on the packed scene, against the persistent kernel's."""
+    tris = S.clutter(20, 4)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    line = 3 << 16
+    rays = _rays(tris, line + 1, n + l)
+    for d in (rays[:line], rays):
+        for kind in ("closest", "any"):
+            key = "hits" if kind == "closest" else "occluded"
+            want = scene.trace(d, kind=kind, scheme="persistent", counters=True, depth_hist=True)
+            for opts in ({"depth_hist": True}, {"depth_hist": True, "reorder": 3}, {}):
+                got = scene.trace(d, kind=kind, counters=True, **opts)
+                for k in ("counters", "depth_hist", "fullness") if opts else ("counters",):
+                    assert torch.equal(got[k], want[k]), (kind, opts, k)
+                assert torch.equal(got[key].view(torch.uint8), want[key].view(torch.uint8)), (kind, opts)
+    scene.status()
