@@ -61,8 +61,8 @@ constexpr int kPoolWarps = 4;  // per block
 // 0.45 0.47.
 template <int NM, int FMT>
 constexpr int kSoloBlocks = NM > 4 && FMT == kFmtQ8 ? 6 : 7;
-// The same for launches of no more rays than these blocks hold (FEW): up to 128
-// registers. N16L8, 40k / 65k unordered closest-hit rays, us, 3 / 4 / 5 blocks: 92
+// The same for launches of no more rays than these blocks hold, or little more
+// (FEW, kFewLimit): up to 128 registers. N16L8, 40k / 65k unordered closest-hit rays, us, 3 / 4 / 5 blocks: 92
 // 96 98 / 112 105 108 (3 blocks hold 58k rays).
 constexpr int kSoloFewBlocks = 4;
 
@@ -936,8 +936,8 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // the push sequence (and the entries of 4 children) together with the boxes
 // instead of after them. 40k unordered closest-hit rays (L8, 251k triangles), us,
 // of the general per-ray kernel / this one without FEW / with it: N4 119 / 125 /
-// 98, N8 103 / 112 / 96, N12 111 / 131 / 108, N16 103 / 116 / 96. Beyond one
-// wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it.
+// 98, N8 103 / 112 / 96, N12 111 / 131 / 108, N16 103 / 116 / 96. Well beyond
+// one wave of its blocks it loses: N8, 131k rays, 149 without / 189 with it.
 //
 // kLeavesInTurn: a lane that reaches a leaf visits it after the warp's current
 // node step, instead of when every lane has a leaf. A leaf of few triangles

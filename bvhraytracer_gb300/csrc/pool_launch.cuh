@@ -75,10 +75,12 @@ constexpr int kSoloBlock = 64;
 // (251k triangles): N8 primary rays 1k 25 / 25, 4k 60 / 36, 16k 58 / 43, 33k
 // 60 / 61; N8 ambient-occlusion rays 1k 46 / 21, 4k 47 / 24, 16k 56 / 39, 33k
 // 82 / 60, 66k 84 / 82; N16 primary rays 16k 57 / 41, 33k 59 / 76, any-hit rays
-// 16k 61 / 37, 33k 86 / 61, 66k 97 / 91.
-#ifndef BVHGPU_TEAM_MAX_CLOSEST
-#define BVHGPU_TEAM_MAX_CLOSEST 16384
-#endif
+// 16k 61 / 37, 33k 86 / 61, 66k 97 / 91. Closest-hit rays, solo / team time, least
+// and median over primary and random rays, 251k and 33k triangles, leaf sizes 1, 4
+// and 8, both formats: 28k rays N4 0.74 0.93, N8 0.89 1.12, N12 0.89 1.10, N16 1.06
+// 1.30; 33k N8 0.81 1.08, N12 0.79 1.07, N16 0.87 1.20; 18k N4 0.80 0.93.
+template <int NM>
+constexpr uint32_t kTeamMaxClosest = NM <= 4 ? 16384 : NM <= 12 ? 28672 : 32768;
 #ifndef BVHGPU_TEAM_MAX_ANY
 #define BVHGPU_TEAM_MAX_ANY 32768
 #endif
@@ -89,13 +91,21 @@ constexpr int kSoloBlock = 64;
 #endif
 constexpr int kTeamBlock = 64;
 
+// Batches of up to so many blocks' rays per SM run in the solo kernel of one wave,
+// also those that need a little more than one (four blocks, 78k rays). The other
+// solo kernel's time / its, least and median over primary and random rays: 80k
+// rays N4 0.99 1.10, N8 0.97 1.04, FP32 N16 closest-hit 0.86 1.01, Q8 0.83 0.97;
+// 100k N4 0.99 1.09, N8 0.82 1.01, N16 0.81 0.94; 131k N4 0.83 1.03, N8 0.80 0.99.
+template <int NM, int KIND, int FMT>
+constexpr int kFewLimit = NM <= 4 ? 6 : NM <= 8 || (KIND == BVHGPU_CLOSEST && FMT == kFmtFP32) ? 5 : 4;
+
 // The traces of one launch: a team per ray, one thread per ray, pools, or both
 // of these with the rays' own choice between them.
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, typename SRC>
 inline cudaError_t launch_packed(SRC& p, const PackedCfg& c, cudaStream_t s) {
   const int sm_count = c.sm_count;
   cudaError_t e;
-  if (p.n <= (KIND == BVHGPU_ANY ? BVHGPU_TEAM_MAX_ANY : BVHGPU_TEAM_MAX_CLOSEST)) {
+  if (p.n <= (KIND == BVHGPU_ANY ? BVHGPU_TEAM_MAX_ANY : kTeamMaxClosest<NM>)) {
     auto k = trace_team_kernel<NM, PROFILE, KIND, FMT, ORDERED, SRC>;
     constexpr int kMost = 32 / kTeam<NM>;
     // As few rays per warp as keep the warps resident.
@@ -117,7 +127,7 @@ inline cudaError_t launch_packed(SRC& p, const PackedCfg& c, cudaStream_t s) {
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (!pool) {
-    auto k = p.n <= (uint64_t)sm_count * kSoloFewBlocks * 128
+    auto k = p.n <= (uint64_t)sm_count * kFewLimit<NM, KIND, FMT> * 128
                  ? trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, true, SRC>
                  : trace_solo_kernel<NM, PROFILE, KIND, FMT, ORDERED, false, SRC>;
     // A planned launch takes blocks of twice the size: if the pool is chosen,

@@ -99,3 +99,17 @@ def test_counting_traces_of_large_batches(n, l, fmt):
                     assert torch.equal(got[k], want[k]), (kind, opts, k)
                 assert torch.equal(got[key].view(torch.uint8), want[key].view(torch.uint8)), (kind, opts)
     scene.status()
+
+
+@pytest.mark.parametrize("n,l,fmt", [(4, 4, "fp32"), (4, 4, "q8"), (8, 8, "fp32"), (8, 4, "q8"),
+                                     (12, 9, "fp32"), (16, 16, "q8"), (16, 2, "fp32")])
+def test_lines_between_the_kernels_of_small_and_middle_batches(n, l, fmt):
+    """Teams per ray up to 16,384 to 32,768 closest-hit rays by node width, the
+    solo kernel of one wave up to four to six blocks' rays per SM."""
+    tris = S.clutter(30, 5)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format=fmt)
+    block = torch.cuda.get_device_properties(0).multi_processor_count * 128
+    rays = _rays(tris, 6 * block + 1, n + l, extreme=True)
+    for k in (16384, 28672, 32768, 4 * block, 5 * block, 6 * block):
+        _same(scene, rays[:k])
+        _same(scene, rays[:k + 1])
