@@ -376,8 +376,10 @@ static uint64_t pack_bytes(const bvhgpu_scene* s) {
 
 static dev::PackView pack_view(const bvhgpu_scene* s, void* out) {
   const DeviceLayout& L = s->layout;
+  // 4-wide Q8 nodes cost as much as leaves of 8 (see trace_solo_kernel).
+  const int turn = L.node_format == BVHGPU_NODES_Q8 && L.node_stride == 4 ? 8 : L.node_stride;
   const int leaves = (L.most_leaf <= 2 ? dev::kSmallLeaves : 0) |
-                     (L.most_leaf <= L.node_stride ? dev::kLeavesInTurn : 0);
+                     (L.most_leaf <= turn ? dev::kLeavesInTurn : 0);
   return dev::PackView{s->d_pack_nodes, s->d_pack_blocks, out, s->pack_root, (int16_t)L.gang,
                        (int8_t)(L.boxes_nested ? 1 : 0), (int8_t)leaves};
 }

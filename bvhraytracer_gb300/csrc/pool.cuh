@@ -66,8 +66,9 @@ constexpr int kSoloBlocks = NM > 4 && FMT == kFmtQ8 ? 6 : 7;
 // 96 98 / 112 105 108 (3 blocks hold 58k rays).
 constexpr int kSoloFewBlocks = 4;
 
-// PackView::leaves: no leaf has more than two triangles; none has more than a
-// node has child slots (see trace_solo_kernel).
+// PackView::leaves: no leaf has more than two triangles; none costs more than a
+// node: no more triangles than child slots, or 8 with 4-wide Q8 nodes (see
+// trace_solo_kernel).
 constexpr int kSmallLeaves = 1, kLeavesInTurn = 2;
 
 // What a ray's visits need of its scene, and where its result goes.
@@ -946,7 +947,9 @@ __global__ void __launch_bounds__(kPlanWarps * 32) plan_kernel(const __grid_cons
 // (251k triangles), us, general / waiting / in turn: N4L1 335 / 349 / 235, N8L1 316
 // / 363 / 239, N8L8 301 / 253 / 223. With leaves larger than nodes waiting is
 // better: N4L8, 0.26M unordered any-hit rays of the fast profile, 172 waiting / 190
-// in turn.
+// in turn. On Q8 nodes, which are decoded first, 4-wide ones gain up to L8: 131k
+// primary rays 258 / 317 / 223, random closest-hit rays of all sizes 0.90 to 1.17
+// times as fast (median 1.01 to 1.04).
 template <int NM, int PROFILE, int KIND, int FMT, bool ORDERED, bool FEW, typename SRC>
 __global__ void __launch_bounds__(128, FEW ? kSoloFewBlocks : kSoloBlocks<NM, FMT>)
     trace_solo_kernel(const __grid_constant__ SRC p) {

@@ -113,3 +113,15 @@ def test_lines_between_the_kernels_of_small_and_middle_batches(n, l, fmt):
     for k in (16384, 28672, 32768, 4 * block, 5 * block, 6 * block):
         _same(scene, rays[:k])
         _same(scene, rays[:k + 1])
+
+
+@pytest.mark.parametrize("n,l", [(2, 8), (4, 7), (4, 8), (4, 9), (3, 16)])
+def test_leaves_in_turn_on_q8_nodes(n, l):
+    """The leaf sizes where 4-wide Q8 nodes stop visiting leaves in turn."""
+    tris = S.clutter(25, 6)
+    scene = pkg.Scene(pkg.Bvh(tris, n, l), node_format="q8")
+    rays = _rays(tris, 140001, n + l, extreme=True)
+    for k in (40000, 140001):
+        _same(scene, rays[:k])
+    cam, target, _ = S.clutter_viewpoints(25, 6)
+    _same(scene, pkg.camera_rays(cam, target, 768, 512))
