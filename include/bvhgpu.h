@@ -208,7 +208,7 @@ typedef struct {
                         are ordered (Q8: and nested), without a stack limit, run on the
                         packed scene in every scheme, and workgroup, block, policy, refill
                         and stack_local then change nothing; the scheme's own kernel
-                        records counters (per-ray: on the packed scene too) and step
+                        records counters (large per-ray ones on the packed scene) and step
                         logs, and runs every other scene. */
   int32_t profile;   /* BVHGPU_PROFILE_* */
   int32_t workgroup; /* stream scheme: packet = workgroup^2 rays (8, 16); 0 = 16 */
